@@ -1,6 +1,6 @@
 // blamm_gpu.cu -- libblamm_gpu.so: the C ABI declared in include/blamm_gpu.h.
 //
-// Host half of the GB300 scan: motif-bank planning (length-sorted N tiles,
+// Host half of the GB300 scan: motif-bank planning (length-sorted motif tiles,
 // fixed-point BF16 hi/lo split, per-column guard band), device buffers, and
 // the drivers that chain pack -> fused tcgen05 scan -> FP32 rescoring (or the
 // plain FP32 kernel) on the context's stream.
@@ -75,16 +75,17 @@ struct blamm_ctx {
     // tensor-core plan (valid for plan_terms; rebuilt on mode/threshold change)
     int plan_terms = 0;
     bool plan_valid = false;
-    std::vector<TileDesc> tiles;
+    int ntiles = 0;
+    std::vector<TileDesc> tiles;  // ntiles + 1: the last one holds the end offset
     std::vector<float> guard;    // per column
-    std::vector<double> bias_T;  // per column: threshold - guard on the column grid
-    int erows = 0;  // one-hot pair entries per E stage
-    uint32_t b_term_max = 0, tmem_cols = 0;
-    int acc_stages = 2;
+    int erows = 0;               // one-hot entries per E stage
+    int plan_tg = 1;             // most tiles per group whose A fits in shared memory (evened out)
+    bool plan_stream = false;    // not even one tile fits: A is streamed
     TileDesc *d_tiles = nullptr;
-    uint8_t *d_bbuf = nullptr;
+    uint8_t *d_abuf = nullptr;
     int32_t *d_slot_col = nullptr;
-    size_t cap_tiles = 0, cap_bbuf = 0, cap_slot_col = 0;
+    float *d_slot_thr = nullptr;
+    size_t cap_tiles = 0, cap_abuf = 0, cap_slot_col = 0, cap_slot_thr = 0;
     // per-column fixed-point BF16 terms and guard bands of the bank (for colq_terms terms)
     bool colq_valid = false;
     int colq_terms = 0;
@@ -93,7 +94,8 @@ struct blamm_ctx {
     std::vector<uint32_t> colq_off;  // column c's 4L values start at colq_off[c]
     std::vector<uint16_t> colq_hi, colq_lo;
     std::vector<uint8_t> colq_e8;  // E4M3 codes of P(c) x 2^colq_k[c] (the E4M3 form)
-    // planner knobs (the autotuner sets them): widest N tile, fixed cycles per job
+    // planner knobs: widest tile (columns beyond a tile's 128 rows have no effect) and the
+    // fixed cycles per job (kept for callers that set and read it; no plan depends on it)
     int plan_nmax = 256;
     double plan_job_cost = 700.0;
 
@@ -179,6 +181,19 @@ static int ensure(blamm_ctx *ctx, T **ptr, size_t *cap, size_t need)
     return BLAMM_OK;
 }
 
+// Candidate record slots: `need` rounded up to whole blocks (the scan counts on it), and a
+// spare block behind them, where the scan puts what does not fit.
+static int ensure_cand(blamm_ctx *ctx, int64_t need)
+{
+    need = std::max<int64_t>(1, (need + kRecBlock - 1) / kRecBlock) * kRecBlock;
+    if (ctx->d_cand && need <= ctx->cand_cap) return BLAMM_OK;
+    size_t cap = ctx->d_cand ? (size_t)(ctx->cand_cap + kRecBlock) : 0;
+    ctx->cand_cap = 0;
+    const int rc = ensure(ctx, &ctx->d_cand, &cap, (size_t)(need + kRecBlock));
+    if (!rc) ctx->cand_cap = need;
+    return rc;
+}
+
 static int scanned_columns(const blamm_ctx *ctx)
 {
     return ctx->active.empty() ? ctx->ncols : (int)ctx->active.size();
@@ -218,15 +233,9 @@ inline uint16_t bf16_bits_exact(double v)
     return (uint16_t)(u >> 16);  // exact: v has <= 8 significant bits
 }
 
-// A tile whose longest motif has length L = 4g-3 or 4g-2 leaves motif positions 4g-2 and
-// 4g-1 (the second K core of its last k-step) unused: the bias rides there.
-inline bool bias_folds(int L) { return L % 4 == 1 || L % 4 == 2; }
-
 // E4M3 (sign, 4 exponent bits with bias 7, 3 mantissa bits; exponent 0 subnormal, largest
 // finite 448).  In units of 2^-9 every E4M3 value is an integer: m (subnormal, m < 8) or
 // (8 + m) 2^(e-1).
-constexpr int64_t kE4M3MaxUnits = 448 * 512;
-
 // The E4M3 value nearest to v (ties to even mantissa), as its code; |v| <= 448.
 inline uint8_t e4m3_round(double v)
 {
@@ -258,33 +267,6 @@ inline int64_t e4m3_units(uint8_t code)
     return code & 0x80 ? -a : a;
 }
 
-// Split an integer number of 2^-9 units into E4M3 values that add up to it exactly, the
-// largest first (each step leaves less than an eighth of the rest).  Returns the count,
-// or -1 if more than `cap` pieces would be needed.
-inline int e4m3_pieces(int64_t t, uint8_t *out, int cap)
-{
-    int n = 0;
-    while (t != 0) {
-        if (n == cap) return -1;
-        const int64_t a = t < 0 ? -t : t;
-        uint8_t code;
-        if (a >= kE4M3MaxUnits) {
-            code = 0x7E;  // 448
-        } else if (a < 8) {
-            code = (uint8_t)a;
-        } else {
-            int e = 1;
-            while (e < 15 && a >= ((int64_t)16 << (e - 1))) ++e;
-            const int64_t m = (a >> (e - 1)) - 8;  // rounded down: the piece never exceeds a
-            code = (uint8_t)((e << 3) | (int)m);
-        }
-        if (t < 0) code |= 0x80;
-        out[n++] = code;
-        t -= e4m3_units(code);
-    }
-    return n;
-}
-
 }  // namespace
 
 static int build_plan(blamm_ctx *ctx, int terms)
@@ -311,53 +293,13 @@ static int build_plan(blamm_ctx *ctx, int terms)
     if (e8 && lmax_sel > kMaxE4M3Len)
         return fail(ctx, BLAMM_ERR_UNSUPPORTED, "motif length %d exceeds the E4M3 form's limit %d", lmax_sel,
                     kMaxE4M3Len);
-    const int gmax_all = std::max(1, (lmax_sel + kpos - 1) / kpos);
-    const int erows_all = kBM + kpos * gmax_all + 8;
-    const long long smem_limit = (long long)ctx->max_smem;
-    // everything but the B tiles (E stages, bias A tile, candidate staging, ...)
-    const long long other = (long long)tc_smem_layout(0u, terms, erows_all, 256).total;
-    const long long b_term_cap = (smem_limit - other) / nterm;
-    const int ncap = std::max(32, std::min(256, ctx->plan_nmax / 32 * 32));
-    // widest tile whose B terms (g motif k-steps + 1 bias k-step) fit shared memory
-    auto nmax_for = [&](int g) {
-        long long n = b_term_cap / (32LL * (g + 1));
-        n = n / 32 * 32;
-        return (int)std::min<long long>(ncap, n);
-    };
-    if (nmax_for(gmax_all) < 32)
-        return fail(ctx, BLAMM_ERR_UNSUPPORTED, "motif bank does not fit shared memory");
-
-    // DP over sorted columns: tile = contiguous run of sorted columns.
-    // Per-job cycle model: MMA = (terms*g + bias)*N/2, epilogue ~ N, plus a fixed cost per
-    // job (hand-offs); the bias MMA is folded into the last k-step when the tile's longest
-    // motif leaves that k-step's second K core unused.
-    const double kInf = 1e300;
-    std::vector<double> f(nsel + 1, kInf);
-    std::vector<int> from(nsel + 1, -1);
-    f[0] = 0.0;
-    // A tile's cost depends only on its padded width N and its last (longest) column, and
-    // f is non-decreasing, so for each N the tile that starts as far left as N allows is
-    // the best: 8 candidates per end column instead of 256, same optimum.
-    for (int j = 1; j <= nsel; ++j) {
-        const int L = ctx->len[order[j - 1]];
-        const int g = std::max(1, (L + kpos - 1) / kpos);
-        const int bias = !e8 && bias_folds(L) ? 0 : 1;
-        for (int N = 32; N <= 256; N += 32) {
-            if (N > nmax_for(g)) break;
-            const int i = std::max(0, j - N);
-            const double mma = (nterm * g + bias) * N / 2.0, epi = 1.0 * N;
-            const double cost = std::max(std::max(mma, epi), 300.0) + ctx->plan_job_cost;
-            if (f[i] + cost < f[j]) {
-                f[j] = f[i] + cost;
-                from[j] = i;
-            }
-            if (i == 0) break;
-        }
-        if (from[j] < 0) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "tile planning failed");
-    }
+    const int gmax = std::max(1, (lmax_sel + kpos - 1) / kpos);
+    // Tiles: at most 128 columns each, longest motifs first, cut from the long end, so that
+    // only the tile of the shortest motifs is partly empty.  A job of a tile costs its
+    // k-steps whatever its number of columns, so no other cut is cheaper.
+    const int width = std::min(kTileCols, std::max(32, std::min(256, ctx->plan_nmax / 32 * 32)));
     std::vector<std::pair<int, int>> spans;
-    for (int j = nsel; j > 0; j = from[j]) spans.push_back({from[j], j});
-    std::reverse(spans.begin(), spans.end());
+    for (int j = nsel; j > 0; j -= width) spans.push_back({std::max(0, j - width), j});
     const int ncols = ctx->ncols;
 
     // per-column quantisation and guard band: computed once per bank and number of terms
@@ -416,125 +358,76 @@ static int build_plan(blamm_ctx *ctx, int terms)
     ctx->guard.assign(ncols, 0.0f);
     for (const int c : order) ctx->guard[c] = (float)guard_d[c];
 
-    // tiles, slots, B buffer.  B term layout (canonical no-swizzle K-major):
-    // element (column i, K index kk) of a tile with g motif k-steps sits at
-    // ((i/8 * 2(g+1) + kk/8) * 8 + i%8) * 8 + kk%8.  The hi term holds the bias,
-    // -T split into three BF16-exact pieces on the column's grid, in K indices
-    // 16g..16g+2 (the bias MMA's k-step) or, in a folded tile, 16g-8..16g-6 (the
-    // second K core of k-step g-1, which no motif of the tile reaches).  The E4M3 form
-    // (1 byte per element, 16 per core row): byte ((i/8 * 2(g+1) + kk/16) * 8 + i%8) * 16
-    // + kk%16, K index 4j + b for position j, base b; the bias k-step (K 32g..32g+31)
-    // holds -T x 2^k (T on the grid 2^-(9+k)) as up to 32 E4M3 pieces.
+    // Tiles, slots, A buffer.  A of one k-step of one term (kStepBytes): row i, K core cc (0, 1),
+    // byte x of 16 at (16 cc + i / 8) * 128 + (i % 8) * 16 + x; K index 4j + b for motif
+    // position j, base b, 8 (BF16) or 16 (E4M3) of them per core.  A tile's terms follow one
+    // another.
     std::vector<TileDesc> tiles;
-    std::vector<int32_t> slot_col;
-    std::vector<uint8_t> bbuf;
-    ctx->bias_T.assign(ncols, 0.0);
-    int gmax = 1;
-    uint32_t btmax = 0;
-    int nmax = 0;
+    const size_t nslots = spans.size() * kTileCols;
+    std::vector<int32_t> slot_col(nslots, -1);
+    std::vector<float> slot_thr(nslots, std::numeric_limits<float>::infinity());
+    int nsteps = 0;
     for (auto &sp : spans) {
-        const int cnt = sp.second - sp.first;
-        const int L = ctx->len[order[sp.second - 1]];
-        const int g = std::max(1, (L + kpos - 1) / kpos);
-        const int N = (cnt + 31) / 32 * 32;
-        TileDesc td{};
-        td.slot0 = (int32_t)slot_col.size();
-        td.n = N;
-        td.g = g;
-        td.b_bytes = N * 32 * (g + 1);  // 32 bytes per column and k-step in both forms
-        td.fold = !e8 && bias_folds(L) ? 1 : 0;
-        const int kb = td.fold ? 16 * g - 8 : 16 * g;  // K index of the first bias piece
-        size_t off = (bbuf.size() + 1023) / 1024 * 1024;
-        td.b_off = (int64_t)off;
-        bbuf.resize(off + (size_t)td.b_bytes * nterm, 0);
-        if (e8) {
-            uint8_t *b8 = bbuf.data() + off;
-            auto at = [&](int i, int kk) {
-                return ((size_t)((i / 8) * 2 * (g + 1) + kk / 16) * 8 + i % 8) * 16 + kk % 16;
-            };
-            for (int i = 0; i < N; ++i) {
-                const int c = i < cnt ? order[sp.first + i] : -1;
-                slot_col.push_back(c);
-                // T x 2^k in units of 2^-9, kept within the scores a window can reach
-                // (|sum q| x 2^k <= 64 L): below it every window is a candidate, above it none
-                // is (a padding column: T = 1.0, never a candidate)
-                int64_t Tint = 512;
-                if (c >= 0) {
-                    const int k = kcol[c];
-                    const double lim = (double)(64 * ctx->len[c] + 1) * 512.0;
-                    const double t = ((double)ctx->thr[c] - guard_d[c]) * std::ldexp(1.0, 9 + k);
-                    Tint = std::isnan(t) ? (int64_t)lim : (int64_t)std::floor(std::max(-lim, std::min(lim, t)));
-                    ctx->bias_T[c] = std::ldexp((double)Tint, -9 - k);
-                }
-                uint8_t pcs[32];
-                const int np = e4m3_pieces(-Tint, pcs, 32);
-                if (np < 0) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "E4M3 bias of column %d needs over 32 pieces", c);
-                for (int q = 0; q < np; ++q) b8[at(i, 32 * g + q)] = pcs[q];
-                if (c < 0) continue;
-                const uint32_t o = ctx->colq_off[c], nk = ctx->colq_off[c + 1] - o;
-                for (uint32_t kk = 0; kk < nk; ++kk) b8[at(i, (int)kk)] = ctx->colq_e8[o + kk];
-            }
-            tiles.push_back(td);
-            gmax = std::max(gmax, g);
-            btmax = std::max<uint32_t>(btmax, (uint32_t)td.b_bytes);
-            nmax = std::max(nmax, N);
-            continue;
-        }
-        uint16_t *b_hi = reinterpret_cast<uint16_t *>(bbuf.data() + off);
-        uint16_t *b_lo = terms == 2 ? reinterpret_cast<uint16_t *>(bbuf.data() + off + td.b_bytes) : nullptr;
-        auto elem = [&](int i, int kk) {
-            return ((size_t)((i / 8) * 2 * (g + 1) + kk / 8) * 8 + i % 8) * 8 + kk % 8;
-        };
-        for (int i = 0; i < N; ++i) {
-            const int c = i < cnt ? order[sp.first + i] : -1;
-            slot_col.push_back(c);
-            // bias: T on the grid u = 2^-(k+8), clamped to +-2^23 u (a padding column
-            // gets T = 2^22 u at k = 0: never a candidate)
-            int k = 0;
-            int64_t Tint = (int64_t)1 << 22;
-            if (c >= 0) {
-                k = kcol[c];
-                const double t = ((double)ctx->thr[c] - guard_d[c]) * std::ldexp(1.0, k + 8);
-                const double lim = std::ldexp(1.0, 23);
-                Tint = std::isnan(t) ? (int64_t)lim : (int64_t)std::floor(std::max(-lim, std::min(lim, t)));
-                ctx->bias_T[c] = (double)Tint * std::ldexp(1.0, -(k + 8));
-            }
-            const int64_t pa = (int64_t)std::llround((double)Tint / 65536.0);
-            const int64_t rem = Tint - pa * 65536;
-            const int64_t pb = (int64_t)std::llround((double)rem / 256.0);
-            const int64_t pc = rem - pb * 256;
-            const int64_t pieces[3] = {pa * 65536, pb * 256, pc};
-            for (int s = 0; s < 3; ++s)
-                if (pieces[s] != 0) b_hi[elem(i, kb + s)] = bf16_bits_exact(-std::ldexp((double)pieces[s], -(k + 8)));
-            if (c < 0) continue;
+        const int g = std::max(1, (ctx->len[order[sp.second - 1]] + kpos - 1) / kpos);
+        tiles.push_back(TileDesc{g, nsteps});
+        nsteps += g * nterm;
+    }
+    tiles.push_back(TileDesc{0, nsteps});
+    std::vector<uint8_t> abuf((size_t)nsteps * kStepBytes, 0);
+    for (size_t t = 0; t < spans.size(); ++t) {
+        const auto &sp = spans[t];
+        for (int i = 0; i < sp.second - sp.first; ++i) {
+            const int c = order[sp.first + i], k = kcol[c];
+            const size_t slot = t * kTileCols + i;
+            slot_col[slot] = c;
+            // T = threshold - guard, rounded down to the accumulator's grid (u = 2^-(k+8), or
+            // 2^-9 on the E4M3 form's scale 2^k) and kept within the scores a window can reach
+            // (2^23 u; 64 L 2^-k): below them every window is a candidate, above them none is
+            const double thr = (double)ctx->thr[c] - guard_d[c];
+            const double lim = e8 ? (double)(64 * ctx->len[c] + 1) * 512.0 : std::ldexp(1.0, 23);
+            const double x = std::ldexp(thr, e8 ? 9 + k : 8 + k);
+            const double Tint = std::isnan(x) ? lim : std::floor(std::max(-lim, std::min(lim, x)));
+            slot_thr[slot] = (float)std::ldexp(Tint, e8 ? -9 : -(k + 8));  // exact: |Tint| <= 2^23
             const uint32_t o = ctx->colq_off[c], nk = ctx->colq_off[c + 1] - o;
+            uint8_t *row = abuf.data() + (size_t)tiles[t].off * kStepBytes + (i / 8) * 128 + (i % 8) * 16;
+            const size_t term = (size_t)tiles[t].g * kStepBytes;
             for (uint32_t kk = 0; kk < nk; ++kk) {
-                b_hi[elem(i, (int)kk)] = ctx->colq_hi[o + kk];
-                if (b_lo) b_lo[elem(i, (int)kk)] = ctx->colq_lo[o + kk];
+                if (e8) {
+                    row[(size_t)(kk / 16) * 2048 + kk % 16] = ctx->colq_e8[o + kk];
+                    continue;
+                }
+                uint8_t *at = row + (size_t)(kk / 8) * 2048 + 2 * (kk % 8);
+                std::memcpy(at, &ctx->colq_hi[o + kk], 2);
+                if (terms == 2) std::memcpy(at + term, &ctx->colq_lo[o + kk], 2);
             }
         }
-        tiles.push_back(td);
-        gmax = std::max(gmax, g);
-        btmax = std::max<uint32_t>(btmax, (uint32_t)td.b_bytes);
-        nmax = std::max(nmax, N);
     }
 
     // upload (buffers are reused; the copies are ordered on the context's stream)
     int rc = ensure(ctx, &ctx->d_tiles, &ctx->cap_tiles, tiles.size());
-    if (!rc) rc = ensure(ctx, &ctx->d_bbuf, &ctx->cap_bbuf, bbuf.size());
-    if (!rc) rc = ensure(ctx, &ctx->d_slot_col, &ctx->cap_slot_col, slot_col.size());
+    if (!rc) rc = ensure(ctx, &ctx->d_abuf, &ctx->cap_abuf, abuf.size());
+    if (!rc) rc = ensure(ctx, &ctx->d_slot_col, &ctx->cap_slot_col, nslots);
+    if (!rc) rc = ensure(ctx, &ctx->d_slot_thr, &ctx->cap_slot_thr, nslots);
     if (rc) return rc;
     CK(cudaMemcpyAsync(ctx->d_tiles, tiles.data(), sizeof(TileDesc) * tiles.size(), cudaMemcpyHostToDevice,
                        ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_bbuf, bbuf.data(), bbuf.size(), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_slot_col, slot_col.data(), sizeof(int32_t) * slot_col.size(),
-                       cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_abuf, abuf.data(), abuf.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_slot_col, slot_col.data(), sizeof(int32_t) * nslots, cudaMemcpyHostToDevice,
+                       ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_slot_thr, slot_thr.data(), sizeof(float) * nslots, cudaMemcpyHostToDevice,
+                       ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));  // the host vectors go out of scope
     ctx->tiles = tiles;
-    ctx->erows = kBM + kpos * gmax + 8;
-    ctx->b_term_max = btmax;
-    ctx->tmem_cols = 512u;  // the whole TMEM: 4 accumulators of <= 128 columns or 2 of <= 256
-    ctx->acc_stages = nmax <= 128 ? 4 : 2;
+    ctx->ntiles = (int)spans.size();
+    ctx->erows = kBlockPos + kpos * gmax + 8;
+    // groups: as many of the first (longest) tiles as fit beside the E stages, then evened out
+    const TcSmem L0 = tc_smem_layout(0, ctx->erows);
+    const int room = (ctx->max_smem - (int)L0.total) / kStepBytes;
+    int tg = 0;
+    while (tg < ctx->ntiles && tiles[tg + 1].off <= room) ++tg;
+    ctx->plan_stream = ctx->ntiles > 0 && tg == 0;
+    const int ng = tg > 0 ? (ctx->ntiles + tg - 1) / tg : std::max(1, ctx->ntiles);
+    ctx->plan_tg = std::max(1, (ctx->ntiles + ng - 1) / ng);
     ctx->plan_terms = terms;
     ctx->plan_valid = true;
     return BLAMM_OK;
@@ -566,22 +459,28 @@ int blamm_ctx_create(int device, blamm_ctx **out)
             return fail(ctx, BLAMM_ERR_UNSUPPORTED, "compute capability %d.%d is not sm_100-class",
                         prop.major, prop.minor);
         ctx->sm_count = prop.multiProcessorCount;
-        // scan window (positions, a multiple of 128): BLAMM_SCAN_WINDOW overrides the default
+        // scan window (positions, a multiple of 256): BLAMM_SCAN_WINDOW overrides the default
         ctx->ewindow = kEWindowDefault;
         if (const char *w = std::getenv("BLAMM_SCAN_WINDOW"))
-            ctx->ewindow = std::max<int64_t>(kBM, std::atoll(w) / kBM * kBM);
+            ctx->ewindow = std::max<int64_t>(kBlockPos, std::atoll(w) / kBlockPos * kBlockPos);
         ctx->max_smem = (int)prop.sharedMemPerBlockOptin;
         cudaFuncAttributes fa;
         // fails if no sm_103a image fits
-        for (const void *k : {(const void *)scan_tc_kernel<false, false, 1>,
-                              (const void *)scan_tc_kernel<false, false, 2>,
-                              (const void *)scan_tc_kernel<true, false, 1>,
-                              (const void *)scan_tc_kernel<true, false, 2>,
-                              (const void *)scan_tc_kernel<false, true, 1>,
-                              (const void *)scan_tc_kernel<false, true, 2>,
-                              (const void *)scan_tc_kernel<false, false, kE4M3>,
-                              (const void *)scan_tc_kernel<true, false, kE4M3>,
-                              (const void *)scan_tc_kernel<false, true, kE4M3>}) {
+        for (const void *k : {(const void *)scan_tc_kernel<false, false, 1, false>,
+                              (const void *)scan_tc_kernel<false, false, 2, false>,
+                              (const void *)scan_tc_kernel<true, false, 1, false>,
+                              (const void *)scan_tc_kernel<true, false, 2, false>,
+                              (const void *)scan_tc_kernel<false, true, 1, false>,
+                              (const void *)scan_tc_kernel<false, true, 2, false>,
+                              (const void *)scan_tc_kernel<false, false, 1, true>,
+                              (const void *)scan_tc_kernel<false, false, 2, true>,
+                              (const void *)scan_tc_kernel<true, false, 1, true>,
+                              (const void *)scan_tc_kernel<true, false, 2, true>,
+                              (const void *)scan_tc_kernel<false, true, 1, true>,
+                              (const void *)scan_tc_kernel<false, true, 2, true>,
+                              (const void *)scan_tc_kernel<false, false, kE4M3, false>,
+                              (const void *)scan_tc_kernel<true, false, kE4M3, false>,
+                              (const void *)scan_tc_kernel<false, true, kE4M3, false>}) {
             CK(cudaFuncGetAttributes(&fa, k));
             if (fa.maxThreadsPerBlock < kTcThreads)
                 return fail(ctx, BLAMM_ERR_UNSUPPORTED,
@@ -612,8 +511,8 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    void *bufs[] = {ctx->d_P,      ctx->d_len,   ctx->d_thr,      ctx->d_tiles, ctx->d_bbuf,
-                    ctx->d_slot_col, ctx->d_prof, ctx->d_bases, ctx->d_seq2, ctx->d_zmask, ctx->d_e16,
+    void *bufs[] = {ctx->d_P,      ctx->d_len,   ctx->d_thr,      ctx->d_tiles, ctx->d_abuf,
+                    ctx->d_slot_col, ctx->d_slot_thr, ctx->d_prof, ctx->d_bases, ctx->d_seq2, ctx->d_zmask, ctx->d_e16,
                     ctx->d_runs,   ctx->d_cand,  ctx->d_hits,     ctx->d_counters, ctx->d_status,
                     ctx->d_active, ctx->d_chunk_bases[0], ctx->d_chunk_bases[1], ctx->d_chunk_runs[0],
                     ctx->d_chunk_runs[1], ctx->d_raw, ctx->d_stream, ctx->d_srun[0], ctx->d_srun[1],
@@ -644,7 +543,7 @@ static int64_t call_buffer_bytes(const blamm_ctx *ctx)
                      8 * ctx->cap_runs + 8 * (ctx->cap_chunk_runs[0] + ctx->cap_chunk_runs[1]) +
                      ctx->cap_chunk_bases[0] + ctx->cap_chunk_bases[1] + ctx->cap_raw + ctx->cap_stream +
                      8 * (ctx->cap_srun[0] + ctx->cap_srun[1] + ctx->cap_srun[2] + ctx->cap_shdr)) +
-           16 * ctx->cand_cap + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
+           16 * (ctx->cand_cap > 0 ? ctx->cand_cap + kRecBlock : 0) + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
 }
 
 int blamm_ctx_call_bytes(const blamm_ctx *ctx, int64_t *bytes)
@@ -809,9 +708,9 @@ static int ensure_plan(blamm_ctx *ctx)
 // The tensor-core scan runs over windows of at most ctx->ewindow positions (16 Mi by
 // default): per window the one-hot entries of its positions (e16_kernel or e8_kernel, 16 B
 // each) and one scan launch, so the entry array holds one window (256 MB) whatever the stream
-// length.  A window's scan reads up to entry (its positions) + 127 + 4 * 64 + 2 (BF16) or
-// + 127 + 8 * 32 + 3 (E4M3), and the entry kernels read up to base i + 3 of the padded
-// stream: entries = positions + kStreamPad - 64 stay inside both.
+// length.  A window's scan copies up to entry (its positions rounded up to 256) + 4 * 64 (BF16)
+// or + 8 * 8 (E4M3), and the entry kernels read up to base i + 3 of the padded stream:
+// entries = positions + kStreamPad - 64 stay inside both.
 static int64_t e16_entries(const blamm_ctx *ctx, int64_t n) { return std::min(n, ctx->ewindow) + kStreamPad - 64; }
 
 static int launch_pack(blamm_ctx *ctx, const char *d_bases, int64_t n)
@@ -839,29 +738,29 @@ static TcParams tc_params(const blamm_ctx *ctx, int64_t n)
 {
     TcParams p{};
     p.n = n;
-    p.n_mtiles = (n + kBM - 1) / kBM;
     p.tiles = ctx->d_tiles;
-    p.ntiles = (int32_t)ctx->tiles.size();
+    p.ntiles = (int32_t)ctx->ntiles;
     p.terms = ctx->plan_terms;
-    p.bbuf = ctx->d_bbuf;
+    p.abuf = ctx->d_abuf;
     p.slot_col = ctx->d_slot_col;
+    p.slot_thr = ctx->d_slot_thr;
     p.erows = ctx->erows;
-    p.b_term_max = ctx->b_term_max;
-    p.tmem_cols = ctx->tmem_cols;
-    p.acc_stages = ctx->acc_stages;
     p.wait_limit = ctx->wait_limit;
     p.dump_ncols = ctx->ncols;
     return p;
 }
 
+static int64_t scan_blocks(int64_t n) { return (n + kBlockPos - 1) / kBlockPos; }
+
 // The scan kernel counts jobs and record slots in 32 bits.
 constexpr int64_t kMaxJobs = 0x7fffffff;
 constexpr int64_t kMaxRecordSlots = (int64_t(1) << 31) - 1024;
 
-static int check_jobs(blamm_ctx *ctx, long long njobs)
+static int check_jobs(blamm_ctx *ctx, int64_t n)
 {
+    const long long njobs = (long long)ctx->ntiles * scan_blocks(n);
     return njobs > kMaxJobs ? fail(ctx, BLAMM_ERR_UNSUPPORTED,
-                                   "%lld scan jobs (tiles x 128-position blocks) exceed one launch's %lld; "
+                                   "%lld scan jobs (tiles x 256-position blocks) exceed one launch's %lld; "
                                    "scan the stream in parts", njobs, (long long)kMaxJobs)
                             : BLAMM_OK;
 }
@@ -882,9 +781,11 @@ static int64_t record_slots_guess(const blamm_ctx *ctx, int64_t n, double per = 
 static RescoreParams rescore_params(const blamm_ctx *ctx, const uint4 *cand, const unsigned long long *cand_count,
                                     int64_t cand_cap, const uint32_t *seq2,
                                     const uint32_t *zmask, int64_t n, const int64_t *d_runs, int64_t nruns,
-                                    blamm_hit *d_hits, unsigned long long *hit_count, int64_t hit_cap)
+                                    blamm_hit *d_hits, unsigned long long *hit_count, int64_t hit_cap,
+                                    unsigned long long *ncand)
 {
     RescoreParams r{};
+    r.ncand = ncand;
     r.cand = cand;
     r.slot_col = ctx->d_slot_col;
     r.cand_count = cand_count;
@@ -907,40 +808,56 @@ static RescoreParams rescore_params(const blamm_ctx *ctx, const uint4 *cand, con
 }
 
 // One launch of the scan kernel instance that p asks for.
-template <bool kDump, bool kProf>
+template <bool kDump, bool kProf, bool kStream>
 static void launch_tc_as(const TcParams &p, int grid, uint32_t smem, cudaStream_t st)
 {
-    if (p.terms == 2) scan_tc_kernel<kDump, kProf, 2><<<grid, kTcThreads, smem, st>>>(p);
-    else if (p.terms == kE4M3) scan_tc_kernel<kDump, kProf, kE4M3><<<grid, kTcThreads, smem, st>>>(p);
-    else scan_tc_kernel<kDump, kProf, 1><<<grid, kTcThreads, smem, st>>>(p);
+    if (p.terms == 2) scan_tc_kernel<kDump, kProf, 2, kStream><<<grid, kTcThreads, smem, st>>>(p);
+    else if (!kStream && p.terms == kE4M3) scan_tc_kernel<kDump, kProf, kE4M3, false><<<grid, kTcThreads, smem, st>>>(p);
+    else scan_tc_kernel<kDump, kProf, 1, kStream><<<grid, kTcThreads, smem, st>>>(p);
 }
 
+template <bool kStream>
 static void launch_tc(const TcParams &p, bool dump, int grid, uint32_t smem, cudaStream_t st)
 {
-    if (dump) launch_tc_as<true, false>(p, grid, smem, st);
-    else if (p.prof) launch_tc_as<false, true>(p, grid, smem, st);
-    else launch_tc_as<false, false>(p, grid, smem, st);
+    if (dump) launch_tc_as<true, false, kStream>(p, grid, smem, st);
+    else if (p.prof) launch_tc_as<false, true, kStream>(p, grid, smem, st);
+    else launch_tc_as<false, false, kStream>(p, grid, smem, st);
 }
 
 // The scan of n positions of a packed stream (p: the plan, candidates, counters, status),
 // window by window: the window's one-hot entries into e16, then its scan launch.  Returns the
 // largest grid used; adds the launches to *launches.
 static int launch_tc_windows(blamm_ctx *ctx, TcParams p, const uint32_t *seq2, const uint32_t *zmask, uint4 *e16,
-                             int64_t n, bool dump, uint32_t smem, int *launches, int *grid_out)
+                             int64_t n, bool dump, int *launches, int *grid_out)
 {
-    const int64_t n_mtiles = (n + kBM - 1) / kBM, wt = std::max<int64_t>(1, ctx->ewindow / kBM);
+    const int64_t nblocks = scan_blocks(n), wb = std::max<int64_t>(1, ctx->ewindow / kBlockPos);
     int gmax = 0;
-    for (int64_t m0 = 0; m0 < n_mtiles; m0 += wt) {
-        const int64_t mt = std::min(wt, n_mtiles - m0), base = m0 * kBM;
-        const int64_t ne = std::min(mt * kBM, n - base) + kStreamPad - 64;
+    for (int64_t b0 = 0; b0 < nblocks; b0 += wb) {
+        const int64_t nb = std::min(wb, nblocks - b0), base = b0 * kBlockPos;
+        const int64_t ne = std::min(nb * kBlockPos, n - base) + kStreamPad - 64;
         if (p.terms == kE4M3) e8_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, ctx->stream>>>(seq2, zmask, base, ne, e16);
         else e16_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, ctx->stream>>>(seq2, zmask, base, ne, e16);
         CK(cudaGetLastError());
         p.e16 = e16;
-        p.n_mtiles = mt;
-        p.m0 = (int32_t)m0;
-        const int grid = (int)std::min<long long>(ctx->sm_count, (long long)ctx->tiles.size() * mt);
-        launch_tc(p, dump, grid, smem, ctx->stream);
+        p.nblocks = (int32_t)nb;
+        p.chunk0 = (uint32_t)(base / 32);
+        // Tiles per group: the plan's, or fewer where a CTA would get less than about 8 units
+        // (units differ by one between CTAs); blocks fewer than CTAs go out in ranges.
+        const int64_t per_cta = (int64_t)ctx->ntiles * nb / ctx->sm_count;
+        const int tg = ctx->plan_stream ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(ctx->plan_tg, per_cta / 8));
+        const int ng = (ctx->ntiles + tg - 1) / tg;
+        p.tg = (ctx->ntiles + ng - 1) / ng;
+        const int grid = (int)std::min<int64_t>(ctx->sm_count, (int64_t)ng * nb);
+        p.contiguous = nb < grid ? 1 : 0;
+        // (the longest tiles come first: the first group is the largest)
+        const int steps = ctx->tiles[std::min(p.tg, ctx->ntiles)].off;
+        p.a_bytes = (uint32_t)(ctx->plan_stream ? kChunks * kChunkBlocks : steps) * kStepBytes;
+        // at least ~116 KB so that two CTAs never share an SM (each allocates all of TMEM)
+        const uint32_t smem = std::max<uint32_t>(tc_smem_layout(p.a_bytes, p.erows).total, 116 * 1024);
+        if ((int)smem > ctx->max_smem)
+            return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", smem, ctx->max_smem);
+        if (ctx->plan_stream) launch_tc<true>(p, dump, grid, smem, ctx->stream);
+        else launch_tc<false>(p, dump, grid, smem, ctx->stream);
         CK(cudaGetLastError());
         gmax = std::max(gmax, grid);
         if (launches) *launches += 2;
@@ -955,28 +872,15 @@ static int run_tc(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t nrun
 {
     int rc = ensure_plan(ctx);
     if (rc) return rc;
-    const int64_t n_mtiles = (n + kBM - 1) / kBM;
-    const long long njobs = (long long)ctx->tiles.size() * n_mtiles;
-    if ((rc = check_jobs(ctx, njobs))) return rc;
-    if (ctx->cand_cap == 0) {
-        size_t cap = 0;
-        rc = ensure(ctx, &ctx->d_cand, &cap, (size_t)record_slots_guess(ctx, n));
-        if (rc) return rc;
-        ctx->cand_cap = (int64_t)cap;
-    }
-    const TcSmem L = tc_smem_layout(ctx->b_term_max, ctx->plan_terms, ctx->erows,
-                                    (int)ctx->tiles.size());
-    if ((int)L.total > ctx->max_smem)
-        return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", L.total, ctx->max_smem);
-    // at least ~116 KB so that two CTAs never share an SM (each allocates TMEM)
-    const uint32_t smem = std::max<uint32_t>(L.total, 116 * 1024);
+    if ((rc = check_jobs(ctx, n))) return rc;
+    if (ctx->cand_cap == 0 && (rc = ensure_cand(ctx, record_slots_guess(ctx, n)))) return rc;
+    const bool any = n > 0 && ctx->ntiles > 0;
     for (int attempt = 0; attempt < 3; ++attempt) {
         CK(cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
         CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
         TcParams p = tc_params(ctx, n);
         p.cand = ctx->d_cand;
         p.cand_count = ctx->d_counters;
-        p.ncand = ctx->d_counters + 3;
         p.cand_cap = ctx->cand_cap;
         p.status = ctx->d_status;
         p.wait_limit = ctx->wait_limit;
@@ -992,10 +896,10 @@ static int run_tc(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t nrun
             p.prof = ctx->d_prof;
         }
         int grid = 0;
-        if (njobs > 0) {
+        if (any) {
             CK(cudaEventRecord(ctx->ev[4], ctx->stream));
-            if ((rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, dump != nullptr, smem,
-                                        launches, &grid)))
+            if ((rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, dump != nullptr, launches,
+                                        &grid)))
                 return rc;
             CK(cudaEventRecord(ctx->ev[5], ctx->stream));
         }
@@ -1005,8 +909,8 @@ static int run_tc(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t nrun
         CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof status, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         if (status) return fail(ctx, BLAMM_ERR_TIMEOUT, "scan kernel: a device wait timed out");
-        if (njobs > 0) cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[4], ctx->ev[5]);
-        if (ctx->prof_on && njobs > 0) {
+        if (any) cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[4], ctx->ev[5]);
+        if (ctx->prof_on && any) {
             ctx->prof.resize((size_t)32 * grid);
             CK(cudaMemcpy(ctx->prof.data(), ctx->d_prof, sizeof(long long) * 32 * grid, cudaMemcpyDeviceToHost));
             ctx->prof_ctas = grid;
@@ -1015,25 +919,19 @@ static int run_tc(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t nrun
         ctx->rec_slots = (int64_t)ncand;
         if ((int64_t)ncand <= ctx->cand_cap) break;
         // grow and re-run
-        size_t cap = 0;
-        CK(cudaFreeAsync(ctx->d_cand, ctx->stream));
-        ctx->d_cand = nullptr;
-        ctx->cand_cap = 0;
         if ((int64_t)ncand >= kMaxRecordSlots)
             return fail(ctx, BLAMM_ERR_OVERFLOW, "%llu candidate records exceed one launch's %lld", ncand,
                         (long long)kMaxRecordSlots);
-        rc = ensure(ctx, &ctx->d_cand, &cap,
-                    (size_t)std::min<int64_t>((int64_t)(ncand + ncand / 4 + 1024), kMaxRecordSlots));
+        rc = ensure_cand(ctx, std::min<int64_t>((int64_t)(ncand + ncand / 4 + 1024), kMaxRecordSlots));
         if (rc) return rc;
-        ctx->cand_cap = (int64_t)cap;
         if (attempt == 2) return fail(ctx, BLAMM_ERR_OVERFLOW, "candidate buffer overflow");
     }
     const RescoreParams r = rescore_params(ctx, ctx->d_cand, ctx->d_counters, ctx->cand_cap,
                                            ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits,
-                                           ctx->d_counters + 1, hit_cap);
+                                           ctx->d_counters + 1, hit_cap, ctx->d_counters + 3);
     const int64_t nc = ctx->rec_slots;
     if (nc > 0) {
-        const int threads = 256;
+        const int threads = kRescoreThreads;
         const int64_t blocks = std::min<int64_t>((nc + threads - 1) / threads, (int64_t)ctx->sm_count * 16);
         CK(cudaEventRecord(ctx->ev[6], ctx->stream));
         rescore_kernel<<<(unsigned)blocks, threads, 0, ctx->stream>>>(r);
@@ -1134,7 +1032,7 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
     if (ctx->plain_timed) cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[4], ctx->ev[5]);
     if (ctx->rescore_timed) cudaEventElapsedTime(&ctx->stats.rescore_ms, ctx->ev[6], ctx->ev[7]);
     ctx->stats.hits = (int64_t)nh;
-    ctx->stats.tiles = (int32_t)(ctx->mode == BLAMM_MODE_FP32 ? 0 : ctx->tiles.size());
+    ctx->stats.tiles = (int32_t)(ctx->mode == BLAMM_MODE_FP32 ? 0 : ctx->ntiles);
     ctx->stats.launches = launches;
     *n_hits = (int64_t)nh;
     return (int64_t)nh > hit_cap ? fail(ctx, BLAMM_ERR_OVERFLOW, "%lld hits > capacity %lld",
@@ -1266,27 +1164,19 @@ static int enqueue_chunk(blamm_ctx *ctx, const char *d_bases, int64_t n, const i
     }
     CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), ctx->stream));      // record slots of this chunk
     CK(cudaMemsetAsync(cnt + 3, 0, sizeof(unsigned long long), ctx->stream));  // its candidates
-    const int64_t n_mtiles = (n + kBM - 1) / kBM;
-    const long long njobs = (long long)ctx->tiles.size() * n_mtiles;
-    int rc = check_jobs(ctx, njobs);
+    int rc = check_jobs(ctx, n);
     if (rc) return rc;
-    const TcSmem L = tc_smem_layout(ctx->b_term_max, ctx->plan_terms, ctx->erows, (int)ctx->tiles.size());
-    if ((int)L.total > ctx->max_smem)
-        return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", L.total, ctx->max_smem);
     TcParams p = tc_params(ctx, n);
     p.cand = ctx->d_cand;
     p.cand_count = cnt;
-    p.ncand = cnt + 3;
     p.cand_cap = ctx->cand_cap;
     p.status = ctx->d_status;
     p.wait_limit = ctx->wait_limit;
     p.dump_ncols = ctx->ncols;
-    if ((rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, false,
-                                std::max<uint32_t>(L.total, 116 * 1024), nullptr, nullptr)))
-        return rc;
+    if ((rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, false, nullptr, nullptr))) return rc;
     const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask,
-                                           n, d_runs, nruns, d_hits, cnt + 1, hit_cap);
-    rescore_kernel<<<(unsigned)(ctx->sm_count * 8), 256, 0, ctx->stream>>>(r);
+                                           n, d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
+    rescore_kernel<<<(unsigned)(ctx->sm_count * 8), kRescoreThreads, 0, ctx->stream>>>(r);
     CK(cudaGetLastError());
     return BLAMM_OK;
 }
@@ -1318,11 +1208,7 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         // candidates: four times the usual first guess for a chunk (a chunk that still
         // overflows sends the whole call to the synchronous path)
         const double want = (double)record_slots_guess(ctx, span, 250.0);
-        if ((double)ctx->cand_cap < want) {
-            size_t cap = ctx->cand_cap > 0 ? (size_t)ctx->cand_cap : 0;
-            if ((rc = ensure(ctx, &ctx->d_cand, &cap, (size_t)want))) return rc;
-            ctx->cand_cap = (int64_t)cap;
-        }
+        if ((rc = ensure_cand(ctx, (int64_t)want))) return rc;
     }
     size_t hc = (size_t)ctx->hits_cap;
     if ((rc = ensure(ctx, &ctx->d_hits, &hc, (size_t)std::max<int64_t>(hit_cap, 1)))) return rc;
@@ -1417,7 +1303,7 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
     blamm_stats total{};
     total.positions = n;
     total.columns = scanned_columns(ctx);
-    total.tiles = (int32_t)(tc ? ctx->tiles.size() : 0);
+    total.tiles = (int32_t)(tc ? ctx->ntiles : 0);
     total.launches = 0;
     for (int64_t k = 0; k < nchunks; ++k) {  // packing + scan (+ rescoring and a one-hot build per window)
         const int64_t len = std::min(n, (k + 1) * kPipeChunk + ov) - k * kPipeChunk;
@@ -1748,13 +1634,11 @@ int blamm_debug_scores(blamm_ctx *ctx, const char *bases, int64_t n, int64_t p0,
                                         cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = fail(ctx, BLAMM_ERR_CUDA, "%s", cudaGetErrorString(e));
-        // the accumulator holds sum(q) - T; report sum(q) (exact: both are on the column grid)
-        for (int64_t i = 0; rc == BLAMM_OK && i < npos; ++i)
+        // the E4M3 form's accumulator is scaled by 2^k (exact: a power of two)
+        for (int64_t i = 0; rc == BLAMM_OK && ctx->plan_terms == kE4M3 && i < npos; ++i)
             for (int c = 0; c < ctx->ncols; ++c) {
                 float &v = out[i * ctx->ncols + c];
-                // the E4M3 form's accumulator is scaled by 2^k (exact: a power of two)
-                const double sv = ctx->plan_terms == kE4M3 ? std::ldexp((double)v, -ctx->colq_k[c]) : (double)v;
-                v = (float)(sv + ctx->bias_T[c]);
+                v = (float)std::ldexp((double)v, -ctx->colq_k[c]);
             }
     }
     cudaFree(d_dump);
@@ -1784,7 +1668,7 @@ constexpr size_t kStaticSeq2Off = 0;
 constexpr size_t kStaticZmaskOff = round256(kStaticSeq2Off + sizeof(uint32_t) * 2 * kStaticWords32);
 constexpr size_t kStaticE16Off = round256(kStaticZmaskOff + sizeof(uint32_t) * kStaticWords32);
 constexpr size_t kStaticCandOff = round256(kStaticE16Off + sizeof(uint4) * (kStaticMaxBases + kStreamPad));
-constexpr size_t kStaticCountOff = round256(kStaticCandOff + sizeof(uint4) * kStaticCandCap);
+constexpr size_t kStaticCountOff = round256(kStaticCandOff + sizeof(uint4) * (kStaticCandCap + kRecBlock));
 constexpr size_t kStaticStatusOff = round256(kStaticCountOff + sizeof(unsigned long long) * 4);
 constexpr size_t kStaticBytes = round256(kStaticStatusOff + sizeof(int));  // about 97 MiB
 
@@ -1865,22 +1749,14 @@ int blamm_scan_device_static(blamm_ctx *ctx, const char *d_bases, int64_t n, con
         if ((rc = launch_plain(ctx, p))) return rc;
         ++launches;
     } else {
-        const int64_t n_mtiles = (n + kBM - 1) / kBM;
-        const long long njobs = (long long)ctx->tiles.size() * n_mtiles;
-        const TcSmem L = tc_smem_layout(ctx->b_term_max, ctx->plan_terms, ctx->erows, (int)ctx->tiles.size());
-        if ((int)L.total > ctx->max_smem)
-            return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", L.total, ctx->max_smem);
-        const uint32_t smem = std::max<uint32_t>(L.total, 116 * 1024);
         TcParams p = tc_params(ctx, n);
         p.cand = cand;
         p.cand_count = counters;
-        p.ncand = counters + 3;
         p.cand_cap = kStaticCandCap;
         p.status = status;
         p.wait_limit = ctx->wait_limit;
         p.dump_ncols = ctx->ncols;
-        (void)njobs;
-        if ((rc = launch_tc_windows(ctx, p, seq2, zmask, e16, n, false, smem, &launches, nullptr))) return rc;
+        if ((rc = launch_tc_windows(ctx, p, seq2, zmask, e16, n, false, &launches, nullptr))) return rc;
         unsigned long long ncand = 0;
         int st = 0;
         CK(cudaMemcpyAsync(&ncand, counters, sizeof ncand, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1893,8 +1769,8 @@ int blamm_scan_device_static(blamm_ctx *ctx, const char *d_bases, int64_t n, con
                         "fewer positions per call)", ncand, (long long)kStaticCandCap);
         if (ncand > 0) {
             const RescoreParams r = rescore_params(ctx, cand, counters, kStaticCandCap, seq2, zmask, n,
-                                                   d_run_start, nruns, d_hits, counters + 1, hit_cap);
-            const int threads = 256;
+                                                   d_run_start, nruns, d_hits, counters + 1, hit_cap, counters + 3);
+            const int threads = kRescoreThreads;
             const int64_t blocks = std::min<int64_t>(((int64_t)ncand + threads - 1) / threads,
                                                      (int64_t)ctx->sm_count * 16);
             rescore_kernel<<<(unsigned)blocks, threads, 0, ctx->stream>>>(r);
@@ -1908,7 +1784,7 @@ int blamm_scan_device_static(blamm_ctx *ctx, const char *d_bases, int64_t n, con
     const unsigned long long nh = cnt[1];
     if (tc) ctx->stats.candidates = (int64_t)cnt[3];
     ctx->stats.hits = (int64_t)nh;
-    ctx->stats.tiles = (int32_t)(tc ? ctx->tiles.size() : 0);
+    ctx->stats.tiles = (int32_t)(tc ? ctx->ntiles : 0);
     ctx->stats.launches = launches;
     *n_hits = (int64_t)nh;
     return (int64_t)nh > hit_cap ? fail(ctx, BLAMM_ERR_OVERFLOW, "%lld hits > capacity %lld", (long long)nh,
@@ -1937,12 +1813,7 @@ int blamm_reserve(blamm_ctx *ctx, int64_t max_positions, int64_t max_candidates)
         if ((rc = ensure(ctx, &ctx->d_e16, &ctx->cap_e16, (size_t)e16_entries(ctx, max_positions)))) return rc;
         // record slots: at most one record per candidate, plus the blocks the warps reserve
         const int64_t slots = std::min(max_candidates + record_slots_reserved(ctx->sm_count), kMaxRecordSlots);
-        if (slots > ctx->cand_cap) {
-            size_t cap = ctx->cand_cap > 0 ? (size_t)ctx->cand_cap : 0;
-            rc = ensure(ctx, &ctx->d_cand, &cap, (size_t)slots);
-            if (rc) return rc;
-            ctx->cand_cap = (int64_t)cap;
-        }
+        if ((rc = ensure_cand(ctx, slots))) return rc;
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return BLAMM_OK;
@@ -1977,27 +1848,20 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
         PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_run_start, nruns, d_hits, hit_cap, cnt + 1);
         return launch_plain(ctx, p);
     }
-    const int64_t n_mtiles = (n + kBM - 1) / kBM;
-    const long long njobs = (long long)ctx->tiles.size() * n_mtiles;
-    if (int rc = check_jobs(ctx, njobs)) return rc;
-    const TcSmem L = tc_smem_layout(ctx->b_term_max, ctx->plan_terms, ctx->erows, (int)ctx->tiles.size());
-    if ((int)L.total > ctx->max_smem)
-        return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", L.total, ctx->max_smem);
+    if (int rc = check_jobs(ctx, n)) return rc;
     TcParams p = tc_params(ctx, n);
     p.cand = ctx->d_cand;
     p.cand_count = cnt;
-    p.ncand = cnt + 3;
     p.cand_cap = ctx->cand_cap;
     p.status = reinterpret_cast<int *>(cnt + 2);
     p.wait_limit = ctx->wait_limit;
     p.dump_ncols = ctx->ncols;
-    if (int rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, false,
-                                   std::max<uint32_t>(L.total, 116 * 1024), nullptr, nullptr))
+    if (int rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, false, nullptr, nullptr))
         return rc;
     const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask,
-                                           n, d_run_start, nruns, d_hits, cnt + 1, hit_cap);
+                                           n, d_run_start, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
     // a fixed grid: the candidate count is only known on the device
-    rescore_kernel<<<(unsigned)(ctx->sm_count * 8), 256, 0, ctx->stream>>>(r);
+    rescore_kernel<<<(unsigned)(ctx->sm_count * 8), kRescoreThreads, 0, ctx->stream>>>(r);
     CK(cudaGetLastError());
     return BLAMM_OK;
 }
@@ -2081,10 +1945,7 @@ int blamm_autotune(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t
     int rc = ensure(ctx, &ctx->d_hits, &hc, (size_t)1 << 20);
     if (rc) return rc;
     ctx->hits_cap = (int64_t)hc;
-    const int nmax_opts[] = {128, 192, 256};
-    const double cost_opts[] = {200.0, 700.0, 1500.0};
-    const int keep_nmax = ctx->plan_nmax, keep_terms = ctx->auto_terms;
-    const double keep_cost = ctx->plan_job_cost;
+    const int keep_terms = ctx->auto_terms;
     // BLAMM_MODE_AUTO also chooses the form: one BF16 term halves the MMAs of two and
     // widens the guard band (more candidates to rescore), one E4M3 term (motifs up to 64
     // positions) halves them again with a still wider band, so the whole call's kernel
@@ -2097,38 +1958,27 @@ int blamm_autotune(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t
     int term_opts[3] = {1, 2, kE4M3};
     const int nterm_opts = ctx->mode == BLAMM_MODE_AUTO ? (lmax_sel <= kMaxE4M3Len ? 3 : 2) : 1;
     float best = std::numeric_limits<float>::infinity();
-    int bn = keep_nmax, bt = keep_terms;
-    double bc = keep_cost;
-    for (int ti = 0; ti < nterm_opts; ++ti)
-        for (int nm : nmax_opts)
-            for (double jc : cost_opts) {
-                if (ctx->mode == BLAMM_MODE_AUTO) ctx->auto_terms = term_opts[ti];
-                ctx->plan_nmax = nm;
-                ctx->plan_job_cost = jc;
+    int bt = keep_terms;
+    for (int ti = 0; ti < nterm_opts; ++ti) {
+        if (ctx->mode == BLAMM_MODE_AUTO) ctx->auto_terms = term_opts[ti];
+        ctx->plan_valid = false;
+        float t[5];
+        for (float &ms : t) {
+            int64_t nh = 0;
+            rc = scan_core(ctx, d_bases, ns, d_run_start, nrs, ctx->d_hits, ctx->hits_cap, &nh);
+            if (rc && rc != BLAMM_ERR_OVERFLOW) {
+                ctx->auto_terms = keep_terms;
                 ctx->plan_valid = false;
-                float t[3];
-                for (int rep = 0; rep < 3; ++rep) {
-                    int64_t nh = 0;
-                    rc = scan_core(ctx, d_bases, ns, d_run_start, nrs, ctx->d_hits, ctx->hits_cap, &nh);
-                    if (rc && rc != BLAMM_ERR_OVERFLOW) {
-                        ctx->plan_nmax = keep_nmax;
-                        ctx->plan_job_cost = keep_cost;
-                        ctx->auto_terms = keep_terms;
-                        ctx->plan_valid = false;
-                        return rc;
-                    }
-                    t[rep] = ctx->stats.kernel_ms;
-                }
-                std::sort(t, t + 3);
-                if (t[1] < best) {
-                    best = t[1];
-                    bn = nm;
-                    bc = jc;
-                    bt = ctx->auto_terms;
-                }
+                return rc;
             }
-    ctx->plan_nmax = bn;
-    ctx->plan_job_cost = bc;
+            ms = ctx->stats.kernel_ms;
+        }
+        std::sort(t, t + 5);
+        if (t[2] < best) {
+            best = t[2];
+            bt = ctx->auto_terms;
+        }
+    }
     ctx->auto_terms = bt;
     ctx->plan_valid = false;
     if ((rc = ensure_plan(ctx))) return rc;

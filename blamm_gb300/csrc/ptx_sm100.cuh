@@ -146,6 +146,42 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, l
     return mbar_wait(bar, parity, &never, limit_cycles);
 }
 
+// ---------------------------------------------------------------- shared memory
+__device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
+__device__ __forceinline__ uint32_t ld_shared(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// A predicated 16-byte store: no branch around it.
+__device__ __forceinline__ void st_global_v4_if(bool f, void *a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %0, 0;\n\t"
+        "@p st.global.v4.b32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"((int)f),
+        "l"(a), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+}
+
+// ---------------------------------------------------------------- hardware barriers
+// A barrier of `threads` threads (whole warps): some arrive and go on, the others wait.
+__device__ __forceinline__ void named_sync(uint32_t id, uint32_t threads)
+{
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ void named_arrive(uint32_t id, uint32_t threads)
+{
+    asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
@@ -283,22 +319,52 @@ __device__ __forceinline__ void tmem_ld_max_32x32b_x32(uint32_t taddr, uint32_t 
         : "memory");
 }
 
+// The same for 16 columns.
+__device__ __forceinline__ void tmem_ld_max_32x32b_x16(uint32_t taddr, uint32_t (&r)[16], float &red)
+{
+    asm volatile(
+        "tcgen05.ld.red.sync.aligned.32x32b.x16.max.f32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, %16, [%17];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15]), "=f"(red)
+        : "r"(taddr)
+        : "memory");
+}
+
 __device__ __forceinline__ void tmem_wait_ld()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Empty asm that "redefines" 32 registers: placed after tcgen05.wait::ld (both
+// Empty asm that "redefines" the registers: placed after tcgen05.wait::ld (both
 // volatile, so they keep their order), it stops the compiler from moving uses
 // of the loaded registers above the wait.
-__device__ __forceinline__ void reg_fence(uint32_t (&r)[32])
+template <int N>
+__device__ __forceinline__ void reg_fence(uint32_t (&r)[N])
 {
-    asm volatile(""
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
-                   "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
-                   "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]),
-                   "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]),
-                   "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]));
+#pragma unroll
+    for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+
+// Two FP32 values in one 64-bit register pair, and their packed sum (round to nearest).
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+
+__device__ __forceinline__ void unpack2(uint64_t v, uint32_t &lo, uint32_t &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+}
+
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // tcgen05.wait::ld that also "redefines" the destination registers of the

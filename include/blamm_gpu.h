@@ -69,7 +69,7 @@ typedef struct {
     int64_t columns;     /* motif columns scanned */
     int64_t candidates;  /* positions x columns that passed the guard band */
     int64_t hits;        /* occurrences found */
-    int32_t tiles;       /* motif tiles (tcgen05 N tiles) */
+    int32_t tiles;       /* motif tiles (up to 128 columns each) */
     int32_t launches;    /* kernels launched by the last scan */
     float kernel_ms;     /* device time of all kernels of the call (CUDA events) */
     float total_ms;      /* time of the whole call incl. copies (device events; wall time
@@ -155,7 +155,7 @@ int blamm_filter_score(blamm_ctx *ctx, float *d_R, int m, int n, const float *d_
  * enqueues packing, the scan and the rescoring on the context's stream and
  * returns.  counts is device memory of 4 uint64, set when the stream gets
  * there: [0] candidate record slots used (a record holds the candidates of one
- * position in a 32-column chunk; each CTA's warps take slots in blocks), [1]
+ * column in a 32-position chunk; each CTA's warps take slots in blocks), [1]
  * hits, [2] status (non-zero: a device wait timed out), [3] candidates.  Hits
  * beyond hit_cap and records beyond the reservation (max_candidates plus the
  * blocks the warps hold) are counted but not stored; the caller compares counts
@@ -177,19 +177,17 @@ int blamm_scan_graph_launch(blamm_ctx *ctx, void *graph);
 void blamm_scan_graph_destroy(void *graph);
 
 /* Autotuner: time the tensor-core scan of the first min(n, 16 Mi) positions
- * (device data) under several tile plans -- widest N tile 128 / 192 / 256 x
- * the planner's fixed cost per job, and in BLAMM_MODE_AUTO one and two BF16
- * terms and one E4M3 term (motifs up to 64 positions) -- and keep the fastest
- * for later scans of this context (the time of
- * all kernels of the call: packing, scan, rescoring; median of three).
- * *best_ms (optional) receives that time.  Nothing to tune in BLAMM_MODE_FP32.
+ * (device data) -- in BLAMM_MODE_AUTO with one and two BF16 terms and one E4M3 term
+ * (motifs up to 64 positions) -- and keep the fastest form for later scans of this
+ * context (the time of all kernels of the call: packing, scan, rescoring; median of
+ * five).  *best_ms (optional) receives that time.  Nothing to tune in BLAMM_MODE_FP32.
  * The chosen term count: blamm_get_terms. */
 int blamm_autotune(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t *d_run_start,
                    int64_t nruns, float *best_ms);
 
-/* The planner's knobs that the autotuner sets: the widest N tile (32..256
- * columns; at most 128 gives four TMEM accumulators instead of two) and the
- * fixed cycles per job of its cost model.  Setting them replans. */
+/* The planner's knobs: the widest motif tile (32..256 columns; a tile holds at most
+ * 128, so 128 and more plan alike) and the fixed cycles per job of a cost model (kept
+ * and reported; the plan does not depend on it).  Setting them replans. */
 int blamm_set_plan_options(blamm_ctx *ctx, int max_tile_columns, float job_cost);
 /* The tensor-core form of the current mode: 1 or 2 BF16 terms, 8 for one E4M3 term
  * (BLAMM_MODE_E4M3, or BLAMM_MODE_AUTO after the autotuner chose it); 0 for FP32. */
@@ -298,9 +296,9 @@ int blamm_guard_band(const blamm_ctx *ctx, float *out);
 /* Role timing of the tensor-core scan kernel: enable (1) / disable (0) it for
  * later scans; read the last scan's counters (32 int64 per CTA, clock cycles:
  * 0 / 1 the even / odd issuer's waits for a free accumulator, 2 issuers' waits
- * for B tiles, 3 MMA loop, 4 loader waits for a free E stage, 5 loader waits at
- * tile changes, 7 drain warp 0's waits for an accumulator, 8 its loop, 9 its
- * drain (full accumulator to hand-back), 10 jobs, 11 even issuer's waits for E
+ * for motif tiles, 3 MMA loop, 4 loader waits for a free E stage, 5 loader waits at
+ * tile group changes, 7 drain warp 0's waits for an accumulator, 8 its loop, 9 its
+ * drain (full accumulator to hand-back), 10 tiles x 128-position blocks, 11 even issuer's waits for E
  * windows, 12 drain warp 0's rounds with candidates, 13 its record block
  * changes, 15 its candidate test and record writing).  *nctas receives the
  * CTA count.  The timing variant of the kernel is slower than the scan itself. */
@@ -331,7 +329,7 @@ int blamm_release_buffers(blamm_ctx *ctx);
  * declares (about 97 MiB per device, reserved when the library's device code
  * is loaded there).  Limits: n <= 4 Mi positions per call (more gives
  * BLAMM_ERR_ARG) and at most 2 Mi tensor-core candidate record slots per call
- * (a record holds one position's candidates in a 32-column chunk; each CTA's
+ * (a record holds one column's candidates in a 32-position chunk; each CTA's
  * warps take slots in blocks, about 0.6 Mi of them on a full GPU; more gives
  * BLAMM_ERR_OVERFLOW: scan fewer positions per call).  The counters and the
  * status word are set to zero at the start of every call.  Preconditions are
