@@ -136,6 +136,11 @@ struct blamm_ctx {
     int64_t *d_srun[3] = {nullptr, nullptr, nullptr}, *d_shdr = nullptr;
     size_t cap_srun[3] = {0, 0, 0}, cap_shdr = 0;
     int64_t stream_n = 0, stream_nruns = 0, stream_nseqs = 0;
+    // FASTA parsing: tile summaries, the parser before each tile, totals (96 bytes per 16 KB of text)
+    IngTile *d_ing_tiles = nullptr;
+    IngPrefix *d_ing_prefix = nullptr;
+    unsigned long long *d_ing_totals = nullptr;
+    size_t cap_ing_tiles = 0, cap_ing_prefix = 0, cap_ing_totals = 0;
     bool prof_on = false;
     long long *d_prof = nullptr;
     std::vector<long long> prof;  // last scan's role timing, 32 counters per CTA
@@ -466,21 +471,12 @@ int blamm_ctx_create(int device, blamm_ctx **out)
         ctx->max_smem = (int)prop.sharedMemPerBlockOptin;
         cudaFuncAttributes fa;
         // fails if no sm_103a image fits
+        // (the raw-score and role-timing instances are set up when they are launched)
         for (const void *k : {(const void *)scan_tc_kernel<false, false, 1, false>,
                               (const void *)scan_tc_kernel<false, false, 2, false>,
-                              (const void *)scan_tc_kernel<true, false, 1, false>,
-                              (const void *)scan_tc_kernel<true, false, 2, false>,
-                              (const void *)scan_tc_kernel<false, true, 1, false>,
-                              (const void *)scan_tc_kernel<false, true, 2, false>,
-                              (const void *)scan_tc_kernel<false, false, 1, true>,
-                              (const void *)scan_tc_kernel<false, false, 2, true>,
-                              (const void *)scan_tc_kernel<true, false, 1, true>,
-                              (const void *)scan_tc_kernel<true, false, 2, true>,
-                              (const void *)scan_tc_kernel<false, true, 1, true>,
-                              (const void *)scan_tc_kernel<false, true, 2, true>,
                               (const void *)scan_tc_kernel<false, false, kE4M3, false>,
-                              (const void *)scan_tc_kernel<true, false, kE4M3, false>,
-                              (const void *)scan_tc_kernel<false, true, kE4M3, false>}) {
+                              (const void *)scan_tc_kernel<false, false, 1, true>,
+                              (const void *)scan_tc_kernel<false, false, 2, true>}) {
             CK(cudaFuncGetAttributes(&fa, k));
             if (fa.maxThreadsPerBlock < kTcThreads)
                 return fail(ctx, BLAMM_ERR_UNSUPPORTED,
@@ -516,7 +512,7 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
                     ctx->d_runs,   ctx->d_cand,  ctx->d_hits,     ctx->d_counters, ctx->d_status,
                     ctx->d_active, ctx->d_chunk_bases[0], ctx->d_chunk_bases[1], ctx->d_chunk_runs[0],
                     ctx->d_chunk_runs[1], ctx->d_raw, ctx->d_stream, ctx->d_srun[0], ctx->d_srun[1],
-                    ctx->d_srun[2], ctx->d_shdr};
+                    ctx->d_srun[2], ctx->d_shdr, ctx->d_ing_tiles, ctx->d_ing_prefix, ctx->d_ing_totals};
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -542,7 +538,9 @@ static int64_t call_buffer_bytes(const blamm_ctx *ctx)
     return (int64_t)(ctx->cap_bases + 4 * ctx->cap_words32 + 4 * ctx->cap_zmask + 16 * ctx->cap_e16 +
                      8 * ctx->cap_runs + 8 * (ctx->cap_chunk_runs[0] + ctx->cap_chunk_runs[1]) +
                      ctx->cap_chunk_bases[0] + ctx->cap_chunk_bases[1] + ctx->cap_raw + ctx->cap_stream +
-                     8 * (ctx->cap_srun[0] + ctx->cap_srun[1] + ctx->cap_srun[2] + ctx->cap_shdr)) +
+                     8 * (ctx->cap_srun[0] + ctx->cap_srun[1] + ctx->cap_srun[2] + ctx->cap_shdr) +
+                     sizeof(IngTile) * ctx->cap_ing_tiles + sizeof(IngPrefix) * ctx->cap_ing_prefix +
+                     8 * ctx->cap_ing_totals) +
            16 * (ctx->cand_cap > 0 ? ctx->cand_cap + kRecBlock : 0) + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
 }
 
@@ -577,6 +575,9 @@ int blamm_release_buffers(blamm_ctx *ctx)
     drop(&ctx->d_stream, &ctx->cap_stream);
     for (int k = 0; k < 3; ++k) drop(&ctx->d_srun[k], &ctx->cap_srun[k]);
     drop(&ctx->d_shdr, &ctx->cap_shdr);
+    drop(&ctx->d_ing_tiles, &ctx->cap_ing_tiles);
+    drop(&ctx->d_ing_prefix, &ctx->cap_ing_prefix);
+    drop(&ctx->d_ing_totals, &ctx->cap_ing_totals);
     ctx->stream_n = ctx->stream_nruns = ctx->stream_nseqs = 0;
     if (ctx->d_cand) cudaFreeAsync(ctx->d_cand, ctx->stream);
     ctx->d_cand = nullptr;
@@ -811,9 +812,14 @@ static RescoreParams rescore_params(const blamm_ctx *ctx, const uint4 *cand, con
 template <bool kDump, bool kProf, bool kStream>
 static void launch_tc_as(const TcParams &p, int grid, uint32_t smem, cudaStream_t st)
 {
-    if (p.terms == 2) scan_tc_kernel<kDump, kProf, 2, kStream><<<grid, kTcThreads, smem, st>>>(p);
-    else if (!kStream && p.terms == kE4M3) scan_tc_kernel<kDump, kProf, kE4M3, false><<<grid, kTcThreads, smem, st>>>(p);
-    else scan_tc_kernel<kDump, kProf, 1, kStream><<<grid, kTcThreads, smem, st>>>(p);
+    auto go = [&](auto *kernel) {
+        if (kDump || kProf)
+            cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kernel<<<grid, kTcThreads, smem, st>>>(p);
+    };
+    if (p.terms == 2) go(scan_tc_kernel<kDump, kProf, 2, kStream>);
+    else if (!kStream && p.terms == kE4M3) go(scan_tc_kernel<kDump, kProf, kE4M3, false>);
+    else go(scan_tc_kernel<kDump, kProf, 1, kStream>);
 }
 
 template <bool kStream>
@@ -2076,29 +2082,6 @@ int blamm_theoretical_hist(blamm_ctx *ctx, const float *P, int p_rows, int ncols
 
 // ------------------------------------------------------------------ FASTA ingest on the GPU
 
-// In-place inclusive scan of v[0..n) with Op; `scratch` holds at least
-// scan_scratch_words(n) values.
-static size_t scan_scratch_words(int64_t n)
-{
-    size_t w = 0;
-    for (int64_t t = (n + kScanTile - 1) / kScanTile; t > 1; t = (t + kScanTile - 1) / kScanTile) w += (size_t)t;
-    return w + 1;
-}
-
-template <class Op>
-static cudaError_t device_scan(cudaStream_t st, int64_t *v, int64_t n, int64_t *scratch)
-{
-    if (n <= 0) return cudaSuccess;
-    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    scan_tiles_kernel<Op><<<(unsigned)tiles, kScanThreads, 0, st>>>(v, n, scratch);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || tiles == 1) return e;
-    e = device_scan<Op>(st, scratch, tiles, scratch + tiles);
-    if (e != cudaSuccess) return e;
-    scan_add_kernel<Op><<<(unsigned)tiles, kScanThreads, 0, st>>>(v, n, scratch);
-    return cudaGetLastError();
-}
-
 // FASTA text on the device -> filtered stream, run table and header offsets.  Outputs go
 // to the caller's buffers, or (resident: the caller's pointers are null) into the
 // context's resident-stream buffers, sized once the counts are known.
@@ -2107,100 +2090,49 @@ static int fasta_parse(blamm_ctx *ctx, const char *d_raw, int64_t nraw, bool res
                        int64_t *n_bases, int64_t *nruns, int64_t *nseqs, uint64_t *nucl_counts)
 {
     cudaStream_t st = ctx->stream;
-    const size_t n = (size_t)nraw, sw = scan_scratch_words(nraw);
-    // four per-byte arrays (line starts, header count, sequence characters, stream bases),
-    // the per-sequence character offsets, scan scratch and a status word
-    int64_t *A = nullptr, *B = nullptr, *Cc = nullptr, *D = nullptr, *sc0 = nullptr, *scr = nullptr;
-    int *bad = nullptr;
-    unsigned long long *nucl = nullptr;
-    int64_t *bseq = nullptr, *bpos = nullptr;
-    int rc = BLAMM_OK;
-    cudaError_t e = cudaMallocAsync(&A, 8 * n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&B, 8 * n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&Cc, 8 * n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&D, 8 * n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&sc0, 8 * n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&scr, 8 * sw, st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&bad, sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMallocAsync(&nucl, 4 * sizeof(unsigned long long), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(nucl, 0, 4 * sizeof(unsigned long long), st);
-    const unsigned grid = (unsigned)std::min<int64_t>((nraw + 255) / 256, (int64_t)ctx->sm_count * 32);
-    if (e == cudaSuccess) {
-        ingest_lines_kernel<<<grid, 256, 0, st>>>(d_raw, nraw, A, B);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = device_scan<MaxOp>(st, A, nraw, scr);
-    if (e == cudaSuccess) e = device_scan<SumOp>(st, B, nraw, scr);
-    if (e == cudaSuccess) {
-        ingest_chars_kernel<<<grid, 256, 0, st>>>(d_raw, nraw, A, B, Cc, D, bad);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = device_scan<SumOp>(st, Cc, nraw, scr);
-    if (e == cudaSuccess) e = device_scan<SumOp>(st, D, nraw, scr);
-    int64_t tot[2] = {0, 0};
-    int badh = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tot[0], B + nraw - 1, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tot[1], D + nraw - 1, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&badh, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    const int64_t ns = tot[0], nb = tot[1];
-    const bool go = e == cudaSuccess && !badh;
-    if (go && resident) {
+    const int64_t ntiles = (nraw + kIngTile - 1) / kIngTile;
+    if (ntiles > 0x7fffffff) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "%lld bytes of text in one call", (long long)nraw);
+    const int vec = (reinterpret_cast<uintptr_t>(d_raw) & 15u) == 0 ? 1 : 0;  // 16-byte loads
+    int rc = ensure(ctx, &ctx->d_ing_tiles, &ctx->cap_ing_tiles, (size_t)ntiles);
+    if (!rc) rc = ensure(ctx, &ctx->d_ing_prefix, &ctx->cap_ing_prefix, (size_t)ntiles);
+    if (!rc) rc = ensure(ctx, &ctx->d_ing_totals, &ctx->cap_ing_totals, (size_t)kIngTotals);
+    if (rc) return rc;
+    ingest_tiles_kernel<<<(unsigned)ntiles, kIngThreads, 0, st>>>(d_raw, nraw, vec, ctx->d_ing_tiles);
+    CK(cudaGetLastError());
+    ingest_scan_kernel<<<1, kIngScanThreads, 0, st>>>(ctx->d_ing_tiles, (int)ntiles, ctx->d_ing_prefix, ctx->d_ing_totals);
+    CK(cudaGetLastError());
+    auto emit = [&]() -> int {
+        ingest_emit_kernel<<<(unsigned)ntiles, kIngThreads, 0, st>>>(d_raw, nraw, vec, ctx->d_ing_prefix, ctx->d_ing_totals,
+                                                                     d_bases, d_run_start, d_run_seq, d_run_seqpos,
+                                                                     d_header_pos);
+        CK(cudaGetLastError());
+        return BLAMM_OK;
+    };
+    if (!resident && (rc = emit())) return rc;
+    unsigned long long tot[kIngTotals];
+    CK(cudaMemcpyAsync(tot, ctx->d_ing_totals, sizeof tot, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (tot[3]) return fail(ctx, BLAMM_ERR_ARG, "Input file does not appear to be in fasta format");
+    const int64_t nb = (int64_t)tot[0], nr = (int64_t)tot[1], ns = (int64_t)tot[2];
+    if (resident) {
+        // (the writes are ordered on the context's stream like everything that reads them)
         rc = ensure(ctx, &ctx->d_shdr, &ctx->cap_shdr, (size_t)std::max<int64_t>(ns, 1));
         if (!rc) rc = ensure(ctx, &ctx->d_stream, &ctx->cap_stream, (size_t)std::max<int64_t>(nb, 1));
-        d_header_pos = ctx->d_shdr;
-        d_bases = ctx->d_stream;
-    }
-    if (go && !rc) {
-        ingest_headers_kernel<<<grid, 256, 0, st>>>(d_raw, nraw, B, Cc, sc0, d_header_pos);
-        e = cudaGetLastError();
-    }
-    const bool have = go && !rc && nb > 0;
-    if (have && e == cudaSuccess) e = cudaMallocAsync(&bseq, 8 * (size_t)nb, st);
-    if (have && e == cudaSuccess) e = cudaMallocAsync(&bpos, 8 * (size_t)nb, st);
-    if (have && e == cudaSuccess) {
-        ingest_bases_kernel<<<grid, 256, 0, st>>>(d_raw, nraw, A, B, Cc, D, sc0, d_bases, bseq, bpos, nucl);
-        e = cudaGetLastError();
-    }
-    unsigned long long nh[4] = {0, 0, 0, 0};
-    if (have && e == cudaSuccess && nucl_counts) e = cudaMemcpyAsync(nh, nucl, sizeof nh, cudaMemcpyDeviceToHost, st);
-    int64_t nr = 0;
-    const unsigned g2 = (unsigned)std::min<int64_t>((nb + 255) / 256, (int64_t)ctx->sm_count * 32);
-    if (have && e == cudaSuccess) {
-        // run flags into A (no longer needed), scanned in place
-        ingest_runflags_kernel<<<g2, 256, 0, st>>>(bseq, bpos, nb, A);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = device_scan<SumOp>(st, A, nb, scr);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&nr, A + nb - 1, 8, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    }
-    if (have && e == cudaSuccess && resident) {
         for (int k = 0; k < 3 && !rc; ++k)
             rc = ensure(ctx, &ctx->d_srun[k], &ctx->cap_srun[k], (size_t)std::max<int64_t>(nr, 1));
+        if (rc) return rc;
+        d_header_pos = ctx->d_shdr;
+        d_bases = ctx->d_stream;
         d_run_start = ctx->d_srun[0];
         d_run_seq = ctx->d_srun[1];
         d_run_seqpos = ctx->d_srun[2];
+        if ((rc = emit())) return rc;
     }
-    if (have && e == cudaSuccess && !rc) {
-        ingest_runs_kernel<<<g2, 256, 0, st>>>(bseq, bpos, nb, A, d_run_start, d_run_seq, d_run_seqpos);
-        e = cudaGetLastError();
-    }
-    void *bufs[] = {A, B, Cc, D, sc0, scr, bad, bseq, bpos, nucl};
-    for (void *b : bufs)
-        if (b) cudaFreeAsync(b, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) e = e2;
-    if (e != cudaSuccess)
-        return fail(ctx, e == cudaErrorMemoryAllocation ? BLAMM_ERR_NOMEM : BLAMM_ERR_CUDA, "FASTA ingest: %s",
-                    cudaGetErrorString(e));
-    if (rc) return rc;
-    if (badh) return fail(ctx, BLAMM_ERR_ARG, "Input file does not appear to be in fasta format");
     *n_bases = nb;
     *nruns = nr;
     *nseqs = ns;
     if (nucl_counts)
-        for (int b = 0; b < 4; ++b) nucl_counts[b] = nh[b];
+        for (int b = 0; b < 4; ++b) nucl_counts[b] = tot[4 + b];
     return BLAMM_OK;
 }
 
