@@ -136,6 +136,8 @@ struct blamm_ctx {
     int64_t *d_srun[3] = {nullptr, nullptr, nullptr}, *d_shdr = nullptr;
     size_t cap_srun[3] = {0, 0, 0}, cap_shdr = 0;
     int64_t stream_n = 0, stream_nruns = 0, stream_nseqs = 0;
+    uint8_t *d_theo = nullptr;  // theoretical histograms: bank, tables, results of a call
+    size_t cap_theo = 0;
     // FASTA parsing: tile summaries, the parser before each tile, totals (96 bytes per 16 KB of text)
     IngTile *d_ing_tiles = nullptr;
     IngPrefix *d_ing_prefix = nullptr;
@@ -512,7 +514,7 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
                     ctx->d_runs,   ctx->d_cand,  ctx->d_hits,     ctx->d_counters, ctx->d_status,
                     ctx->d_active, ctx->d_chunk_bases[0], ctx->d_chunk_bases[1], ctx->d_chunk_runs[0],
                     ctx->d_chunk_runs[1], ctx->d_raw, ctx->d_stream, ctx->d_srun[0], ctx->d_srun[1],
-                    ctx->d_srun[2], ctx->d_shdr, ctx->d_ing_tiles, ctx->d_ing_prefix, ctx->d_ing_totals};
+                    ctx->d_srun[2], ctx->d_shdr, ctx->d_ing_tiles, ctx->d_ing_prefix, ctx->d_ing_totals, ctx->d_theo};
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -540,7 +542,7 @@ static int64_t call_buffer_bytes(const blamm_ctx *ctx)
                      ctx->cap_chunk_bases[0] + ctx->cap_chunk_bases[1] + ctx->cap_raw + ctx->cap_stream +
                      8 * (ctx->cap_srun[0] + ctx->cap_srun[1] + ctx->cap_srun[2] + ctx->cap_shdr) +
                      sizeof(IngTile) * ctx->cap_ing_tiles + sizeof(IngPrefix) * ctx->cap_ing_prefix +
-                     8 * ctx->cap_ing_totals) +
+                     8 * ctx->cap_ing_totals + ctx->cap_theo) +
            16 * (ctx->cand_cap > 0 ? ctx->cand_cap + kRecBlock : 0) + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
 }
 
@@ -578,6 +580,7 @@ int blamm_release_buffers(blamm_ctx *ctx)
     drop(&ctx->d_ing_tiles, &ctx->cap_ing_tiles);
     drop(&ctx->d_ing_prefix, &ctx->cap_ing_prefix);
     drop(&ctx->d_ing_totals, &ctx->cap_ing_totals);
+    drop(&ctx->d_theo, &ctx->cap_theo);
     ctx->stream_n = ctx->stream_nruns = ctx->stream_nseqs = 0;
     if (ctx->d_cand) cudaFreeAsync(ctx->d_cand, ctx->stream);
     ctx->d_cand = nullptr;
@@ -2013,69 +2016,86 @@ int blamm_theoretical_hist(blamm_ctx *ctx, const float *P, int p_rows, int ncols
             return fail(ctx, BLAMM_ERR_ARG, "column %d: bad length %d", h, col_len[h]);
     }
     CK(cudaSetDevice(ctx->device));
-    const int kmax = 8192;
-    const size_t smem = theo_smem_bytes(kmax, nbins, fp64_dp);
-    if (smem > (size_t)ctx->max_smem) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "histogram does not fit");
-    std::vector<int32_t> hof(ncols);
-    for (int c = 0; c < ncols; ++c) hof[c] = hist_of ? hist_of[c] : c;
-    float *d_P = nullptr, *d_pv = nullptr, *d_thr = nullptr;
-    int32_t *d_len = nullptr, *d_hof = nullptr;
-    unsigned long long *d_counts = nullptr;
-    int *d_status = nullptr;
-    const size_t pbytes = sizeof(float) * (size_t)p_rows * ncols;
-    cudaError_t e = cudaMallocAsync(&d_P, pbytes, ctx->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_len, sizeof(int32_t) * ncols, ctx->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_hof, sizeof(int32_t) * ncols, ctx->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync(&d_status, sizeof(int), ctx->stream);
-    if (e == cudaSuccess && npv > 0) e = cudaMallocAsync(&d_pv, sizeof(float) * npv, ctx->stream);
-    if (e == cudaSuccess && npv > 0) e = cudaMallocAsync(&d_thr, sizeof(float) * (size_t)npv * ncols, ctx->stream);
-    if (e == cudaSuccess && counts)
-        e = cudaMallocAsync(&d_counts, sizeof(unsigned long long) * (size_t)ncols * nbins, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_P, P, pbytes, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_len, col_len, sizeof(int32_t) * ncols, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_hof, hof.data(), sizeof(int32_t) * ncols, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess && npv > 0)
-        e = cudaMemcpyAsync(d_pv, pvalues, sizeof(float) * npv, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_status, 0, sizeof(int), ctx->stream);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(theoretical_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int status = 0;
-    if (e == cudaSuccess) {
-        TheoHistParams p{};
-        p.P = d_P;
-        p.p_rows = p_rows;
-        p.ncols = ncols;
-        p.col_len = d_len;
-        p.hist_of = d_hof;
-        for (int k = 0; k < 4; ++k) p.bg[k] = bg_prob[k];
-        p.nbins = nbins;
-        p.max_length = max_length;
-        p.fp64_dp = fp64_dp ? 1 : 0;
-        p.kmax = kmax;
-        p.pvalues = d_pv;
-        p.npv = npv;
-        p.thr = d_thr;
-        p.counts = d_counts;
-        p.status = d_status;
-        theoretical_hist_kernel<<<ncols, 256, smem, ctx->stream>>>(p);
-        e = cudaGetLastError();
+    // the distinct distributions, and the columns that have each
+    std::vector<int32_t> slot(ncols, -1), dist, tab;
+    int lmax = 1;
+    for (int c = 0; c < ncols; ++c) {
+        const int h = hist_of ? hist_of[c] : c;
+        if (slot[h] < 0) {
+            slot[h] = (int32_t)dist.size();
+            dist.push_back(h);
+            lmax = std::max(lmax, (int)col_len[h]);
+        }
     }
-    if (e == cudaSuccess && npv > 0)
-        e = cudaMemcpyAsync(thr, d_thr, sizeof(float) * (size_t)npv * ncols, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && counts)
-        e = cudaMemcpyAsync(counts, d_counts, sizeof(unsigned long long) * (size_t)ncols * nbins,
-                            cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    void *bufs[] = {d_P, d_len, d_hof, d_status, d_pv, d_thr, d_counts};
-    for (void *b : bufs)
-        if (b) cudaFreeAsync(b, ctx->stream);
-    const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess) e = e2;
-    if (e != cudaSuccess) return fail(ctx, BLAMM_ERR_CUDA, "theoretical histograms: %s", cudaGetErrorString(e));
-    if (status) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "a score range exceeds %d keys (fewer bins)", kmax);
-    return BLAMM_OK;
+    const int nd = (int)dist.size();
+    std::vector<int32_t> user0(nd + 1, 0), users(ncols), fill;
+    for (int c = 0; c < ncols; ++c) ++user0[slot[hist_of ? hist_of[c] : c] + 1];
+    for (int i = 0; i < nd; ++i) user0[i + 1] += user0[i];
+    fill.assign(user0.begin(), user0.end() - 1);
+    for (int c = 0; c < ncols; ++c) users[fill[slot[hist_of ? hist_of[c] : c]]++] = c;
+    // one table of 32-bit words: lengths, distributions, users, their offsets, p-values, status
+    tab.assign(col_len, col_len + ncols);
+    tab.insert(tab.end(), dist.begin(), dist.end());
+    tab.insert(tab.end(), users.begin(), users.end());
+    tab.insert(tab.end(), user0.begin(), user0.end());
+    const size_t pv_at = tab.size(), status_at = pv_at + (size_t)npv;
+    tab.resize(status_at + 1, 0);
+    if (npv > 0) std::memcpy(&tab[pv_at], pvalues, sizeof(float) * (size_t)npv);
+    const size_t pbytes = sizeof(float) * (size_t)p_rows * ncols, tbytes = sizeof(int32_t) * tab.size();
+    const size_t thr_bytes = sizeof(float) * (size_t)npv * ncols;
+    const size_t cnt_bytes = counts ? sizeof(unsigned long long) * (size_t)ncols * nbins : 0;
+    auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
+    int rc = ensure(ctx, &ctx->d_theo, &ctx->cap_theo, up(cnt_bytes) + up(pbytes) + up(tbytes) + up(thr_bytes));
+    if (rc) return rc;
+    uint8_t *at = ctx->d_theo;
+    auto take = [&](size_t bytes) {
+        uint8_t *r = at;
+        at += up(bytes);
+        return r;
+    };
+    unsigned long long *d_counts = reinterpret_cast<unsigned long long *>(take(cnt_bytes));
+    float *d_P = reinterpret_cast<float *>(take(pbytes));
+    int32_t *d_tab = reinterpret_cast<int32_t *>(take(tbytes));
+    float *d_thr = reinterpret_cast<float *>(take(thr_bytes));
+    CK(cudaMemcpyAsync(d_P, P, pbytes, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(d_tab, tab.data(), tbytes, cudaMemcpyHostToDevice, ctx->stream));
+    TheoHistParams p{};
+    p.P = d_P;
+    p.p_rows = p_rows;
+    p.ncols = ncols;
+    p.col_len = d_tab;
+    p.dist = d_tab + ncols;
+    p.users = p.dist + nd;
+    p.user0 = p.users + ncols;
+    for (int k = 0; k < 4; ++k) p.bg[k] = bg_prob[k];
+    p.nbins = nbins;
+    p.max_length = max_length;
+    p.lmax = lmax;
+    p.pvalues = reinterpret_cast<const float *>(d_tab + pv_at);
+    p.npv = npv;
+    p.thr = npv > 0 ? d_thr : nullptr;
+    p.counts = counts ? d_counts : nullptr;
+    p.status = d_tab + status_at;
+    // Key ranges are about nbins + L, up to a few times that where the rows' minima differ: 2048
+    // keys leave room for several CTAs per SM, and what exceeds them is run again with 8192.
+    for (const int kmax : {2048, 8192}) {
+        if (kmax == 2048 && nbins > 1024) continue;
+        p.kmax = kmax;
+        const size_t smem = theo_smem_bytes(kmax, nbins, lmax, fp64_dp);
+        if (smem > (size_t)ctx->max_smem) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "histogram does not fit");
+        const auto kernel = fp64_dp ? theoretical_hist64_kernel : theoretical_hist_kernel;
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<nd, kTheoThreads, smem, ctx->stream>>>(p);
+        CK(cudaGetLastError());
+        if (npv > 0) CK(cudaMemcpyAsync(thr, d_thr, thr_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        if (counts) CK(cudaMemcpyAsync(counts, d_counts, cnt_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        int status = 0;
+        CK(cudaMemcpyAsync(&status, p.status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (!status) return BLAMM_OK;
+        CK(cudaMemsetAsync(p.status, 0, sizeof(int), ctx->stream));
+    }
+    return fail(ctx, BLAMM_ERR_UNSUPPORTED, "a score range exceeds %d keys (fewer bins)", p.kmax);
 }
 
 }  // extern "C"
