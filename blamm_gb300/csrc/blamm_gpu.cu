@@ -486,7 +486,9 @@ int blamm_ctx_create(int device, blamm_ctx **out)
                             fa.maxThreadsPerBlock, kTcThreads);
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem));
         }
-        CK(cudaFuncSetAttribute(scan_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CK(cudaFuncSetAttribute(plain_scores_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                ctx->max_smem));
+        CK(cudaFuncSetAttribute(plain_scores_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 ctx->max_smem));
         CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         for (auto &ev : ctx->ev) CK(cudaEventCreate(&ev));
@@ -979,19 +981,23 @@ static PlainParams plain_params(const blamm_ctx *ctx, const uint32_t *seq2, cons
     return p;
 }
 
-// Launch it: a block's columns staged in shared memory (as many as fit, at most 32).
+// Launch it: a block's columns staged in shared memory, as many (at most 64) as leave room for
+// four blocks on an SM; about four rounds of blocks, each walking over its share of the
+// position tiles, so that the staging is paid rarely.
+template <bool kHist>
 static int launch_plain(blamm_ctx *ctx, PlainParams &p)
 {
-    const int threads = 256;
-    int cpb = 32;
-    while (cpb > 1 && (size_t)cpb * (p.p_rows + 2) * 4 + threads + p.lmax + 64 > (size_t)ctx->max_smem) cpb /= 2;
+    const int bins = kHist && p.shared_bins ? p.nbins : 0;
+    int cpb = std::min(64, (p.ncols + 3) / 4 * 4);
+    while (cpb > 4 && plain_smem_bytes(cpb, p.lmax, bins) > (size_t)ctx->max_smem / 4) cpb -= 4;
     p.cols_per_block = cpb;
-    const size_t smem = (size_t)cpb * (p.p_rows + 2) * 4 + threads + p.lmax + 64;
-    const int64_t bx = (p.n + threads - 1) / threads;
+    const size_t smem = plain_smem_bytes(cpb, p.lmax, bins);
+    const int64_t tiles = (p.n + kPlainThreads - 1) / kPlainThreads;
     const int by = (p.ncols + cpb - 1) / cpb;
-    if (bx > 0x7fffffff || by > 65535) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "grid too large");
-    if (bx > 0) {
-        scan_plain_kernel<<<dim3((unsigned)bx, (unsigned)by), threads, smem, ctx->stream>>>(p);
+    if (tiles > 0x7fffffff || by > 65535) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "grid too large");
+    if (tiles > 0) {
+        const int64_t bx = std::min(tiles, std::max<int64_t>(1, (int64_t)ctx->sm_count * 16 / by));
+        plain_scores_kernel<kHist><<<dim3((unsigned)bx, (unsigned)by), kPlainThreads, smem, ctx->stream>>>(p);
         CK(cudaGetLastError());
     }
     return BLAMM_OK;
@@ -1005,7 +1011,7 @@ static int run_plain(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t n
                                  ctx->d_counters + 1);
     if (n == 0) return BLAMM_OK;
     CK(cudaEventRecord(ctx->ev[4], ctx->stream));
-    const int rc = launch_plain(ctx, p);
+    const int rc = launch_plain<false>(ctx, p);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[5], ctx->stream));
     ctx->plain_timed = true;
@@ -1169,7 +1175,7 @@ static int enqueue_chunk(blamm_ctx *ctx, const char *d_bases, int64_t n, const i
     CK(cudaGetLastError());
     if (ctx->mode == BLAMM_MODE_FP32) {
         PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits, hit_cap, cnt + 1);
-        return launch_plain(ctx, p);
+        return launch_plain<false>(ctx, p);
     }
     CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), ctx->stream));      // record slots of this chunk
     CK(cudaMemsetAsync(cnt + 3, 0, sizeof(unsigned long long), ctx->stream));  // its candidates
@@ -1484,7 +1490,7 @@ static int score_histograms_on(blamm_ctx *ctx, const char *d_bases, int64_t n, c
         cleanup();
         return fail(ctx, BLAMM_ERR_CUDA, "%s", cudaGetErrorString(e));
     }
-    HistParams p{};
+    PlainParams p{};
     p.seq2 = ctx->d_seq2;
     p.zmask = ctx->d_zmask;
     p.n = n;
@@ -1499,21 +1505,14 @@ static int score_histograms_on(blamm_ctx *ctx, const char *d_bases, int64_t n, c
     p.width = d_w;
     p.nbins = nbins;
     p.counts = d_counts;
-    const int threads = 256;
-    int cpb = 32;
-    auto need = [&](int c) { return (size_t)c * (p.p_rows + nbins) * 4 + threads + p.lmax + 64; };
-    while (cpb > 1 && need(cpb) > (size_t)ctx->max_smem) cpb /= 2;
-    if (need(cpb) > (size_t)ctx->max_smem) {
+    if ((size_t)(p.p_rows + nbins) * 4 + 256 + p.lmax + 64 > (size_t)ctx->max_smem) {
         cleanup();
         return fail(ctx, BLAMM_ERR_UNSUPPORTED, "too many bins for shared memory");
     }
-    p.cols_per_block = cpb;
-    const int64_t bx = (n + threads - 1) / threads;
-    const int by = (ctx->ncols + cpb - 1) / cpb;
-    e = cudaFuncSetAttribute(score_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem);
-    if (e == cudaSuccess) {
-        score_hist_kernel<<<dim3((unsigned)bx, (unsigned)by), threads, need(cpb), ctx->stream>>>(p);
-        e = cudaGetLastError();
+    p.shared_bins = plain_smem_bytes(4, p.lmax, nbins) <= (size_t)ctx->max_smem ? 1 : 0;
+    if ((rc = launch_plain<true>(ctx, p))) {
+        cleanup();
+        return rc;
     }
     std::vector<unsigned long long> host(nc * nbins);
     if (e == cudaSuccess)
@@ -1755,7 +1754,7 @@ int blamm_scan_device_static(blamm_ctx *ctx, const char *d_bases, int64_t n, con
 
     if (!tc) {
         PlainParams p = plain_params(ctx, seq2, zmask, n, d_run_start, nruns, d_hits, hit_cap, counters + 1);
-        if ((rc = launch_plain(ctx, p))) return rc;
+        if ((rc = launch_plain<false>(ctx, p))) return rc;
         ++launches;
     } else {
         TcParams p = tc_params(ctx, n);
@@ -1855,7 +1854,7 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
     CK(cudaGetLastError());
     if (!tc) {
         PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_run_start, nruns, d_hits, hit_cap, cnt + 1);
-        return launch_plain(ctx, p);
+        return launch_plain<false>(ctx, p);
     }
     if (int rc = check_jobs(ctx, n)) return rc;
     TcParams p = tc_params(ctx, n);

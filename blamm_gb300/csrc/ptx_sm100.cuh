@@ -170,6 +170,13 @@ __device__ __forceinline__ void st_global_v4_if(bool f, void *a, uint32_t x, uin
         : "memory");
 }
 
+__device__ __forceinline__ float4 ld_shared_v4(uint32_t a)
+{
+    float4 v;
+    asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+
 // ---------------------------------------------------------------- hardware barriers
 // A barrier of `threads` threads (whole warps): some arrive and go on, the others wait.
 __device__ __forceinline__ void named_sync(uint32_t id, uint32_t threads)

@@ -152,9 +152,27 @@ __global__ void e16_kernel(const uint32_t *__restrict__ seq2, const uint32_t *__
 }
 
 // ------------------------------------------------------------------------
-// 2. plain FP32 scan: one thread per position, sequential FP32 sums
-//    (the straightforward GPU form of PWMScan::scanThreadBLAS + extractOccurrences)
+// 2. plain FP32 scores: one thread per position, sequential FP32 sums
+//    (the straightforward GPU form of PWMScan::scanThreadBLAS + extractOccurrences),
+//    ending in hits (2a) or in empirical score histograms (2b: Histogram::histThread /
+//    extractObsScore, hist.cpp:70-140)
 // ------------------------------------------------------------------------
+// A block keeps some columns' P in shared memory, four columns side by side, and walks over
+// tiles of 256 positions.  A thread turns the 32 bases from its position on into byte
+// offsets once and uses them for all the columns: a motif position of four columns is one
+// 16-byte load at (offset, column group) and four additions.  The lanes of a warp read at
+// most five different rows of one motif position, which shared memory serves as a broadcast.
+// Row 4 is zero (masked bases), and so are the rows beyond a column's length: adding +0
+// changes no sum that starts at +0.
+// What bounds it: shared memory, which delivers 128 bytes a cycle and SM whatever the lanes
+// share (a 16-byte load of a warp is four cycles): 32 additions a cycle and SM.  2 Mbp x 256
+// columns: 1.01 ms, 0.93 at that rate (one 4-byte load at a byte-coded address, a branch and an
+// addition per motif position: 2.91); 8 Mbp x 64 columns with 250 bins: 1.09 (2.57 with a
+// division per score).
+constexpr int kPlainThreads = 256;
+constexpr int kPlainReg = 32;  // motif positions whose offsets are kept in registers
+constexpr int kPlainRow = 5 * 16;  // bytes of one motif position of four columns
+
 struct PlainParams {
     const uint32_t *seq2;
     const uint32_t *zmask;
@@ -164,16 +182,23 @@ struct PlainParams {
     const float *P;
     int32_t p_rows;
     int32_t ncols;
-    int32_t cols_per_block;
+    int32_t cols_per_block;  // a multiple of 4
     int32_t lmax;
     const int32_t *col_len;
-    const float *thr;
     const int32_t *cols;  // the ncols bank columns to scan (nullptr: columns 0 .. ncols-1)
+    // hits
+    const float *thr;
     void *hits;  // blamm_hit*
     unsigned long long *hit_count;
     int64_t hit_cap;
     int64_t keep_below;  // hits at positions >= keep_below are dropped (0: none are)
     int64_t pos_base;    // added to the positions written
+    // histograms
+    const float *min_score;
+    const float *width;
+    int32_t nbins;
+    int32_t shared_bins;         // 1: the block's counts are in shared memory until it ends
+    unsigned long long *counts;  // ncols x nbins
 };
 
 struct alignas(16) HitRec {
@@ -204,112 +229,133 @@ __device__ __forceinline__ void emit_hits_warp(bool hit, int64_t pos, int32_t co
     }
 }
 
-__global__ void __launch_bounds__(256) scan_plain_kernel(PlainParams p)
+// Shared memory of a block: P, then per column its length and three values (threshold; or least
+// score, bin width and its reciprocal), then the counts of a histogram.
+__host__ __device__ inline size_t plain_smem_bytes(int cols, int lmax, int bins)
 {
-    extern __shared__ __align__(16) uint8_t smem_plain[];
-    const int cpb = p.cols_per_block;
-    float *sP = reinterpret_cast<float *>(smem_plain);
-    int32_t *sLen = reinterpret_cast<int32_t *>(sP + (size_t)cpb * p.p_rows);
-    float *sThr = reinterpret_cast<float *>(sLen + cpb);
-    uint8_t *sCode = reinterpret_cast<uint8_t *>(sThr + cpb);
-
-    const int64_t p0 = (int64_t)blockIdx.x * blockDim.x;
-    const int c0 = blockIdx.y * cpb;
-    const int nc = min(cpb, p.ncols - c0);
-    for (int i = threadIdx.x; i < nc * p.p_rows; i += blockDim.x) {
-        const int cc = i / p.p_rows;
-        const int col = p.cols ? p.cols[c0 + cc] : c0 + cc;
-        sP[i] = p.P[(size_t)col * p.p_rows + (i - cc * p.p_rows)];
-    }
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-        const int col = p.cols ? p.cols[c0 + i] : c0 + i;
-        sLen[i] = p.col_len[col];
-        sThr[i] = p.thr[col];
-    }
-    const int nwin = blockDim.x + p.lmax;
-    for (int i = threadIdx.x; i < nwin; i += blockDim.x)
-        sCode[i] = (uint8_t)base_code_at(p.seq2, p.zmask, p0 + i);
-    __syncthreads();
-
-    const int64_t pos = p0 + threadIdx.x;
-    int64_t rem = 0;
-    if (pos < p.n) rem = run_end_of(p.run_start, p.nruns, p.n, pos) - pos;
-    const uint8_t *code = sCode + threadIdx.x;
-    for (int cc = 0; cc < nc; ++cc) {
-        const int L = sLen[cc];
-        bool hit = false;
-        float s = 0.0f;
-        if (L <= rem) {
-            const float *col = sP + (size_t)cc * p.p_rows;
-            for (int j = 0; j < L; ++j) {
-                int b = code[j];
-                if (b < 4) s = __fadd_rn(s, col[4 * j + b]);
-            }
-            hit = s >= sThr[cc] && (p.keep_below == 0 || pos < p.keep_below);
-        }
-        emit_hits_warp(hit, pos + p.pos_base, p.cols ? p.cols[c0 + cc] : c0 + cc, s,
-                       reinterpret_cast<HitRec *>(p.hits), p.hit_count, p.hit_cap);
-    }
+    return (size_t)(cols / 4) * lmax * kPlainRow + (size_t)cols * 16 + (size_t)cols * bins * 4;
 }
 
-// ------------------------------------------------------------------------
-// 2b. empirical score histograms: the plain scan with a histogram epilogue
-//     (Histogram::histThread / extractObsScore, hist.cpp:70-140)
-// ------------------------------------------------------------------------
-struct HistParams {
-    const uint32_t *seq2;
-    const uint32_t *zmask;
-    int64_t n;
-    const int64_t *run_start;
-    int64_t nruns;
-    const float *P;
-    int32_t p_rows;
-    int32_t ncols;
-    int32_t cols_per_block;
-    int32_t lmax;
-    const int32_t *col_len;
-    const float *min_score;
-    const float *width;
-    int32_t nbins;
-    unsigned long long *counts;  // ncols x nbins
-};
-
-__global__ void __launch_bounds__(256) score_hist_kernel(HistParams p)
+// (int)(x / w) with the division rounded to nearest, as the reference bins a score: from the
+// product with the reciprocal (r) unless that is so near an integer that the two could fall on
+// different sides (relative error of product and quotient below 2^-22 together; r is NaN
+// where the reciprocal would not be that accurate, and then the division decides).
+__device__ __forceinline__ int bin_of(float x, float w, float r)
 {
-    extern __shared__ __align__(16) uint8_t smem_hist[];
-    const int cpb = p.cols_per_block;
-    float *sP = reinterpret_cast<float *>(smem_hist);
-    unsigned int *sH = reinterpret_cast<unsigned int *>(sP + (size_t)cpb * p.p_rows);
-    uint8_t *sCode = reinterpret_cast<uint8_t *>(sH + (size_t)cpb * p.nbins);
-    const int64_t p0 = (int64_t)blockIdx.x * blockDim.x;
+    const float f = __fmul_rn(x, r);
+    const float near = fabsf(__fsub_rn(f, rintf(f)));
+    int b = (int)f;
+    if (!(near > fabsf(f) * 0x1p-21f)) b = (int)__fdiv_rn(x, w);
+    return b;
+}
+
+template <bool kHist>
+__global__ void __launch_bounds__(kPlainThreads) plain_scores_kernel(PlainParams p)
+{
+    extern __shared__ __align__(16) uint8_t smem_plain[];
+    const int cpb = p.cols_per_block, ngrp = cpb / 4, lmax = p.lmax;
+    float *sP = reinterpret_cast<float *>(smem_plain);
+    int32_t *sLen = reinterpret_cast<int32_t *>(smem_plain + (size_t)ngrp * lmax * kPlainRow);
+    float *sA = reinterpret_cast<float *>(sLen + cpb), *sB = sA + cpb, *sR = sB + cpb;
+    uint32_t *sH = reinterpret_cast<uint32_t *>(sR + cpb);
     const int c0 = blockIdx.y * cpb;
     const int nc = min(cpb, p.ncols - c0);
-    for (int i = threadIdx.x; i < nc * p.p_rows; i += blockDim.x) sP[i] = p.P[(size_t)c0 * p.p_rows + i];
-    for (int i = threadIdx.x; i < nc * p.nbins; i += blockDim.x) sH[i] = 0;
-    const int nwin = blockDim.x + p.lmax;
-    for (int i = threadIdx.x; i < nwin; i += blockDim.x)
-        sCode[i] = (uint8_t)base_code_at(p.seq2, p.zmask, p0 + i);
-    __syncthreads();
-    const int64_t pos = p0 + threadIdx.x;
-    int64_t rem = 0;
-    if (pos < p.n) rem = run_end_of(p.run_start, p.nruns, p.n, pos) - pos;
-    const uint8_t *code = sCode + threadIdx.x;
-    for (int cc = 0; cc < nc; ++cc) {
-        const int L = __ldg(p.col_len + c0 + cc);
-        if (L > rem) continue;
-        const float *col = sP + (size_t)cc * p.p_rows;
-        float s = 0.0f;
-        for (int j = 0; j < L; ++j) {
-            const int b = code[j];
-            if (b < 4) s = __fadd_rn(s, col[4 * j + b]);
+    auto bank = [&](int i) { return p.cols ? p.cols[c0 + i] : c0 + i; };
+    for (int i = threadIdx.x; i < cpb; i += kPlainThreads) {
+        const int col = i < nc ? bank(i) : -1;
+        sLen[i] = col < 0 ? 0 : p.col_len[col];
+        sA[i] = col < 0 ? 0.f : kHist ? p.min_score[col] : p.thr[col];
+        if (kHist) {
+            const float w = sB[i] = col < 0 ? 1.f : p.width[col];
+            sR[i] = fabsf(w) > 0x1p-100f && fabsf(w) < 0x1p100f ? __frcp_rn(w) : __int_as_float(0x7fffffff);
         }
-        int bin = (int)__fdiv_rn(__fsub_rn(s, __ldg(p.min_score + c0 + cc)), __ldg(p.width + c0 + cc));
-        bin = max(0, min(p.nbins - 1, bin));
-        atomicAdd(&sH[cc * p.nbins + bin], 1u);
+    }
+    if (kHist && p.shared_bins)
+        for (int i = threadIdx.x; i < cpb * p.nbins; i += kPlainThreads) sH[i] = 0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < cpb * lmax * 5; i += kPlainThreads) {
+        const int c = i / (lmax * 5), r = i - c * (lmax * 5), j = r / 5, b = r - j * 5;
+        const float v = b < 4 && j < sLen[c] ? p.P[(size_t)bank(c) * p.p_rows + 4 * j + b] : 0.f;
+        sP[((size_t)(c / 4) * lmax + j) * 20 + b * 4 + (c & 3)] = v;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nc * p.nbins; i += blockDim.x)
-        if (sH[i]) atomicAdd(&p.counts[(size_t)c0 * p.nbins + i], (unsigned long long)sH[i]);
+    const uint32_t base = ptx::smem_addr(smem_plain);
+    const int64_t ntiles = (p.n + kPlainThreads - 1) / kPlainThreads;
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int64_t pos = tile * kPlainThreads + threadIdx.x;
+        const int64_t end = pos < p.n ? run_end_of(p.run_start, p.nruns, p.n, pos) : pos;
+        const int rem = (int)min(end - pos, (int64_t)kMaxMotifLen);  // bases from here to the run's end
+        // offsets of the 32 bases from pos on (the padded stream covers the reads)
+        uint32_t off[kPlainReg];
+        {
+            const int64_t w = pos >> 4, wz = pos >> 5;
+            const uint32_t s = 2 * (uint32_t)(pos & 15);
+            const uint32_t w0 = __ldg(p.seq2 + w), w1 = __ldg(p.seq2 + w + 1), w2 = __ldg(p.seq2 + w + 2);
+            const uint32_t code[2] = {__funnelshift_r(w0, w1, s), __funnelshift_r(w1, w2, s)};
+            const uint32_t zero = __funnelshift_r(__ldg(p.zmask + wz), __ldg(p.zmask + wz + 1), (uint32_t)(pos & 31));
+#pragma unroll
+            for (int j = 0; j < kPlainReg; ++j) {
+                const uint32_t b = (zero >> j) & 1u ? 4u : (code[j >> 4] >> (2 * (j & 15))) & 3u;
+                off[j] = base + (uint32_t)(j * kPlainRow) + 16u * b;
+            }
+        }
+        for (int g = 0; g < ngrp; ++g) {
+            const int4 len = reinterpret_cast<const int4 *>(sLen)[g];
+            const int L = max(max(len.x, len.y), max(len.z, len.w));
+            const uint32_t at = (uint32_t)(g * lmax * kPlainRow);
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto add = [&](uint32_t a) {
+                const float4 v = ptx::ld_shared_v4(a);
+                s.x = __fadd_rn(s.x, v.x);
+                s.y = __fadd_rn(s.y, v.y);
+                s.z = __fadd_rn(s.z, v.z);
+                s.w = __fadd_rn(s.w, v.w);
+            };
+#pragma unroll
+            for (int j = 0; j < kPlainReg; j += 4) {
+                if (j >= L) break;
+                add(off[j] + at);
+                if (j + 1 < L) add(off[j + 1] + at);
+                if (j + 2 < L) add(off[j + 2] + at);
+                if (j + 3 < L) add(off[j + 3] + at);
+            }
+            for (int j = kPlainReg; j < L; ++j)
+                add(base + at + (uint32_t)(j * kPlainRow) + 16u * (uint32_t)base_code_at(p.seq2, p.zmask, pos + j));
+            const float sc[4] = {s.x, s.y, s.z, s.w};
+            const int ln[4] = {len.x, len.y, len.z, len.w};
+            if (kHist) {
+                const float4 lo = reinterpret_cast<const float4 *>(sA)[g], wd = reinterpret_cast<const float4 *>(sB)[g];
+                const float4 rc = reinterpret_cast<const float4 *>(sR)[g];
+                const float ls[4] = {lo.x, lo.y, lo.z, lo.w}, ws[4] = {wd.x, wd.y, wd.z, wd.w};
+                const float rs[4] = {rc.x, rc.y, rc.z, rc.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (ln[k] == 0 || ln[k] > rem) continue;
+                    const int b = max(0, min(p.nbins - 1, bin_of(__fsub_rn(sc[k], ls[k]), ws[k], rs[k])));
+                    if (p.shared_bins) atomicAdd(&sH[(4 * g + k) * p.nbins + b], 1u);
+                    else atomicAdd(&p.counts[(size_t)(c0 + 4 * g + k) * p.nbins + b], 1ull);
+                }
+            } else {
+                const float4 th = reinterpret_cast<const float4 *>(sA)[g];
+                const float ts[4] = {th.x, th.y, th.z, th.w};
+                const bool keep = p.keep_below == 0 || pos < p.keep_below;
+                bool hit[4], any = false;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) any |= hit[k] = ln[k] > 0 && ln[k] <= rem && sc[k] >= ts[k] && keep;
+                if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        emit_hits_warp(hit[k], pos + p.pos_base, 4 * g + k < nc ? bank(4 * g + k) : 0, sc[k],
+                                       reinterpret_cast<HitRec *>(p.hits), p.hit_count, p.hit_cap);
+                }
+            }
+        }
+    }
+    if (kHist && p.shared_bins) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < nc * p.nbins; i += kPlainThreads)
+            if (sH[i]) atomicAdd(&p.counts[(size_t)c0 * p.nbins + i], (unsigned long long)sH[i]);
+    }
 }
 
 // ------------------------------------------------------------------------
