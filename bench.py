@@ -877,7 +877,7 @@ def run_ours(a, rank, world, local):
     kern_ms = float(np.mean(scan_ms))
     achieved = n * flops_per_bp / (kern_ms / 1e3) / 1e12
     # a step = packing + (one-hot entries + scan) per scan window + rescoring
-    scan_launches = max(1, (launches // a.steps - 2) // 2)
+    scan_launches = max(1, (launches // a.steps - 1) // 2)  # per window: preparation and scan; one rescoring
     traffic = profile_traffic(int(round(n / scan_launches)), terms)
 
     line = {

@@ -53,7 +53,6 @@ struct blamm_ctx {
     std::string err;
     int mode = BLAMM_MODE_AUTO;
     int auto_terms = 1;  // BLAMM_MODE_AUTO: the form in use, 1 or 2 BF16 terms or kE4M3 (1 until tuned)
-    bool plain_timed = false, rescore_timed = false;
     int lower_scores = 0;  // soft-masked bases add their PWM value (simple scan) when 1
     long long wait_limit = 4000000000LL;  // clock64 cycles (about 2 s)
     int debug_stall = 0;                  // test hook: make the scan kernel's first wait run out
@@ -112,8 +111,7 @@ struct blamm_ctx {
     int64_t cand_cap = 0;     // record slots
     blamm_hit *d_hits = nullptr;
     int64_t hits_cap = 0;
-    unsigned long long *d_counters = nullptr;  // [0] candidates, [1] hits
-    int *d_status = nullptr;
+    unsigned long long *d_counters = nullptr;  // record slots, hits, status (bit 0: a wait timed out), candidates
     // hit filtering of one chunk of a pipelined blamm_scan: hits at chunk positions >=
     // keep_below are dropped (0: none), pos_base is added to the positions written
     int64_t keep_below = 0, pos_base = 0;
@@ -493,7 +491,6 @@ int blamm_ctx_create(int device, blamm_ctx **out)
         CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         for (auto &ev : ctx->ev) CK(cudaEventCreate(&ev));
         CK(cudaMalloc(&ctx->d_counters, 4 * sizeof(unsigned long long)));
-        CK(cudaMalloc(&ctx->d_status, sizeof(int)));
         return BLAMM_OK;
     };
     rc = init();
@@ -513,7 +510,7 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     void *bufs[] = {ctx->d_P,      ctx->d_len,   ctx->d_thr,      ctx->d_tiles, ctx->d_abuf,
                     ctx->d_slot_col, ctx->d_slot_thr, ctx->d_prof, ctx->d_bases, ctx->d_seq2, ctx->d_zmask, ctx->d_e16,
-                    ctx->d_runs,   ctx->d_cand,  ctx->d_hits,     ctx->d_counters, ctx->d_status,
+                    ctx->d_runs,   ctx->d_cand,  ctx->d_hits,     ctx->d_counters,
                     ctx->d_active, ctx->d_chunk_bases[0], ctx->d_chunk_bases[1], ctx->d_chunk_runs[0],
                     ctx->d_chunk_runs[1], ctx->d_raw, ctx->d_stream, ctx->d_srun[0], ctx->d_srun[1],
                     ctx->d_srun[2], ctx->d_shdr, ctx->d_ing_tiles, ctx->d_ing_prefix, ctx->d_ing_totals, ctx->d_theo};
@@ -712,29 +709,55 @@ static int ensure_plan(blamm_ctx *ctx)
 }
 
 // The tensor-core scan runs over windows of at most ctx->ewindow positions (16 Mi by
-// default): per window the one-hot entries of its positions (e16_kernel or e8_kernel, 16 B
-// each) and one scan launch, so the entry array holds one window (256 MB) whatever the stream
+// default): per window its packed bases and one-hot entries (prep_kernel, 16 B per entry) and
+// one scan launch, so the entry array holds one window (256 MB) whatever the stream
 // length.  A window's scan copies up to entry (its positions rounded up to 256) + 4 * 64 (BF16)
-// or + 8 * 8 (E4M3), and the entry kernels read up to base i + 3 of the padded stream:
-// entries = positions + kStreamPad - 64 stay inside both.
+// or + 8 * 8 (E4M3): positions + kStreamPad - 64 entries hold that.
 static int64_t e16_entries(const blamm_ctx *ctx, int64_t n) { return std::min(n, ctx->ewindow) + kStreamPad - 64; }
 
-static int launch_pack(blamm_ctx *ctx, const char *d_bases, int64_t n)
+// One launch of prep_kernel: form 0 (packing only), 1 (BF16 entries) or kE4M3.
+static cudaError_t launch_prep(const PrepParams &a, int form, cudaStream_t st)
+{
+    const int64_t span = std::max(a.pack_end - a.base, form ? a.ne : 0);
+    const unsigned grid = (unsigned)((span + kPrepTile - 1) / kPrepTile);
+    if (form == 0) prep_kernel<0><<<grid, kPrepThreads, 0, st>>>(a);
+    else if (form == kE4M3) prep_kernel<8><<<grid, kPrepThreads, 0, st>>>(a);
+    else prep_kernel<1><<<grid, kPrepThreads, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+// Parameters of the preparation of n bases: counts[i] is set to zero where bit i of zero is set.
+static PrepParams prep_params(const blamm_ctx *ctx, const char *d_bases, int64_t n, uint32_t *seq2, uint32_t *zmask,
+                              unsigned long long *counts, uint32_t zero)
+{
+    PrepParams a{};
+    a.bases = d_bases;
+    a.n = n;
+    a.pack_end = (n + kStreamPad + 31) / 32 * 32;
+    a.seq2 = seq2;
+    a.zmask = zmask;
+    a.lower_scores = ctx->lower_scores;
+    a.counts = counts;
+    a.zero = zero;
+    return a;
+}
+
+// Buffers of the packed stream (and one window's entries) for n positions.
+static int ensure_packed(blamm_ctx *ctx, int64_t n, bool entries)
 {
     const int64_t nwords32 = (n + kStreamPad + 31) / 32;
     int rc = ensure(ctx, &ctx->d_seq2, &ctx->cap_words32, (size_t)(2 * nwords32));
-    if (rc) return rc;
-    rc = ensure(ctx, &ctx->d_zmask, &ctx->cap_zmask, (size_t)nwords32);
-    if (rc) return rc;
-    const int threads = 256;
-    const int64_t blocks = (nwords32 + threads - 1) / threads;
-    pack_kernel<<<(unsigned)blocks, threads, 0, ctx->stream>>>(d_bases, n, ctx->d_seq2, ctx->d_zmask,
-                                                               nwords32, ctx->lower_scores);
-    CK(cudaGetLastError());
-    if (ctx->mode != BLAMM_MODE_FP32) {
-        rc = ensure(ctx, &ctx->d_e16, &ctx->cap_e16, (size_t)e16_entries(ctx, n));
-        if (rc) return rc;
-    }
+    if (!rc) rc = ensure(ctx, &ctx->d_zmask, &ctx->cap_zmask, (size_t)nwords32);
+    if (!rc && entries) rc = ensure(ctx, &ctx->d_e16, &ctx->cap_e16, (size_t)e16_entries(ctx, n));
+    return rc;
+}
+
+// Pack n bases into the context's packed stream (no entries).
+static int launch_pack(blamm_ctx *ctx, const char *d_bases, int64_t n, unsigned long long *counts = nullptr,
+                       uint32_t zero = 0)
+{
+    if (int rc = ensure_packed(ctx, n, false)) return rc;
+    CK(launch_prep(prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, counts, zero), 0, ctx->stream));
     return BLAMM_OK;
 }
 
@@ -835,20 +858,23 @@ static void launch_tc(const TcParams &p, bool dump, int grid, uint32_t smem, cud
     else launch_tc_as<false, false, kStream>(p, grid, smem, st);
 }
 
-// The scan of n positions of a packed stream (p: the plan, candidates, counters, status),
-// window by window: the window's one-hot entries into e16, then its scan launch.  Returns the
-// largest grid used; adds the launches to *launches.
-static int launch_tc_windows(blamm_ctx *ctx, TcParams p, const uint32_t *seq2, const uint32_t *zmask, uint4 *e16,
-                             int64_t n, bool dump, int *launches, int *grid_out)
+// The scan of n bases (p: the plan, candidates, counters, status; a: the packed stream and what
+// the first window sets to zero), window by window: the window's packing and one-hot entries
+// (into e16), then its scan launch.  Returns the largest grid used; adds the launches to
+// *launches.
+static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e16, bool dump, int *launches, int *grid_out)
 {
+    const int64_t n = a.n, pack_end = a.pack_end;
     const int64_t nblocks = scan_blocks(n), wb = std::max<int64_t>(1, ctx->ewindow / kBlockPos);
     int gmax = 0;
     for (int64_t b0 = 0; b0 < nblocks; b0 += wb) {
         const int64_t nb = std::min(wb, nblocks - b0), base = b0 * kBlockPos;
-        const int64_t ne = std::min(nb * kBlockPos, n - base) + kStreamPad - 64;
-        if (p.terms == kE4M3) e8_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, ctx->stream>>>(seq2, zmask, base, ne, e16);
-        else e16_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, ctx->stream>>>(seq2, zmask, base, ne, e16);
-        CK(cudaGetLastError());
+        a.base = base;
+        a.pack_end = b0 + nb < nblocks ? base + nb * kBlockPos : pack_end;
+        a.e = e16;
+        a.ne = std::min(nb * kBlockPos, n - base) + kStreamPad - 64;
+        CK(launch_prep(a, p.terms == kE4M3 ? kE4M3 : 1, ctx->stream));
+        a.zero = 0;
         p.e16 = e16;
         p.nblocks = (int32_t)nb;
         p.chunk0 = (uint32_t)(base / 32);
@@ -874,83 +900,6 @@ static int launch_tc_windows(blamm_ctx *ctx, TcParams p, const uint32_t *seq2, c
         if (launches) *launches += 2;
     }
     if (grid_out) *grid_out = gmax;
-    return BLAMM_OK;
-}
-
-// tcgen05 scan + rescoring; candidates buffer grows (and the scan re-runs) on overflow
-static int run_tc(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t nruns, blamm_hit *d_hits,
-                  int64_t hit_cap, float *dump, int64_t dump_p0, int64_t dump_npos, int *launches)
-{
-    int rc = ensure_plan(ctx);
-    if (rc) return rc;
-    if ((rc = check_jobs(ctx, n))) return rc;
-    if (ctx->cand_cap == 0 && (rc = ensure_cand(ctx, record_slots_guess(ctx, n)))) return rc;
-    const bool any = n > 0 && ctx->ntiles > 0;
-    for (int attempt = 0; attempt < 3; ++attempt) {
-        CK(cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
-        CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
-        TcParams p = tc_params(ctx, n);
-        p.cand = ctx->d_cand;
-        p.cand_count = ctx->d_counters;
-        p.cand_cap = ctx->cand_cap;
-        p.status = ctx->d_status;
-        p.wait_limit = ctx->wait_limit;
-        p.debug_stall = ctx->debug_stall;
-        p.dump = dump;
-        p.dump_p0 = dump_p0;
-        p.dump_npos = dump_npos;
-        p.dump_ncols = ctx->ncols;
-        p.prof = nullptr;
-        if (ctx->prof_on) {
-            if (!ctx->d_prof) CK(cudaMalloc(&ctx->d_prof, sizeof(long long) * 32 * ctx->sm_count));
-            CK(cudaMemsetAsync(ctx->d_prof, 0, sizeof(long long) * 32 * ctx->sm_count, ctx->stream));
-            p.prof = ctx->d_prof;
-        }
-        int grid = 0;
-        if (any) {
-            CK(cudaEventRecord(ctx->ev[4], ctx->stream));
-            if ((rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, dump != nullptr, launches,
-                                        &grid)))
-                return rc;
-            CK(cudaEventRecord(ctx->ev[5], ctx->stream));
-        }
-        unsigned long long ncand = 0;
-        int status = 0;
-        CK(cudaMemcpyAsync(&ncand, ctx->d_counters, sizeof ncand, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof status, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (status) return fail(ctx, BLAMM_ERR_TIMEOUT, "scan kernel: a device wait timed out");
-        if (any) cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[4], ctx->ev[5]);
-        if (ctx->prof_on && any) {
-            ctx->prof.resize((size_t)32 * grid);
-            CK(cudaMemcpy(ctx->prof.data(), ctx->d_prof, sizeof(long long) * 32 * grid, cudaMemcpyDeviceToHost));
-            ctx->prof_ctas = grid;
-        }
-        ctx->stats.candidates = 0;  // counted by the rescoring
-        ctx->rec_slots = (int64_t)ncand;
-        if ((int64_t)ncand <= ctx->cand_cap) break;
-        // grow and re-run
-        if ((int64_t)ncand >= kMaxRecordSlots)
-            return fail(ctx, BLAMM_ERR_OVERFLOW, "%llu candidate records exceed one launch's %lld", ncand,
-                        (long long)kMaxRecordSlots);
-        rc = ensure_cand(ctx, std::min<int64_t>((int64_t)(ncand + ncand / 4 + 1024), kMaxRecordSlots));
-        if (rc) return rc;
-        if (attempt == 2) return fail(ctx, BLAMM_ERR_OVERFLOW, "candidate buffer overflow");
-    }
-    const RescoreParams r = rescore_params(ctx, ctx->d_cand, ctx->d_counters, ctx->cand_cap,
-                                           ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits,
-                                           ctx->d_counters + 1, hit_cap, ctx->d_counters + 3);
-    const int64_t nc = ctx->rec_slots;
-    if (nc > 0) {
-        const int threads = kRescoreThreads;
-        const int64_t blocks = std::min<int64_t>((nc + threads - 1) / threads, (int64_t)ctx->sm_count * 16);
-        CK(cudaEventRecord(ctx->ev[6], ctx->stream));
-        rescore_kernel<<<(unsigned)blocks, threads, 0, ctx->stream>>>(r);
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(ctx->ev[7], ctx->stream));
-        ctx->rescore_timed = true;
-        ++*launches;
-    }
     return BLAMM_OK;
 }
 
@@ -1003,56 +952,109 @@ static int launch_plain(blamm_ctx *ctx, PlainParams &p)
     return BLAMM_OK;
 }
 
-static int run_plain(blamm_ctx *ctx, int64_t n, const int64_t *d_runs, int64_t nruns, blamm_hit *d_hits,
-                     int64_t hit_cap, int *launches)
+// Rescoring behind the scan: the number of record slots is only known on the device, so the
+// grid covers what the scan's warps reserve at least and the usual number of candidates.
+static int launch_rescore(blamm_ctx *ctx, const RescoreParams &r, int64_t n, int scan_grid)
 {
-    CK(cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
-    PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits, hit_cap,
-                                 ctx->d_counters + 1);
-    if (n == 0) return BLAMM_OK;
-    CK(cudaEventRecord(ctx->ev[4], ctx->stream));
-    const int rc = launch_plain<false>(ctx, p);
-    if (rc) return rc;
-    CK(cudaEventRecord(ctx->ev[5], ctx->stream));
-    ctx->plain_timed = true;
-    ++*launches;
+    const int64_t slots = (int64_t)((double)n * scanned_columns(ctx) / 1000.0) + record_slots_reserved(scan_grid);
+    const int64_t blocks = std::min<int64_t>((slots + kRescoreThreads - 1) / kRescoreThreads, (int64_t)ctx->sm_count * 16);
+    rescore_kernel<<<(unsigned)std::max<int64_t>(blocks, 1), kRescoreThreads, 0, ctx->stream>>>(r);
+    CK(cudaGetLastError());
     return BLAMM_OK;
 }
 
+// Raw accumulators of some positions (the raw-score hook).
+struct ScanDump {
+    float *out = nullptr;
+    int64_t p0 = 0, npos = 0;
+};
+
+// One scan of device-resident bases, its counters back on the host: preparation, scan and
+// rescoring are enqueued one behind the other and the host waits once (a candidate buffer that
+// was too small grows and the scan runs again).
 static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t *d_runs, int64_t nruns,
-                     blamm_hit *d_hits, int64_t hit_cap, int64_t *n_hits)
+                     blamm_hit *d_hits, int64_t hit_cap, int64_t *n_hits, const ScanDump &dump = ScanDump())
 {
     if (ctx->ncols == 0) return fail(ctx, BLAMM_ERR_STATE, "blamm_set_motifs was not called");
-    int launches = 0;
+    const bool tc = ctx->mode != BLAMM_MODE_FP32;
+    unsigned long long *cnt = ctx->d_counters;  // record slots, hits, status, candidates
     ctx->stats = blamm_stats{};
-    ctx->plain_timed = ctx->rescore_timed = false;
     ctx->stats.positions = n;
     ctx->stats.columns = scanned_columns(ctx);
-    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
-    int rc = launch_pack(ctx, d_bases, n);
-    if (rc) return rc;
-    launches += 1;  // packing (the tensor-core scan adds its windows' one-hot entries)
-    if (ctx->mode == BLAMM_MODE_FP32) rc = run_plain(ctx, n, d_runs, nruns, d_hits, hit_cap, &launches);
-    else rc = run_tc(ctx, n, d_runs, nruns, d_hits, hit_cap, nullptr, 0, 0, &launches);
-    if (rc) return rc;
-    CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    unsigned long long cnt[4] = {0, 0, 0, 0};  // record slots, hits, -, candidates
-    CK(cudaMemcpyAsync(cnt, ctx->d_counters, sizeof cnt, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    const unsigned long long nh = cnt[1];
-    if (ctx->mode != BLAMM_MODE_FP32) ctx->stats.candidates = (int64_t)cnt[3];
-    float ms = 0.0f;
-    cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
-    ctx->stats.kernel_ms = ms;
-    if (ctx->plain_timed) cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[4], ctx->ev[5]);
-    if (ctx->rescore_timed) cudaEventElapsedTime(&ctx->stats.rescore_ms, ctx->ev[6], ctx->ev[7]);
-    ctx->stats.hits = (int64_t)nh;
-    ctx->stats.tiles = (int32_t)(ctx->mode == BLAMM_MODE_FP32 ? 0 : ctx->ntiles);
+    int rc = BLAMM_OK;
+    if (tc) {
+        if ((rc = ensure_plan(ctx)) || (rc = check_jobs(ctx, n))) return rc;
+        if (ctx->cand_cap == 0 && (rc = ensure_cand(ctx, record_slots_guess(ctx, n)))) return rc;
+    }
+    if ((rc = ensure_packed(ctx, n, tc))) return rc;
+    unsigned long long got[4] = {0, 0, 0, 0};
+    int launches = 0;
+    for (int attempt = 0;; ++attempt) {
+        launches = 0;
+        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+        if (tc) {
+            TcParams p = tc_params(ctx, n);
+            p.cand = ctx->d_cand;
+            p.cand_count = cnt;
+            p.cand_cap = ctx->cand_cap;
+            p.status = reinterpret_cast<int *>(cnt + 2);
+            p.debug_stall = ctx->debug_stall;
+            p.dump = dump.out;
+            p.dump_p0 = dump.p0;
+            p.dump_npos = dump.npos;
+            if (ctx->prof_on) {
+                if (!ctx->d_prof) CK(cudaMalloc(&ctx->d_prof, sizeof(long long) * 32 * ctx->sm_count));
+                CK(cudaMemsetAsync(ctx->d_prof, 0, sizeof(long long) * 32 * ctx->sm_count, ctx->stream));
+                p.prof = ctx->d_prof;
+            }
+            int grid = 0;
+            const PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 15u);
+            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out != nullptr, &launches, &grid))) return rc;
+            CK(cudaEventRecord(ctx->ev[5], ctx->stream));
+            const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
+                                                   d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
+            if ((rc = launch_rescore(ctx, r, n, grid))) return rc;
+            ctx->prof_ctas = ctx->prof_on ? grid : ctx->prof_ctas;
+        } else {
+            if ((rc = launch_pack(ctx, d_bases, n, cnt, 15u))) return rc;
+            CK(cudaEventRecord(ctx->ev[5], ctx->stream));
+            PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits, hit_cap, cnt + 1);
+            if ((rc = launch_plain<false>(ctx, p))) return rc;
+            ++launches;  // (packing)
+        }
+        ++launches;
+        CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+        CK(cudaMemcpyAsync(got, cnt, sizeof got, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if ((int)got[2]) return fail(ctx, BLAMM_ERR_TIMEOUT, "scan kernel: a device wait timed out");
+        ctx->rec_slots = (int64_t)got[0];
+        if (!tc || (int64_t)got[0] <= ctx->cand_cap) break;
+        if ((int64_t)got[0] >= kMaxRecordSlots)
+            return fail(ctx, BLAMM_ERR_OVERFLOW, "%llu candidate records exceed one launch's %lld", got[0],
+                        (long long)kMaxRecordSlots);
+        if (attempt == 2) return fail(ctx, BLAMM_ERR_OVERFLOW, "candidate buffer overflow");
+        rc = ensure_cand(ctx, std::min<int64_t>((int64_t)(got[0] + got[0] / 4 + 1024), kMaxRecordSlots));
+        if (rc) return rc;
+    }
+    if (tc && ctx->prof_on) {
+        ctx->prof.resize((size_t)32 * ctx->prof_ctas);
+        CK(cudaMemcpy(ctx->prof.data(), ctx->d_prof, sizeof(long long) * 32 * ctx->prof_ctas, cudaMemcpyDeviceToHost));
+    }
+    const int64_t nh = (int64_t)got[1];
+    if (tc) ctx->stats.candidates = (int64_t)got[3];
+    cudaEventElapsedTime(&ctx->stats.kernel_ms, ctx->ev[1], ctx->ev[2]);
+    if (tc) {
+        cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[1], ctx->ev[5]);
+        cudaEventElapsedTime(&ctx->stats.rescore_ms, ctx->ev[5], ctx->ev[2]);
+    } else {
+        cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[5], ctx->ev[2]);
+    }
+    ctx->stats.hits = nh;
+    ctx->stats.tiles = (int32_t)(tc ? ctx->ntiles : 0);
     ctx->stats.launches = launches;
-    *n_hits = (int64_t)nh;
-    return (int64_t)nh > hit_cap ? fail(ctx, BLAMM_ERR_OVERFLOW, "%lld hits > capacity %lld",
-                                        (long long)nh, (long long)hit_cap)
-                                 : BLAMM_OK;
+    *n_hits = nh;
+    return nh > hit_cap ? fail(ctx, BLAMM_ERR_OVERFLOW, "%lld hits > capacity %lld", (long long)nh, (long long)hit_cap)
+                        : BLAMM_OK;
 }
 
 extern "C" {
@@ -1168,32 +1170,24 @@ static int scan_host_pipelined_steps(blamm_ctx *ctx, const char *bases, int64_t 
 static int enqueue_chunk(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t *d_runs, int64_t nruns,
                          blamm_hit *d_hits, int64_t hit_cap)
 {
-    unsigned long long *cnt = ctx->d_counters;  // [0] candidates of this chunk, [1] hits of the call
-    const int64_t nwords32 = (n + kStreamPad + 31) / 32;
-    pack_kernel<<<(unsigned)((nwords32 + 255) / 256), 256, 0, ctx->stream>>>(d_bases, n, ctx->d_seq2, ctx->d_zmask,
-                                                                          nwords32, ctx->lower_scores);
-    CK(cudaGetLastError());
+    unsigned long long *cnt = ctx->d_counters;  // [0] record slots and [3] candidates of this chunk, [1] hits of the call
     if (ctx->mode == BLAMM_MODE_FP32) {
+        if (int rc = launch_pack(ctx, d_bases, n)) return rc;
         PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits, hit_cap, cnt + 1);
         return launch_plain<false>(ctx, p);
     }
-    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), ctx->stream));      // record slots of this chunk
-    CK(cudaMemsetAsync(cnt + 3, 0, sizeof(unsigned long long), ctx->stream));  // its candidates
     int rc = check_jobs(ctx, n);
     if (rc) return rc;
     TcParams p = tc_params(ctx, n);
     p.cand = ctx->d_cand;
     p.cand_count = cnt;
     p.cand_cap = ctx->cand_cap;
-    p.status = ctx->d_status;
-    p.wait_limit = ctx->wait_limit;
-    p.dump_ncols = ctx->ncols;
-    if ((rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, false, nullptr, nullptr))) return rc;
-    const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask,
-                                           n, d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
-    rescore_kernel<<<(unsigned)(ctx->sm_count * 8), kRescoreThreads, 0, ctx->stream>>>(r);
-    CK(cudaGetLastError());
-    return BLAMM_OK;
+    p.status = reinterpret_cast<int *>(cnt + 2);
+    int grid = 0;
+    const PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 9u);
+    if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, false, nullptr, &grid))) return rc;
+    return launch_rescore(ctx, rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n, d_runs,
+                                              nruns, d_hits, cnt + 1, hit_cap, cnt + 3), n, grid);
 }
 
 // The copy pipeline without host synchronisation inside a chunk: the host only waits for
@@ -1214,12 +1208,9 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         if ((rc = ensure(ctx, &ctx->d_chunk_bases[b], &ctx->cap_chunk_bases[b], (size_t)span))) return rc;
         if ((rc = ensure(ctx, &ctx->d_chunk_runs[b], &ctx->cap_chunk_runs[b], (size_t)nruns + 1))) return rc;
     }
-    const int64_t nwords32 = (span + kStreamPad + 31) / 32;
-    if ((rc = ensure(ctx, &ctx->d_seq2, &ctx->cap_words32, (size_t)(2 * nwords32)))) return rc;
-    if ((rc = ensure(ctx, &ctx->d_zmask, &ctx->cap_zmask, (size_t)nwords32))) return rc;
+    if ((rc = ensure_packed(ctx, span, tc))) return rc;
     if (tc) {
         if ((rc = ensure_plan(ctx))) return rc;
-        if ((rc = ensure(ctx, &ctx->d_e16, &ctx->cap_e16, (size_t)e16_entries(ctx, span)))) return rc;
         // candidates: four times the usual first guess for a chunk (a chunk that still
         // overflows sends the whole call to the synchronous path)
         const double want = (double)record_slots_guess(ctx, span, 250.0);
@@ -1251,7 +1242,6 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         ctx->cap_h_chunk_counts = (size_t)(4 * nchunks);
     }
     CK(cudaMemsetAsync(ctx->d_counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
-    CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));  // the buffers exist before the copy stream uses them
     int64_t kruns[2] = {0, 0};
     auto issue_in = [&](int64_t k) -> int {
@@ -1308,7 +1298,6 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         // host memory
         CK(cudaMemcpyAsync(hc_k + 4 * k, ctx->d_counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                            ctx->stream));
-        CK(cudaMemcpyAsync(hc_k + 4 * k + 2, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaEventRecord(ctx->done_ev[b], ctx->stream));
         if (k >= 1 && (rc = drain_out(k - 1))) return rc;
     }
@@ -1320,9 +1309,9 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
     total.columns = scanned_columns(ctx);
     total.tiles = (int32_t)(tc ? ctx->ntiles : 0);
     total.launches = 0;
-    for (int64_t k = 0; k < nchunks; ++k) {  // packing + scan (+ rescoring and a one-hot build per window)
+    for (int64_t k = 0; k < nchunks; ++k) {  // preparation and scan (per window), rescoring
         const int64_t len = std::min(n, (k + 1) * kPipeChunk + ov) - k * kPipeChunk;
-        total.launches += (int32_t)(tc ? 2 + 2 * ((len + ctx->ewindow - 1) / ctx->ewindow) : 2);
+        total.launches += (int32_t)(tc ? 1 + 2 * ((len + ctx->ewindow - 1) / ctx->ewindow) : 2);
     }
     int status = 0;
     for (int64_t k = 0; k < nchunks; ++k) {
@@ -1622,8 +1611,6 @@ int blamm_debug_scores(blamm_ctx *ctx, const char *bases, int64_t n, int64_t p0,
     int rc = ensure(ctx, &ctx->d_bases, &ctx->cap_bases, (size_t)n);
     if (rc) return rc;
     CK(cudaMemcpyAsync(ctx->d_bases, bases, (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-    rc = launch_pack(ctx, ctx->d_bases, n);
-    if (rc) return rc;
     int64_t runs0 = 0;
     rc = ensure(ctx, &ctx->d_runs, &ctx->cap_runs, 1);
     if (rc) return rc;
@@ -1631,12 +1618,9 @@ int blamm_debug_scores(blamm_ctx *ctx, const char *bases, int64_t n, int64_t p0,
     float *d_dump = nullptr;
     CK(cudaMalloc(&d_dump, sizeof(float) * (size_t)npos * ctx->ncols));
     CK(cudaMemsetAsync(d_dump, 0, sizeof(float) * (size_t)npos * ctx->ncols, ctx->stream));
-    int launches = 0;
-    size_t hc = (size_t)ctx->hits_cap;
-    rc = ensure(ctx, &ctx->d_hits, &hc, 1);
-    if (rc) { cudaFree(d_dump); return rc; }
-    ctx->hits_cap = (int64_t)hc;
-    rc = run_tc(ctx, n, ctx->d_runs, 1, ctx->d_hits, 0, d_dump, p0, npos, &launches);
+    int64_t nh = 0;
+    rc = scan_core(ctx, ctx->d_bases, n, ctx->d_runs, 1, nullptr, 0, &nh, ScanDump{d_dump, p0, npos});
+    if (rc == BLAMM_ERR_OVERFLOW && nh > 0) rc = BLAMM_OK;  // (no room for hits was given)
     if (rc == BLAMM_OK) {
         cudaError_t e = cudaMemcpyAsync(out, d_dump, sizeof(float) * (size_t)npos * ctx->ncols,
                                         cudaMemcpyDeviceToHost, ctx->stream);
@@ -1677,8 +1661,7 @@ constexpr size_t kStaticZmaskOff = round256(kStaticSeq2Off + sizeof(uint32_t) * 
 constexpr size_t kStaticE16Off = round256(kStaticZmaskOff + sizeof(uint32_t) * kStaticWords32);
 constexpr size_t kStaticCandOff = round256(kStaticE16Off + sizeof(uint4) * (kStaticMaxBases + kStreamPad));
 constexpr size_t kStaticCountOff = round256(kStaticCandOff + sizeof(uint4) * (kStaticCandCap + kRecBlock));
-constexpr size_t kStaticStatusOff = round256(kStaticCountOff + sizeof(unsigned long long) * 4);
-constexpr size_t kStaticBytes = round256(kStaticStatusOff + sizeof(int));  // about 97 MiB
+constexpr size_t kStaticBytes = round256(kStaticCountOff + sizeof(unsigned long long) * 4);  // about 97 MiB
 
 constexpr int kStaticMaxDevices = 64;
 
@@ -1737,58 +1720,39 @@ int blamm_scan_device_static(blamm_ctx *ctx, const char *d_bases, int64_t n, con
     uint4 *e16 = reinterpret_cast<uint4 *>(base + kStaticE16Off);
     uint4 *cand = reinterpret_cast<uint4 *>(base + kStaticCandOff);
     unsigned long long *counters = reinterpret_cast<unsigned long long *>(base + kStaticCountOff);
-    int *status = reinterpret_cast<int *>(base + kStaticStatusOff);
 
     ctx->stats = blamm_stats{};
     ctx->stats.positions = n;
     ctx->stats.columns = scanned_columns(ctx);
     int launches = 0;
-    // the counters (candidates, hits) and the status word start at zero on every call
-    CK(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
-    CK(cudaMemsetAsync(status, 0, sizeof(int), ctx->stream));
-    const int64_t nwords32 = (n + kStreamPad + 31) / 32;
-    pack_kernel<<<(unsigned)((nwords32 + 255) / 256), 256, 0, ctx->stream>>>(d_bases, n, seq2, zmask, nwords32,
-                                                                          ctx->lower_scores);
-    CK(cudaGetLastError());
-    ++launches;
-
+    // (the preparation sets the counters and the status word to zero)
+    const PrepParams a = prep_params(ctx, d_bases, n, seq2, zmask, counters, 15u);
     if (!tc) {
+        CK(launch_prep(a, 0, ctx->stream));
         PlainParams p = plain_params(ctx, seq2, zmask, n, d_run_start, nruns, d_hits, hit_cap, counters + 1);
         if ((rc = launch_plain<false>(ctx, p))) return rc;
-        ++launches;
+        launches = 2;
     } else {
         TcParams p = tc_params(ctx, n);
         p.cand = cand;
         p.cand_count = counters;
         p.cand_cap = kStaticCandCap;
-        p.status = status;
-        p.wait_limit = ctx->wait_limit;
-        p.dump_ncols = ctx->ncols;
-        if ((rc = launch_tc_windows(ctx, p, seq2, zmask, e16, n, false, &launches, nullptr))) return rc;
-        unsigned long long ncand = 0;
-        int st = 0;
-        CK(cudaMemcpyAsync(&ncand, counters, sizeof ncand, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaMemcpyAsync(&st, status, sizeof st, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (st) return fail(ctx, BLAMM_ERR_TIMEOUT, "scan kernel: a device wait timed out");
-        if ((int64_t)ncand > kStaticCandCap)
-            return fail(ctx, BLAMM_ERR_OVERFLOW,
-                        "blamm_scan_device_static: %llu candidate record slots > the static limit %lld (scan "
-                        "fewer positions per call)", ncand, (long long)kStaticCandCap);
-        if (ncand > 0) {
-            const RescoreParams r = rescore_params(ctx, cand, counters, kStaticCandCap, seq2, zmask, n,
-                                                   d_run_start, nruns, d_hits, counters + 1, hit_cap, counters + 3);
-            const int threads = kRescoreThreads;
-            const int64_t blocks = std::min<int64_t>(((int64_t)ncand + threads - 1) / threads,
-                                                     (int64_t)ctx->sm_count * 16);
-            rescore_kernel<<<(unsigned)blocks, threads, 0, ctx->stream>>>(r);
-            CK(cudaGetLastError());
-            ++launches;
-        }
+        p.status = reinterpret_cast<int *>(counters + 2);
+        int grid = 0;
+        if ((rc = launch_tc_windows(ctx, p, a, e16, false, &launches, &grid))) return rc;
+        const RescoreParams r = rescore_params(ctx, cand, counters, kStaticCandCap, seq2, zmask, n, d_run_start, nruns,
+                                               d_hits, counters + 1, hit_cap, counters + 3);
+        if ((rc = launch_rescore(ctx, r, n, grid))) return rc;
+        ++launches;
     }
-    unsigned long long cnt[4] = {0, 0, 0, 0};  // record slots, hits, -, candidates
+    unsigned long long cnt[4] = {0, 0, 0, 0};  // record slots, hits, status, candidates
     CK(cudaMemcpyAsync(cnt, counters, sizeof cnt, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    if ((int)cnt[2]) return fail(ctx, BLAMM_ERR_TIMEOUT, "scan kernel: a device wait timed out");
+    if (tc && (int64_t)cnt[0] > kStaticCandCap)
+        return fail(ctx, BLAMM_ERR_OVERFLOW,
+                    "blamm_scan_device_static: %llu candidate record slots > the static limit %lld (scan "
+                    "fewer positions per call)", cnt[0], (long long)kStaticCandCap);
     const unsigned long long nh = cnt[1];
     if (tc) ctx->stats.candidates = (int64_t)cnt[3];
     ctx->stats.hits = (int64_t)nh;
@@ -1812,13 +1776,10 @@ int blamm_reserve(blamm_ctx *ctx, int64_t max_positions, int64_t max_candidates)
     if (!ctx || max_positions < 0 || max_candidates < 0) return BLAMM_ERR_ARG;
     if (ctx->ncols == 0) return fail(ctx, BLAMM_ERR_STATE, "blamm_set_motifs was not called");
     CK(cudaSetDevice(ctx->device));
-    const int64_t nwords32 = (max_positions + kStreamPad + 31) / 32;
-    int rc = ensure(ctx, &ctx->d_seq2, &ctx->cap_words32, (size_t)(2 * nwords32));
-    if (!rc) rc = ensure(ctx, &ctx->d_zmask, &ctx->cap_zmask, (size_t)nwords32);
+    int rc = ensure_packed(ctx, max_positions, ctx->mode != BLAMM_MODE_FP32);
     if (rc) return rc;
     if (ctx->mode != BLAMM_MODE_FP32) {
         if ((rc = ensure_plan(ctx))) return rc;
-        if ((rc = ensure(ctx, &ctx->d_e16, &ctx->cap_e16, (size_t)e16_entries(ctx, max_positions)))) return rc;
         // record slots: at most one record per candidate, plus the blocks the warps reserve
         const int64_t slots = std::min(max_candidates + record_slots_reserved(ctx->sm_count), kMaxRecordSlots);
         if ((rc = ensure_cand(ctx, slots))) return rc;
@@ -1846,13 +1807,14 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
     if (n > 0 && (!d_bases || !d_run_start || nruns <= 0 || (hit_cap > 0 && !d_hits)))
         return fail(ctx, BLAMM_ERR_ARG, "null buffer");
     CK(cudaSetDevice(ctx->device));
-    CK(cudaMemsetAsync(d_counts, 0, 4 * sizeof(uint64_t), ctx->stream));
-    if (n == 0) return BLAMM_OK;
+    if (n == 0) {
+        CK(cudaMemsetAsync(d_counts, 0, 4 * sizeof(uint64_t), ctx->stream));
+        return BLAMM_OK;
+    }
     unsigned long long *cnt = reinterpret_cast<unsigned long long *>(d_counts);
-    pack_kernel<<<(unsigned)((nwords32 + 255) / 256), 256, 0, ctx->stream>>>(d_bases, n, ctx->d_seq2, ctx->d_zmask,
-                                                                          nwords32, ctx->lower_scores);
-    CK(cudaGetLastError());
+    const PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 15u);
     if (!tc) {
+        CK(launch_prep(a, 0, ctx->stream));
         PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_run_start, nruns, d_hits, hit_cap, cnt + 1);
         return launch_plain<false>(ctx, p);
     }
@@ -1862,16 +1824,10 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
     p.cand_count = cnt;
     p.cand_cap = ctx->cand_cap;
     p.status = reinterpret_cast<int *>(cnt + 2);
-    p.wait_limit = ctx->wait_limit;
-    p.dump_ncols = ctx->ncols;
-    if (int rc = launch_tc_windows(ctx, p, ctx->d_seq2, ctx->d_zmask, ctx->d_e16, n, false, nullptr, nullptr))
-        return rc;
-    const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask,
-                                           n, d_run_start, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
-    // a fixed grid: the candidate count is only known on the device
-    rescore_kernel<<<(unsigned)(ctx->sm_count * 8), kRescoreThreads, 0, ctx->stream>>>(r);
-    CK(cudaGetLastError());
-    return BLAMM_OK;
+    int grid = 0;
+    if (int rc = launch_tc_windows(ctx, p, a, ctx->d_e16, false, nullptr, &grid)) return rc;
+    return launch_rescore(ctx, rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
+                                              d_run_start, nruns, d_hits, cnt + 1, hit_cap, cnt + 3), n, grid);
 }
 
 int blamm_scan_graph_create(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t *d_run_start,

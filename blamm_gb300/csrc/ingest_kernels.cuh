@@ -24,6 +24,8 @@
 #pragma once
 #include <cstdint>
 
+#include "scan_kernels.cuh"
+
 namespace blamm {
 
 constexpr int kIngThreads = 256;
@@ -79,24 +81,10 @@ struct IngMasks {
     uint64_t b1, b2;  // bits 1 and 2 of the characters: A 0 0, C 1 0, G 1 1, T 0 1
 };
 
-// 0x80 in every byte of x that is zero (exact, no borrow between bytes)
-__device__ __forceinline__ uint32_t ing_zero_bytes(uint32_t x)
-{
-    return ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);
-}
-
 // The 0x80 bits of two words' bytes as 8 mask bits at bit 7 (dot products with the bits' weights)
 __device__ __forceinline__ uint32_t ing_bits(uint32_t lo, uint32_t hi)
 {
     return __dp4a(hi, 0x80402010u, __dp4a(lo, 0x08040201u, 0u));
-}
-
-// 0x80 in every byte that is one of ACGTacgt: bits 1-2 of a base name the only letter it can be
-__device__ __forceinline__ uint32_t ing_base_bytes(uint32_t x)
-{
-    const uint32_t c = (x >> 1) & 0x03030303u;          // A 0, C 1, T 2, G 3
-    const uint32_t t = (c | c >> 4) & 0x00ff00ffu;      // two nibbles per 16 bits
-    return ing_zero_bytes((x & 0xDFDFDFDFu) ^ __byte_perm(0x47544341u, 0u, t | t >> 8));
 }
 
 __device__ __forceinline__ void ing_load(const char *raw, int64_t n, int64_t at, bool vec, uint32_t (&w)[16])
@@ -134,8 +122,8 @@ __device__ __forceinline__ IngMasks ing_masks(const uint32_t (&w)[16])
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const uint32_t x = w[8 * h + 2 * k], y = w[8 * h + 2 * k + 1];
-            nl[h] |= (ing_bits(ing_zero_bytes(x ^ 0x0A0A0A0Au), ing_zero_bytes(y ^ 0x0A0A0A0Au)) >> 7) << (8 * k);
-            base[h] |= (ing_bits(ing_base_bytes(x), ing_base_bytes(y)) >> 7) << (8 * k);
+            nl[h] |= (ing_bits(zero_bytes(x ^ 0x0A0A0A0Au), zero_bytes(y ^ 0x0A0A0A0Au)) >> 7) << (8 * k);
+            base[h] |= (ing_bits(base_bytes(x), base_bytes(y)) >> 7) << (8 * k);
             if (kCodes) {
                 b1[h] |= (ing_bits((x << 6) & 0x80808080u, (y << 6) & 0x80808080u) >> 7) << (8 * k);
                 b2[h] |= (ing_bits((x << 5) & 0x80808080u, (y << 5) & 0x80808080u) >> 7) << (8 * k);

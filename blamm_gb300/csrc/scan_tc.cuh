@@ -2,7 +2,7 @@
 // one persistent CTA per SM.
 //
 // Score of motif column c at position p:  sum_j P(4j + base(p+j), c).
-// After packing, e16_kernel writes one 16-byte entry per stream position of a
+// prep_kernel packs the stream and writes one 16-byte entry per position of a
 // window of at most 16 Mi positions (the scan runs once per window, so the entry
 // array stays 256 MB whatever the stream length),
 // E[i] = onehot(base i) ++ onehot(base i+1) (2 bases x 4 channels x bf16).
