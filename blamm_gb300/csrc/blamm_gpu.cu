@@ -23,6 +23,7 @@
 #include "scan_tc.cuh"
 #include "hist_kernels.cuh"
 #include "ingest_kernels.cuh"
+#include "plan_kernels.cuh"
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -76,7 +77,6 @@ struct blamm_ctx {
     bool plan_valid = false;
     int ntiles = 0;
     std::vector<TileDesc> tiles;  // ntiles + 1: the last one holds the end offset
-    std::vector<float> guard;    // per column
     int erows = 0;               // one-hot entries per E stage
     int plan_tg = 1;             // most tiles per group whose A fits in shared memory (evened out)
     bool plan_stream = false;    // not even one tile fits: A is streamed
@@ -85,6 +85,7 @@ struct blamm_ctx {
     int32_t *d_slot_col = nullptr;
     float *d_slot_thr = nullptr;
     size_t cap_tiles = 0, cap_abuf = 0, cap_slot_col = 0, cap_slot_thr = 0;
+    std::vector<int32_t> slot_col;  // (the upload's source)
     // per-column fixed-point BF16 terms and guard bands of the bank (for colq_terms terms)
     bool colq_valid = false;
     int colq_terms = 0;
@@ -93,6 +94,8 @@ struct blamm_ctx {
     std::vector<uint32_t> colq_off;  // column c's 4L values start at colq_off[c]
     std::vector<uint16_t> colq_hi, colq_lo;
     std::vector<uint8_t> colq_e8;  // E4M3 codes of P(c) x 2^colq_k[c] (the E4M3 form)
+    uint8_t *d_colq = nullptr;     // on the device: guards, exponents, offsets, terms (colq_at: their places)
+    size_t cap_colq = 0, colq_at[5] = {0, 0, 0, 0, 0};
     // planner knobs: widest tile (columns beyond a tile's 128 rows have no effect) and the
     // fixed cycles per job (kept for callers that set and read it; no plan depends on it)
     int plan_nmax = 256;
@@ -274,18 +277,37 @@ inline int64_t e4m3_units(uint8_t code)
 
 }  // namespace
 
+// The quantised bank on the device.
+static int upload_colq(blamm_ctx *ctx)
+{
+    const size_t nc = (size_t)ctx->ncols;
+    const void *src[5] = {ctx->colq_guard.data(), ctx->colq_k.data(), ctx->colq_off.data(),
+                          ctx->colq_e8.empty() ? (const void *)ctx->colq_hi.data() : ctx->colq_e8.data(),
+                          ctx->colq_lo.data()};
+    const size_t bytes[5] = {8 * nc, 4 * nc, 4 * nc, ctx->colq_e8.size() + 2 * ctx->colq_hi.size(), 2 * ctx->colq_lo.size()};
+    size_t total = 0;
+    for (int i = 0; i < 5; ++i) {
+        ctx->colq_at[i] = total;
+        total += (bytes[i] + 255) & ~size_t(255);
+    }
+    if (int rc = ensure(ctx, &ctx->d_colq, &ctx->cap_colq, total)) return rc;
+    for (int i = 0; i < 5; ++i)
+        if (bytes[i]) CK(cudaMemcpyAsync(ctx->d_colq + ctx->colq_at[i], src[i], bytes[i], cudaMemcpyHostToDevice, ctx->stream));
+    return BLAMM_OK;
+}
+
 static int build_plan(blamm_ctx *ctx, int terms)
 {
-    // the scanned columns, sorted by length (the reference's order already is, fwd/rc interleaved)
-    std::vector<int> order;
-    if (ctx->active.empty()) {
-        order.resize(ctx->ncols);
-        for (int i = 0; i < ctx->ncols; ++i) order[i] = i;
-    } else {
-        order.assign(ctx->active.begin(), ctx->active.end());
+    // the scanned columns, sorted by length (a stable counting sort)
+    const int nsel = scanned_columns(ctx);
+    std::vector<int> first(kMaxMotifLen + 2, 0), order(nsel);
+    auto col_at = [&](int i) { return ctx->active.empty() ? i : (int)ctx->active[i]; };
+    for (int i = 0; i < nsel; ++i) ++first[ctx->len[col_at(i)] + 1];
+    for (int l = 0; l <= kMaxMotifLen; ++l) first[l + 1] += first[l];
+    for (int i = 0; i < nsel; ++i) {
+        const int c = col_at(i);
+        order[first[ctx->len[c]]++] = c;
     }
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ctx->len[a] < ctx->len[b]; });
-    const int nsel = (int)order.size();
     const int lmax_sel = nsel ? ctx->len[order.back()] : 1;
     if (lmax_sel > kMaxTcLen)
         return fail(ctx, BLAMM_ERR_UNSUPPORTED,
@@ -355,73 +377,59 @@ static int build_plan(blamm_ctx *ctx, int terms)
             const double gamma = nl * u / (1.0 - nl * u);
             ctx->colq_guard[c] = (eq + gamma * a) * (1.0 + 1e-9) + std::ldexp(1.0, -60);
         }
+        if (int rc = upload_colq(ctx)) return rc;
         ctx->colq_terms = terms;
         ctx->colq_valid = true;
     }
-    const std::vector<int> &kcol = ctx->colq_k;
-    const std::vector<double> &guard_d = ctx->colq_guard;
-    ctx->guard.assign(ncols, 0.0f);
-    for (const int c : order) ctx->guard[c] = (float)guard_d[c];
 
-    // Tiles, slots, A buffer.  A of one k-step of one term (kStepBytes): row i, K core cc (0, 1),
-    // byte x of 16 at (16 cc + i / 8) * 128 + (i % 8) * 16 + x; K index 4j + b for motif
-    // position j, base b, 8 (BF16) or 16 (E4M3) of them per core.  A tile's terms follow one
-    // another.
+    // Tiles and slots; the thresholds and A are built on the device from the quantised bank.
+    // A of one k-step of one term is kStepBytes; a tile's terms follow one another.
     std::vector<TileDesc> tiles;
     const size_t nslots = spans.size() * kTileCols;
-    std::vector<int32_t> slot_col(nslots, -1);
-    std::vector<float> slot_thr(nslots, std::numeric_limits<float>::infinity());
+    ctx->slot_col.assign(nslots, -1);
     int nsteps = 0;
-    for (auto &sp : spans) {
+    for (size_t t = 0; t < spans.size(); ++t) {
+        const auto &sp = spans[t];
         const int g = std::max(1, (ctx->len[order[sp.second - 1]] + kpos - 1) / kpos);
         tiles.push_back(TileDesc{g, nsteps});
         nsteps += g * nterm;
+        std::copy(order.begin() + sp.first, order.begin() + sp.second, ctx->slot_col.begin() + t * kTileCols);
     }
     tiles.push_back(TileDesc{0, nsteps});
-    std::vector<uint8_t> abuf((size_t)nsteps * kStepBytes, 0);
-    for (size_t t = 0; t < spans.size(); ++t) {
-        const auto &sp = spans[t];
-        for (int i = 0; i < sp.second - sp.first; ++i) {
-            const int c = order[sp.first + i], k = kcol[c];
-            const size_t slot = t * kTileCols + i;
-            slot_col[slot] = c;
-            // T = threshold - guard, rounded down to the accumulator's grid (u = 2^-(k+8), or
-            // 2^-9 on the E4M3 form's scale 2^k) and kept within the scores a window can reach
-            // (2^23 u; 64 L 2^-k): below them every window is a candidate, above them none is
-            const double thr = (double)ctx->thr[c] - guard_d[c];
-            const double lim = e8 ? (double)(64 * ctx->len[c] + 1) * 512.0 : std::ldexp(1.0, 23);
-            const double x = std::ldexp(thr, e8 ? 9 + k : 8 + k);
-            const double Tint = std::isnan(x) ? lim : std::floor(std::max(-lim, std::min(lim, x)));
-            slot_thr[slot] = (float)std::ldexp(Tint, e8 ? -9 : -(k + 8));  // exact: |Tint| <= 2^23
-            const uint32_t o = ctx->colq_off[c], nk = ctx->colq_off[c + 1] - o;
-            uint8_t *row = abuf.data() + (size_t)tiles[t].off * kStepBytes + (i / 8) * 128 + (i % 8) * 16;
-            const size_t term = (size_t)tiles[t].g * kStepBytes;
-            for (uint32_t kk = 0; kk < nk; ++kk) {
-                if (e8) {
-                    row[(size_t)(kk / 16) * 2048 + kk % 16] = ctx->colq_e8[o + kk];
-                    continue;
-                }
-                uint8_t *at = row + (size_t)(kk / 8) * 2048 + 2 * (kk % 8);
-                std::memcpy(at, &ctx->colq_hi[o + kk], 2);
-                if (terms == 2) std::memcpy(at + term, &ctx->colq_lo[o + kk], 2);
-            }
-        }
-    }
-
-    // upload (buffers are reused; the copies are ordered on the context's stream)
     int rc = ensure(ctx, &ctx->d_tiles, &ctx->cap_tiles, tiles.size());
-    if (!rc) rc = ensure(ctx, &ctx->d_abuf, &ctx->cap_abuf, abuf.size());
+    if (!rc) rc = ensure(ctx, &ctx->d_abuf, &ctx->cap_abuf, (size_t)nsteps * kStepBytes);
     if (!rc) rc = ensure(ctx, &ctx->d_slot_col, &ctx->cap_slot_col, nslots);
     if (!rc) rc = ensure(ctx, &ctx->d_slot_thr, &ctx->cap_slot_thr, nslots);
     if (rc) return rc;
+    // (copies from pageable memory return when the source has been read)
     CK(cudaMemcpyAsync(ctx->d_tiles, tiles.data(), sizeof(TileDesc) * tiles.size(), cudaMemcpyHostToDevice,
                        ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_abuf, abuf.data(), abuf.size(), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_slot_col, slot_col.data(), sizeof(int32_t) * nslots, cudaMemcpyHostToDevice,
+    CK(cudaMemcpyAsync(ctx->d_slot_col, ctx->slot_col.data(), sizeof(int32_t) * nslots, cudaMemcpyHostToDevice,
                        ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_slot_thr, slot_thr.data(), sizeof(float) * nslots, cudaMemcpyHostToDevice,
-                       ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));  // the host vectors go out of scope
+    if (!spans.empty()) {
+        PlanParams p{};
+        p.tiles = ctx->d_tiles;
+        p.ntiles = (int32_t)spans.size();
+        p.slot_col = ctx->d_slot_col;
+        p.slot_thr = ctx->d_slot_thr;
+        p.abuf = ctx->d_abuf;
+        p.nsteps = nsteps;
+        p.terms = terms;
+        p.P = ctx->d_P;
+        p.p_rows = ctx->p_rows;
+        p.col_len = ctx->d_len;
+        p.thr = ctx->d_thr;
+        p.guard = reinterpret_cast<const double *>(ctx->d_colq + ctx->colq_at[0]);
+        p.k = reinterpret_cast<const int32_t *>(ctx->d_colq + ctx->colq_at[1]);
+        p.off = reinterpret_cast<const uint32_t *>(ctx->d_colq + ctx->colq_at[2]);
+        p.hi = reinterpret_cast<const uint16_t *>(ctx->d_colq + ctx->colq_at[3]);
+        p.lo = reinterpret_cast<const uint16_t *>(ctx->d_colq + ctx->colq_at[4]);
+        p.e8 = ctx->d_colq + ctx->colq_at[3];
+        plan_thr_kernel<<<(unsigned)((nslots + 7) / 8), 256, 0, ctx->stream>>>(p);
+        CK(cudaGetLastError());
+        plan_fill_kernel<<<(unsigned)nsteps, 256, 0, ctx->stream>>>(p);
+        CK(cudaGetLastError());
+    }
     ctx->tiles = tiles;
     ctx->ntiles = (int)spans.size();
     ctx->erows = kBlockPos + kpos * gmax + 8;
@@ -509,7 +517,7 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     void *bufs[] = {ctx->d_P,      ctx->d_len,   ctx->d_thr,      ctx->d_tiles, ctx->d_abuf,
-                    ctx->d_slot_col, ctx->d_slot_thr, ctx->d_prof, ctx->d_bases, ctx->d_seq2, ctx->d_zmask, ctx->d_e16,
+                    ctx->d_slot_col, ctx->d_slot_thr, ctx->d_colq, ctx->d_prof, ctx->d_bases, ctx->d_seq2, ctx->d_zmask, ctx->d_e16,
                     ctx->d_runs,   ctx->d_cand,  ctx->d_hits,     ctx->d_counters,
                     ctx->d_active, ctx->d_chunk_bases[0], ctx->d_chunk_bases[1], ctx->d_chunk_runs[0],
                     ctx->d_chunk_runs[1], ctx->d_raw, ctx->d_stream, ctx->d_srun[0], ctx->d_srun[1],
@@ -1598,7 +1606,11 @@ int blamm_guard_band(const blamm_ctx *ctx, float *out)
     }
     int rc = ensure_plan(c);
     if (rc) return rc;
-    std::copy(c->guard.begin(), c->guard.end(), out);
+    for (int i = 0; i < c->ncols; ++i) out[i] = 0.0f;  // (columns that are not scanned)
+    for (int i = 0; i < scanned_columns(c); ++i) {
+        const int col = c->active.empty() ? i : (int)c->active[i];
+        out[col] = (float)c->colq_guard[col];
+    }
     return BLAMM_OK;
 }
 

@@ -1,0 +1,168 @@
+// plan_kernels.cuh -- the tensor-core plan of a set of columns, built on the device from the
+// quantised bank: thresholds on the accumulator's scale, and the A tiles.
+//
+// Threshold.  A window is a candidate iff its quantised sum reaches T, so T may be any lower
+// bound of sum(q) over the windows that are hits: T = thr - (worst sum(P - q)) is one, but the
+// worst case takes, at every position, the base whose quantisation lost most -- mostly a base
+// with a large negative score, which no hit can have many of.  Of all base choices, only those
+// with sum(P) >= thr' matter (thr' = thr minus the bound on the reference's own FP32
+// rounding), and for every lambda >= 0
+//     min { sum(q) : sum(P) >= thr' } >= lambda thr' + sum_j min_b (q_jb - lambda P_jb)
+// (Lagrangian bound; a masked base is a fifth choice with q = P = 0).  lambda = 1 is the worst
+// case above; the best lambda is usually a few thousandths (BF16) or hundredths (E4M3) more.
+// A warp takes the largest bound over 64 values of lambda, less a margin for its own FP32
+// arithmetic, or the worst case where that is larger.  Candidates per hit on a 512-motif bank:
+// E4M3 1.87 -> 1.13 at p = 1e-4 and 1.96 -> 1.01 at 1e-5, one BF16 term 1.24 -> 1.06.
+#pragma once
+#include <cstdint>
+
+#include "scan_kernels.cuh"
+#include "scan_tc.cuh"
+
+namespace blamm {
+
+struct PlanParams {
+    const TileDesc *tiles;    // ntiles + 1
+    int32_t ntiles;
+    const int32_t *slot_col;  // per slot: motif column, -1 for padding
+    float *slot_thr;
+    uint8_t *abuf;
+    int32_t nsteps;
+    int32_t terms;            // 1, 2 or kE4M3
+    // the bank and its quantised terms: column c's values start at entry off[c] (4 per position)
+    const float *P;
+    int32_t p_rows;
+    const int32_t *col_len;
+    const float *thr;
+    const uint32_t *off;
+    const uint16_t *hi, *lo;  // BF16
+    const uint8_t *e8;        // E4M3 codes of P x 2^k
+    const int32_t *k;         // exponents: grid 2^-k (BF16), scale 2^k (E4M3)
+    const double *guard;      // worst case of sum(P - q), with the reference's own rounding
+};
+
+// An E4M3 code in units of 2^-9.
+__device__ __forceinline__ float e4m3_units_f(uint32_t code)
+{
+    const int e = (int)(code >> 3) & 15, m = (int)code & 7;
+    const float a = e == 0 ? (float)m : ldexpf((float)(8 + m), e - 1);
+    return code & 0x80u ? -a : a;
+}
+
+// One warp per slot: its threshold.
+__global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
+{
+    const int slot = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (slot >= p.ntiles * kTileCols) return;
+    const int c = p.slot_col[slot];
+    if (c < 0) {
+        if (lane == 0) p.slot_thr[slot] = __int_as_float(0x7f800000);
+        return;
+    }
+    const bool e8 = p.terms == kE4M3;
+    const int L = p.col_len[c], s = p.k[c] + (e8 ? 9 : 8);  // everything below in units of 2^-s
+    const float *P = p.P + (size_t)c * p.p_rows;
+    const uint32_t o = p.off[c];
+    // lambda: 0, 1 - d, 1, 1 + d with d in powers of 2^(3/8) from 2^-14
+    float lam[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;  // 0..63
+        lam[h] = i == 0    ? 0.0f
+                 : i == 1  ? 1.0f
+                 : i < 16  ? 1.0f - exp2f(-1.0f - 0.875f * (float)(i - 2))
+                           : 1.0f + exp2f(-14.0f + 0.34f * (float)(i - 16));
+    }
+    float sum[2] = {0.f, 0.f}, mag = 0.f, maxabs = 0.f;
+    for (int j = 0; j < L; ++j) {
+        float q[4], x[4], mq = 0.f, mx = 0.f;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float v = __ldg(P + 4 * j + b);
+            const uint32_t at = o + 4 * j + b;
+            x[b] = ldexpf(v, s);
+            if (e8) {
+                q[b] = e4m3_units_f(__ldg(p.e8 + at));
+            } else {
+                q[b] = ldexpf(__uint_as_float((uint32_t)__ldg(p.hi + at) << 16), s);
+                if (p.terms == 2) q[b] += ldexpf(__uint_as_float((uint32_t)__ldg(p.lo + at) << 16), s);  // exact
+            }
+            mq = fmaxf(mq, fabsf(q[b]));
+            mx = fmaxf(mx, fabsf(x[b]));
+        }
+        maxabs += mx;
+        mag += mq + mx;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float m = 0.f;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) m = fminf(m, fmaf(-lam[h], x[b], q[b]));
+            sum[h] += m;
+        }
+    }
+    // the reference's own rounding: |fl(sum) - sum| <= (L - 1) 2^-24 sum |P| (1 + 2^-14)
+    const float thr = ldexpf(p.thr[c], s) - (float)L * 0x1p-24f * maxabs;
+    float best = __int_as_float(0xff800000);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float l = fmaxf(lam[h], 1.0f);
+        const float margin = (float)(L + 8) * 0x1p-23f * l * (fabsf(thr) + mag);
+        best = fmaxf(best, fmaf(lam[h], thr, sum[h]) - margin);  // (NaN: not taken)
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, d));
+    if (lane != 0) return;
+    // down to the grid, kept within the scores a window can reach (2^23 units; 64 L scaled):
+    // below them every window is a candidate, above them none is
+    const double worst = ((double)p.thr[c] - p.guard[c]) * exp2((double)s);
+    const double lim = e8 ? (double)(64 * L + 1) * 512.0 : 8388608.0;
+    double t = worst;
+    if ((double)best > t) t = (double)best;
+    const double units = isnan(t) ? lim : floor(fmax(-lim, fmin(lim, t)));
+    p.slot_thr[slot] = ldexpf((float)units, e8 ? -9 : -s);  // exact: |units| <= 2^23
+}
+
+// One block per k-step of a term: 256 units of 16 bytes, unit u = K core u / 128, row u % 128
+// (at (16 core + row / 8) * 128 + (row % 8) * 16 of the step).  A core holds 2 (BF16) or 4 (E4M3)
+// motif positions; rows without a column and positions beyond a column's length are zero.
+__global__ void __launch_bounds__(256) plan_fill_kernel(PlanParams p)
+{
+    const int step = blockIdx.x;
+    int t = 0, hi = p.ntiles;  // the tile: the last one that starts at or before the step
+    while (hi - t > 1) {
+        const int mid = (t + hi) >> 1;
+        if (p.tiles[mid].off <= step) t = mid;
+        else hi = mid;
+    }
+    const TileDesc td = p.tiles[t];
+    const int within = step - td.off, term = within / td.g, k = within - term * td.g;
+    const int core = threadIdx.x >> 7, row = threadIdx.x & 127;
+    const int c = p.slot_col[t * kTileCols + row];
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (c >= 0) {
+        const int L = p.col_len[c];
+        const uint32_t o = p.off[c];
+        if (p.terms == kE4M3) {
+            const int j = 8 * k + 4 * core;
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(p.e8 + o);
+            if (j < L) v.x = src[j];
+            if (j + 1 < L) v.y = src[j + 1];
+            if (j + 2 < L) v.z = src[j + 2];
+            if (j + 3 < L) v.w = src[j + 3];
+        } else {
+            const int j = 4 * k + 2 * core;
+            const uint2 *src = reinterpret_cast<const uint2 *>((term ? p.lo : p.hi) + o);
+            if (j < L) {
+                const uint2 w = src[j];
+                v.x = w.x, v.y = w.y;
+            }
+            if (j + 1 < L) {
+                const uint2 w = src[j + 1];
+                v.z = w.x, v.w = w.y;
+            }
+        }
+    }
+    reinterpret_cast<uint4 *>(p.abuf + (size_t)step * kStepBytes)[threadIdx.x] = v;
+}
+
+}  // namespace blamm

@@ -32,9 +32,9 @@
 // accumulation that keeps 24 significant bits holds sum(q) exactly (the
 // raw-score dump instance compares the accumulator with the exact sum on
 // every position and column of a test bank).  A position is a candidate iff
-// sum(q) >= T, T the column's threshold minus its guard band, rounded down to the
-// grid.  The guard band bounds |sum(q) - sum(P)| plus the reference's own FP32
-// rounding of sum(P), so every reference hit is a candidate; candidates are
+// sum(q) >= T, T a lower bound of sum(q) over the windows that are hits of the
+// column, the reference's own FP32 rounding included, rounded down to the grid
+// (plan_kernels.cuh), so every reference hit is a candidate; candidates are
 // rescored in exact sequential FP32.
 //
 // The E4M3 form (kTerms = kE4M3, kind::f8f6f4, motifs up to 64 positions): entries hold

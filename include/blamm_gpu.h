@@ -291,7 +291,8 @@ int blamm_last_stats(const blamm_ctx *ctx, blamm_stats *out);
  * guard band is applied to -- in the current tcgen05 mode. */
 int blamm_debug_scores(blamm_ctx *ctx, const char *bases, int64_t n, int64_t p0, int64_t npos,
                        float *out);
-/* The guard band of each column in the current mode (ncols floats). */
+/* The guard band of each column in the current mode (ncols floats): the worst case over all
+ * windows.  The scan narrows it to the windows that can reach the column's threshold. */
 int blamm_guard_band(const blamm_ctx *ctx, float *out);
 /* Role timing of the tensor-core scan kernel: enable (1) / disable (0) it for
  * later scans; read the last scan's counters (32 int64 per CTA, clock cycles:
