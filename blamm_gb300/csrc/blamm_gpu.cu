@@ -16,6 +16,7 @@
 #include <limits>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "blamm_gpu.h"
@@ -151,6 +152,8 @@ struct blamm_ctx {
 
     blamm_stats stats{};
     int64_t rec_slots = 0;  // record slots the last tensor-core scan reserved
+    uint8_t *h_stage = nullptr;  // pinned: inputs of short host scans, counters and first hits on their way back
+    size_t cap_stage = 0;
 };
 
 // ------------------------------------------------------------------ errors
@@ -187,6 +190,40 @@ static int ensure(blamm_ctx *ctx, T **ptr, size_t *cap, size_t need)
     CK(cudaMallocAsync((void **)ptr, n * sizeof(T), ctx->stream));
     *cap = n;
     return BLAMM_OK;
+}
+
+// Pinned staging of at least `bytes` (nothing may be in flight on it: every user waits).
+static int ensure_stage(blamm_ctx *ctx, size_t bytes)
+{
+    if (bytes <= ctx->cap_stage) return BLAMM_OK;
+    if (ctx->h_stage) CK(cudaFreeHost(ctx->h_stage));
+    ctx->h_stage = nullptr;
+    ctx->cap_stage = 0;
+    CK(cudaHostAlloc((void **)&ctx->h_stage, bytes, 0));
+    ctx->cap_stage = bytes;
+    return BLAMM_OK;
+}
+
+// memcpy, from a few threads where it is long (most of it is the destination's page faults).
+static void copy_out(void *dst, const void *src, size_t bytes)
+{
+    constexpr size_t kPart = size_t(2) << 20;
+    uint8_t *d = static_cast<uint8_t *>(dst);
+    const uint8_t *s = static_cast<const uint8_t *>(src);
+    std::thread help[3];
+    const size_t parts = std::min<size_t>(4, bytes / kPart);
+    size_t done = bytes;  // [done, bytes) is with the helpers
+    try {
+        for (size_t k = 1; k < parts; ++k) {
+            const size_t at = bytes / parts * (parts - k);
+            help[k - 1] = std::thread([=] { std::memcpy(d + at, s + at, done - at); });
+            done = at;
+        }
+    } catch (...) {  // no more threads: the rest is copied here
+    }
+    std::memcpy(d, s, done);
+    for (auto &t : help)
+        if (t.joinable()) t.join();
 }
 
 // Candidate record slots: `need` rounded up to whole blocks (the scan counts on it), and a
@@ -298,6 +335,9 @@ static int upload_colq(blamm_ctx *ctx)
 
 static int build_plan(blamm_ctx *ctx, int terms)
 {
+    // an earlier plan's uploads may still read the host tables that this one rewrites
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->plan_valid = false;
     // the scanned columns, sorted by length (a stable counting sort)
     const int nsel = scanned_columns(ctx);
     std::vector<int> first(kMaxMotifLen + 2, 0), order(nsel);
@@ -384,7 +424,8 @@ static int build_plan(blamm_ctx *ctx, int terms)
 
     // Tiles and slots; the thresholds and A are built on the device from the quantised bank.
     // A of one k-step of one term is kStepBytes; a tile's terms follow one another.
-    std::vector<TileDesc> tiles;
+    std::vector<TileDesc> &tiles = ctx->tiles;
+    tiles.clear();
     const size_t nslots = spans.size() * kTileCols;
     ctx->slot_col.assign(nslots, -1);
     int nsteps = 0;
@@ -401,7 +442,7 @@ static int build_plan(blamm_ctx *ctx, int terms)
     if (!rc) rc = ensure(ctx, &ctx->d_slot_col, &ctx->cap_slot_col, nslots);
     if (!rc) rc = ensure(ctx, &ctx->d_slot_thr, &ctx->cap_slot_thr, nslots);
     if (rc) return rc;
-    // (copies from pageable memory return when the source has been read)
+    // (their sources live in the context, unchanged until the stream has been waited for)
     CK(cudaMemcpyAsync(ctx->d_tiles, tiles.data(), sizeof(TileDesc) * tiles.size(), cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_slot_col, ctx->slot_col.data(), sizeof(int32_t) * nslots, cudaMemcpyHostToDevice,
@@ -430,7 +471,6 @@ static int build_plan(blamm_ctx *ctx, int terms)
         plan_fill_kernel<<<(unsigned)nsteps, 256, 0, ctx->stream>>>(p);
         CK(cudaGetLastError());
     }
-    ctx->tiles = tiles;
     ctx->ntiles = (int)spans.size();
     ctx->erows = kBlockPos + kpos * gmax + 8;
     // groups: as many of the first (longest) tiles as fit beside the E stages, then evened out
@@ -534,6 +574,7 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
     for (auto &h : ctx->h_chunk_runs)
         if (h) cudaFreeHost(h);
     if (ctx->h_chunk_counts) cudaFreeHost(ctx->h_chunk_counts);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -595,6 +636,9 @@ int blamm_release_buffers(blamm_ctx *ctx)
     if (ctx->d_hits) cudaFreeAsync(ctx->d_hits, ctx->stream);
     ctx->d_hits = nullptr;
     ctx->hits_cap = 0;
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
+    ctx->h_stage = nullptr;
+    ctx->cap_stage = 0;
     CK(cudaStreamSynchronize(ctx->stream));
     // give the freed memory back to the device: the stream-ordered pool would keep it
     cudaMemPool_t pool;
@@ -971,6 +1015,11 @@ static int launch_rescore(blamm_ctx *ctx, const RescoreParams &r, int64_t n, int
     return BLAMM_OK;
 }
 
+// A host scan's hits lie behind its counters in one buffer, so that the first of them come
+// back in the same copy.
+constexpr size_t kHitsAt = 64;
+static_assert(kHitsAt % sizeof(blamm_hit) == 0, "hits behind the counters");
+
 // Raw accumulators of some positions (the raw-score hook).
 struct ScanDump {
     float *out = nullptr;
@@ -980,12 +1029,14 @@ struct ScanDump {
 // One scan of device-resident bases, its counters back on the host: preparation, scan and
 // rescoring are enqueued one behind the other and the host waits once (a candidate buffer that
 // was too small grows and the scan runs again).
+// fetch: bytes that come back behind the counters (to `back`, pinned: the counters, then these).
 static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t *d_runs, int64_t nruns,
-                     blamm_hit *d_hits, int64_t hit_cap, int64_t *n_hits, const ScanDump &dump = ScanDump())
+                     blamm_hit *d_hits, int64_t hit_cap, int64_t *n_hits, const ScanDump &dump = ScanDump(),
+                     unsigned long long *d_counters = nullptr, unsigned long long *back = nullptr, size_t fetch = 0)
 {
     if (ctx->ncols == 0) return fail(ctx, BLAMM_ERR_STATE, "blamm_set_motifs was not called");
     const bool tc = ctx->mode != BLAMM_MODE_FP32;
-    unsigned long long *cnt = ctx->d_counters;  // record slots, hits, status, candidates
+    unsigned long long *cnt = d_counters ? d_counters : ctx->d_counters;  // record slots, hits, status, candidates
     ctx->stats = blamm_stats{};
     ctx->stats.positions = n;
     ctx->stats.columns = scanned_columns(ctx);
@@ -1032,8 +1083,9 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
         }
         ++launches;
         CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-        CK(cudaMemcpyAsync(got, cnt, sizeof got, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(back ? back : got, cnt, back ? kHitsAt + fetch : sizeof got, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
+        if (back) std::memcpy(got, back, sizeof got);
         if ((int)got[2]) return fail(ctx, BLAMM_ERR_TIMEOUT, "scan kernel: a device wait timed out");
         ctx->rec_slots = (int64_t)got[0];
         if (!tc || (int64_t)got[0] <= ctx->cand_cap) break;
@@ -1359,6 +1411,58 @@ static int scan_host_pipelined(blamm_ctx *ctx, const char *bases, int64_t n, con
     return rc;
 }
 
+// One scan with host run starts and hits, of host bases or (bases null) of device bases.  A
+// short input travels through pinned staging in one copy, and the first hits come back with
+// the counters: a short call is a copy, three kernels, a copy and one wait.
+constexpr size_t kStageIn = size_t(256) << 10;
+constexpr int64_t kStageHits = 16384;
+
+static int scan_host_once(blamm_ctx *ctx, const char *bases, const char *d_bases, int64_t n, const int64_t *run_start,
+                          int64_t nruns, blamm_hit *hits, int64_t hit_cap, int64_t *n_hits)
+{
+    const auto t0 = std::chrono::steady_clock::now();
+    const size_t run_bytes = sizeof(int64_t) * (size_t)nruns, at = (run_bytes + 15) & ~size_t(15);
+    const size_t in_bytes = at + (bases ? (size_t)n : 0);
+    // hits that come back with the counters: about twice what p = 1e-4 gives
+    const int64_t first = std::min<int64_t>(
+        hit_cap, std::max<int64_t>(512, std::min<int64_t>(kStageHits, n * (int64_t)scanned_columns(ctx) / 5000)));
+    const size_t back_at = in_bytes <= kStageIn ? (in_bytes + 63) & ~size_t(63) : 0;
+    const size_t fetch = sizeof(blamm_hit) * (size_t)first;
+    int rc = ensure_stage(ctx, std::max(back_at + kHitsAt + fetch, size_t(64) << 10));
+    if (!rc) rc = ensure(ctx, &ctx->d_bases, &ctx->cap_bases, in_bytes);
+    size_t hc = (size_t)ctx->hits_cap;
+    if (!rc) rc = ensure(ctx, &ctx->d_hits, &hc, (size_t)hit_cap + kHitsAt / sizeof(blamm_hit));
+    if (rc) return rc;
+    ctx->hits_cap = (int64_t)hc;
+    char *d_in = ctx->d_bases;
+    if (in_bytes <= kStageIn) {
+        std::memcpy(ctx->h_stage, run_start, run_bytes);
+        if (bases) std::memcpy(ctx->h_stage + at, bases, (size_t)n);
+        CK(cudaMemcpyAsync(d_in, ctx->h_stage, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    } else {
+        CK(cudaMemcpyAsync(d_in, run_start, run_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        if (bases) CK(cudaMemcpyAsync(d_in + at, bases, (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    blamm_hit *d_hits = ctx->d_hits + kHitsAt / sizeof(blamm_hit);
+    rc = scan_core(ctx, bases ? d_in + at : d_bases, n, reinterpret_cast<const int64_t *>(d_in), nruns, d_hits, hit_cap,
+                   n_hits, ScanDump(), reinterpret_cast<unsigned long long *>(ctx->d_hits),
+                   reinterpret_cast<unsigned long long *>(ctx->h_stage + back_at), fetch);
+    if (rc && rc != BLAMM_ERR_OVERFLOW) {
+        // no copy out of the caller's buffers may be in flight when the call returns
+        cudaStreamSynchronize(ctx->stream);
+        return rc;
+    }
+    const int64_t ncopy = std::min<int64_t>(*n_hits, hit_cap), now = std::min(ncopy, first);
+    if (now > 0) std::memcpy(hits, ctx->h_stage + back_at + kHitsAt, sizeof(blamm_hit) * (size_t)now);
+    if (ncopy > now) {
+        CK(cudaMemcpyAsync(hits + now, d_hits + now, sizeof(blamm_hit) * (size_t)(ncopy - now), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+    }
+    ctx->stats.total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    return rc;
+}
+
 int blamm_scan(blamm_ctx *ctx, const char *bases, int64_t n, const int64_t *run_start, int64_t nruns,
                blamm_hit *hits, int64_t hit_cap, int64_t *n_hits)
 {
@@ -1381,28 +1485,7 @@ int blamm_scan(blamm_ctx *ctx, const char *bases, int64_t n, const int64_t *run_
             std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
         return rc;
     }
-    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    int rc = ensure(ctx, &ctx->d_bases, &ctx->cap_bases, (size_t)n);
-    if (rc) return rc;
-    rc = ensure(ctx, &ctx->d_runs, &ctx->cap_runs, (size_t)nruns);
-    if (rc) return rc;
-    size_t hc = (size_t)ctx->hits_cap;
-    rc = ensure(ctx, &ctx->d_hits, &hc, (size_t)std::max<int64_t>(hit_cap, 1));
-    if (rc) return rc;
-    ctx->hits_cap = (int64_t)hc;
-    CK(cudaMemcpyAsync(ctx->d_bases, bases, (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_runs, run_start, sizeof(int64_t) * nruns, cudaMemcpyHostToDevice, ctx->stream));
-    rc = scan_core(ctx, ctx->d_bases, n, ctx->d_runs, nruns, ctx->d_hits, hit_cap, n_hits);
-    if (rc && rc != BLAMM_ERR_OVERFLOW) return rc;
-    const int64_t ncopy = std::min<int64_t>(*n_hits, hit_cap);
-    if (ncopy > 0)
-        CK(cudaMemcpyAsync(hits, ctx->d_hits, sizeof(blamm_hit) * ncopy, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    float ms = 0.0f;
-    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[3]);
-    ctx->stats.total_ms = ms;
-    return rc;
+    return scan_host_once(ctx, bases, nullptr, n, run_start, nruns, hits, hit_cap, n_hits);
 }
 
 int blamm_filter_score(blamm_ctx *ctx, float *d_R, int m, int n, const float *d_threshold, int *d_occIdx,
@@ -2054,12 +2137,26 @@ int blamm_theoretical_hist(blamm_ctx *ctx, const float *P, int p_rows, int ncols
         CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kernel<<<nd, kTheoThreads, smem, ctx->stream>>>(p);
         CK(cudaGetLastError());
-        if (npv > 0) CK(cudaMemcpyAsync(thr, d_thr, thr_bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        if (counts) CK(cudaMemcpyAsync(counts, d_counts, cnt_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        // Results up to 16 MB come back through pinned staging: a caller's fresh pages are then
+        // touched by the CPU only (8 MB straight into pages that are unmapped soon after took
+        // 0.2 ms or 7, depending on the process; this way 0.3).
+        const bool stage = cnt_bytes + thr_bytes <= (size_t(16) << 20);
+        uint8_t *to_thr = reinterpret_cast<uint8_t *>(thr), *to_counts = reinterpret_cast<uint8_t *>(counts);
+        if (stage) {
+            if ((rc = ensure_stage(ctx, cnt_bytes + thr_bytes))) return rc;
+            to_counts = ctx->h_stage;
+            to_thr = ctx->h_stage + cnt_bytes;
+        }
+        if (npv > 0) CK(cudaMemcpyAsync(to_thr, d_thr, thr_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        if (counts) CK(cudaMemcpyAsync(to_counts, d_counts, cnt_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         int status = 0;
         CK(cudaMemcpyAsync(&status, p.status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        if (!status) return BLAMM_OK;
+        if (!status) {
+            if (stage && npv > 0) std::memcpy(thr, to_thr, thr_bytes);
+            if (stage && counts) copy_out(counts, to_counts, cnt_bytes);
+            return BLAMM_OK;
+        }
         CK(cudaMemsetAsync(p.status, 0, sizeof(int), ctx->stream));
     }
     return fail(ctx, BLAMM_ERR_UNSUPPORTED, "a score range exceeds %d keys (fewer bins)", p.kmax);
@@ -2197,25 +2294,7 @@ int blamm_scan_stream(blamm_ctx *ctx, int64_t begin, int64_t n, const int64_t *r
             return fail(ctx, BLAMM_ERR_ARG, "run_start must ascend strictly inside [0, n)");
     CK(cudaSetDevice(ctx->device));
     if (ctx->ncols == 0) return fail(ctx, BLAMM_ERR_STATE, "blamm_set_motifs was not called");
-    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    int rc = ensure(ctx, &ctx->d_runs, &ctx->cap_runs, (size_t)nruns);
-    if (rc) return rc;
-    size_t hc = (size_t)ctx->hits_cap;
-    rc = ensure(ctx, &ctx->d_hits, &hc, (size_t)std::max<int64_t>(hit_cap, 1));
-    if (rc) return rc;
-    ctx->hits_cap = (int64_t)hc;
-    CK(cudaMemcpyAsync(ctx->d_runs, run_start, sizeof(int64_t) * nruns, cudaMemcpyHostToDevice, ctx->stream));
-    rc = scan_core(ctx, ctx->d_stream + begin, n, ctx->d_runs, nruns, ctx->d_hits, hit_cap, n_hits);
-    if (rc && rc != BLAMM_ERR_OVERFLOW) return rc;
-    const int64_t ncopy = std::min<int64_t>(*n_hits, hit_cap);
-    if (ncopy > 0)
-        CK(cudaMemcpyAsync(hits, ctx->d_hits, sizeof(blamm_hit) * ncopy, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    float ms = 0.0f;
-    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[3]);
-    ctx->stats.total_ms = ms;
-    return rc;
+    return scan_host_once(ctx, nullptr, ctx->d_stream + begin, n, run_start, nruns, hits, hit_cap, n_hits);
 }
 
 }  // extern "C"
