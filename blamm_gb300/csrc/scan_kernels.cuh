@@ -37,8 +37,8 @@ __device__ __forceinline__ int base_code_at(const uint32_t *seq2, const uint32_t
 // reference's sum), zero-masked bases adding nothing (adding +0 changes no sum that starts
 // at +0).  The 2-bit codes and mask bits of 16 positions come from two words of each array
 // (the padded stream covers the reads); the P values of 8 positions are loaded together, so
-// their latencies overlap (one load at a time, each behind the last one's branch, the sums of
-// 17.6 M candidates took 0.79 ms; together 0.33 ms with the block's list below).
+// their latencies overlap (2.9 M candidates over 16 Mi positions and 1024 columns: 0.167 ms
+// with one load at a time, each behind the last one's branch, 0.149 with 8 together).
 __device__ __forceinline__ float window_score(const uint32_t *seq2, const uint32_t *zmask, const float *pc,
                                               int64_t pos, int L)
 {
@@ -423,8 +423,9 @@ __global__ void __launch_bounds__(kPlainThreads) plain_scores_kernel(PlainParams
 // 3. rescoring of tensor-core candidates: run check + exact FP32 score
 // ------------------------------------------------------------------------
 // Candidates come as 16-byte records {chunk, slot, mask, 0}: bit i of mask = position
-// 32 chunk + i is a candidate of the tile slot's motif column.  The scan writes them in blocks of kRecBlockSlots slots; slot 0 of a block holds the number of
-// records that follow it (the rest of the block is unused).
+// 32 chunk + i is a candidate of the tile slot's motif column.  The scan writes them in
+// blocks of kRecBlockSlots slots; slot 0 of a block holds the number of records that follow
+// it (the rest of the block is unused).
 constexpr int kRecBlockSlots = 128;
 
 struct RescoreParams {

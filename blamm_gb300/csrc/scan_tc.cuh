@@ -44,11 +44,12 @@
 //
 // Roles (640 threads, warp w on SM sub-partition w % 4): warps 0-15 drain TMEM
 // (lane quarter = warp % 4, two of the block's eight 32-position chunks each) and
-// test for candidates; warps 19 and 18 issue the MMAs of the even and the odd jobs
-// (a job is one tile on one block; the whole warp runs the loop, one elected lane
-// issues), so that one issuer's waits, commits and loop overhead overlap the
-// other's MMAs; warp 17 (one lane) loads A tiles and E windows with TMA bulk copies
-// up to kEStages blocks ahead; warp 19 also allocates TMEM.
+// test for candidates; warp 16 reserves the drain warps' record blocks; warps 19 and 18
+// issue the MMAs of the even and the odd jobs (a job is one tile on one block; the
+// whole warp runs the loop, one elected lane issues), so that one issuer's waits,
+// commits and loop overhead overlap the other's MMAs; warp 17 (one lane) loads A
+// tiles and E windows with TMA bulk copies up to kEStages blocks ahead; warp 19 also
+// allocates TMEM.
 //
 // What bounds it.  A job's accumulator is half of TMEM, so only two jobs are in
 // flight, and the time per job is the larger of its MMAs (128 cycles each; 5.1 a job
@@ -63,19 +64,23 @@
 // the tensor cores' operand reads; the issuer saw the last one ~300 cycles late) 1.51,
 // 1.48, 2.48; masks in eight short chains, predicated stores, one room check per round,
 // no shared memory in the issuers' loop, issuers off the loader's sub-partition 1.42,
-// 1.33, 2.41; with the rare path taken out 1.35, 1.00, 2.35; MMAs alone 1.20, 0.74, 2.39.
+// 1.33, 2.41; fewer candidates (tighter thresholds) 1.40, 1.20, 2.41; record blocks
+// reserved by a warp of their own and a warp index that is known to be uniform 1.35,
+// 1.15, 2.39.  Of that, E4M3: without the mask arithmetic 0.96, without the whole rare
+// path 0.78; the records' stores cost nothing.  MMAs alone 1.20, 0.74, 2.39.
 // Measured and not kept: accumulators of 128 columns (four stages; an MMA of N = 128
 // takes 1.1-1.2 times its share and every barrier is met twice as often) with 16, 20 or
-// 24 drain warps 1.5-1.9; 16- and 64-column TMEM loads 1.50 and 1.35 (E4M3); the rare
-// values through a shared-memory queue 2.2; one issuer 1.64 (BF16).
+// 24 drain warps 1.5-1.9; TMEM loads of 16 columns, so that a candidate costs half a mask,
+// 1.28 against 1.15 (E4M3), of 64 columns 1.35 against 1.33; the rare values through a
+// shared-memory queue 2.2; one issuer 1.64 (BF16).
 //
 // A drain warp hands its accumulator back right after its two TMEM loads; a chunk
 // holds a candidate iff the maximum that the load returns reaches the lane's
 // threshold, and only then (rare) are the masks built and one 16-byte record
 // (chunk, slot, mask) per lane with candidates written to global memory, into a
-// block of record slots the warp reserved (kRecBlock slots per atomic, the next
-// block reserved one block ahead; slot 0 of a block counts its records).  The
-// rescoring kernel expands the masks.
+// block of record slots (kRecBlock slots per atomic; slot 0 of a block counts its
+// records).  Warp 16 keeps the next block ready for every drain warp, so that none of
+// them has an atomic in flight.  The rescoring kernel expands the masks.
 //
 // Work: the tiles are cut into groups of `tg` consecutive tiles whose A fits in
 // shared memory; a unit is (group, block of 256 positions), and units are dealt to
@@ -105,10 +110,12 @@ constexpr int kTileCols = 128;   // motif columns per tile (= UMMA M, TMEM lanes
 constexpr int kBlockPos = 256;   // positions per block (= UMMA N, TMEM columns)
 constexpr int kMaxTcLen = BLAMM_MAX_TC_MOTIF_LEN;  // longest motif on the tensor-core path
 constexpr int kEpiWarps = 16;    // TMEM drain warps (4 per lane quarter)
+constexpr int kBlockWarp = 16;   // reserves record blocks for the drain warps
 constexpr int kLoadWarp = 17;    // TMA bulk copies of A tiles and E windows
 constexpr int kMmaWarp2 = 18;    // issuer of the odd jobs
 constexpr int kMmaWarp = 19;     // issuer of the even jobs; TMEM allocation
 constexpr int kRecBlock = kRecBlockSlots;  // candidate record slots a drain warp reserves at a time
+constexpr uint32_t kNoBlock = 0xFFFFFFFFu;  // no slot index: the capacity is below 2^31
 constexpr int kTcThreads = 640;  // 20 warps (registers are allocated per 4 warps)
 constexpr int kEStages = 6;      // E windows in flight
 constexpr int kE4M3 = 8;         // kTerms of the E4M3 form (one term, K = 32 per MMA)
@@ -170,7 +177,9 @@ struct TcSmem {
 enum {
     CTL_ABORT = 0,     // set by the first wait that times out
     CTL_TMEM = 1,      // TMEM base address
-    CTL_WORDS = 4
+    CTL_DONE = 2,      // drain warps that have finished
+    CTL_BLOCK = 4,     // per drain warp: its next record block (kNoBlock: none yet)
+    CTL_WORDS = CTL_BLOCK + kEpiWarps
 };
 
 __host__ __device__ inline TcSmem tc_smem_layout(uint32_t a_bytes, int erows)
@@ -230,6 +239,14 @@ __device__ __forceinline__ uint32_t ge_mask(const uint32_t (&v)[32], uint64_t nt
     return ~(m[0] + (m[4] << 16));
 }
 
+// One block of record slots.  The capacity is a multiple of kRecBlock below 2^31; a block
+// reserved beyond it becomes the spare block behind the buffer, which nothing reads.
+__device__ __forceinline__ uint32_t reserve_block(const TcParams &p)
+{
+    const unsigned long long b = atomicAdd(p.cand_count, (unsigned long long)kRecBlock);
+    return b < (unsigned long long)p.cand_cap ? (uint32_t)b : (uint32_t)p.cand_cap;
+}
+
 // The units of one CTA: unit u = group * nblocks + block, advanced without divisions after
 // the first.  Indices are 32-bit (the host launches at most 2^31 - 1 jobs).
 struct UnitIter {
@@ -285,10 +302,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
     volatile int *ctl = reinterpret_cast<volatile int *>(smem + L.ctl);
     volatile int *s_abort = ctl + CTL_ABORT;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (by a shuffle: the compiler then knows that roles and descriptors are warp-uniform)
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
     // ---- set-up
-    if (threadIdx.x < CTL_WORDS && threadIdx.x != CTL_TMEM) ctl[threadIdx.x] = 0;
+    if (threadIdx.x < CTL_WORDS && threadIdx.x != CTL_TMEM) ctl[threadIdx.x] = threadIdx.x >= CTL_BLOCK ? (int)kNoBlock : 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kEStages; ++s) {
             ptx::mbar_init(bars + 8 * (BAR_EFULL + s), 1);
@@ -324,7 +342,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
     it.init(p, ngroups);
 
     if (warp == kMmaWarp || warp == kMmaWarp2) {
-        // ============ MMA issuers: warp 16 the even jobs, warp 17 the odd ones ============
+        // ============ MMA issuers: warp 19 the even jobs, warp 18 the odd ones ============
         // Both walk every job of the CTA.  The whole warp runs the loop (warp-uniform
         // descriptors, one vote per wait); one elected lane issues each MMA and commit.
         const uint32_t mine = warp == kMmaWarp ? 0u : 1u;
@@ -510,35 +528,47 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
             pr[4] += t_we;
             pr[5] += t_tile;
         }
+    } else if (warp == kBlockWarp) {
+        // ============ record blocks: one ahead for every drain warp ============
+        for (bool done = false; !done;) {
+            done = ctl[CTL_DONE] == kEpiWarps;  // (read first: no block is taken after that)
+            if (lane < kEpiWarps) {
+                const uint32_t b = (uint32_t)ctl[CTL_BLOCK + lane];
+                if (done) {  // every reserved block states its count
+                    if (b != kNoBlock) p.cand[b] = make_uint4(0u, 0u, 0u, 0u);
+                } else if (b == kNoBlock) {
+                    ctl[CTL_BLOCK + lane] = (int)reserve_block(p);
+                }
+            }
+            __syncwarp();
+            if (!done) __nanosleep(500);
+        }
     } else if (warp < kEpiWarps) {
         // ===================== epilogue (warps 0-15) ======================
         const int q = warp & 3;     // TMEM lanes (motif rows) 32q .. 32q+31
         const int grp = warp >> 2;  // the block's 32-position chunks 2 grp and 2 grp + 1
         const uint32_t lt = (1u << lane) - 1u;
         const uint32_t row = (uint32_t)(q * 32 + lane);  // this lane's motif row in a tile
-        // record blocks (slot indices): the current one and, in lane 0, the next one, reserved
-        // one block ahead so that the atomic's latency stays off the drain path.  The capacity is
-        // a multiple of kRecBlock below 2^31; a block reserved beyond it becomes the spare block
-        // behind the buffer, which nothing reads.
-        const uint32_t cap = (uint32_t)p.cand_cap;
-        auto reserve = [&]() -> uint32_t {
-            const unsigned long long b = atomicAdd(p.cand_count, (unsigned long long)kRecBlock);
-            return b < (unsigned long long)cap ? (uint32_t)b : cap;
-        };
+        // The current record block (slot indices).  The next one is usually waiting in shared
+        // memory: an atomic's answer takes a microsecond, and even a warp that does not look
+        // at it is held up by its next load.
         uint32_t rec = 0, left = 0;  // the current block's next record, how many still fit
         bool have = false;           // there is a current block
-        uint32_t nxt_blk = 0;
-        if (lane == 0) nxt_blk = reserve();
-        auto close_block = [&]() {  // slot 0 of a block: its number of records
+        auto close_block = [&]() {   // slot 0 of a block: its number of records
             const uint32_t n = (uint32_t)(kRecBlock - 1) - left;
             if (have && lane == 0) p.cand[rec - n - 1u] = make_uint4(n, 0u, 0u, 0u);
             have = true;
         };
         auto next_block = [&]() {
             close_block();
-            rec = __shfl_sync(0xffffffffu, nxt_blk, 0) + 1u;
+            uint32_t b = (uint32_t)ctl[CTL_BLOCK + warp];
+            __syncwarp();
+            if (lane == 0) {
+                if (b == kNoBlock) b = reserve_block(p);
+                else ctl[CTL_BLOCK + warp] = (int)kNoBlock;
+            }
+            rec = __shfl_sync(0xffffffffu, b, 0) + 1u;
             left = (uint32_t)(kRecBlock - 1);
-            if (lane == 0) nxt_blk = reserve();
         };
         long long t_af = 0, t_dr = 0, n_rare = 0, t_red = 0, t_full = 0;
         const long long t_start = tick<kProf>();
@@ -625,9 +655,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
                 if (kProf) t_red += tick<kProf>() - tr0;
             }
         }
-        // every reserved block states its count: the current one and the one reserved ahead
         close_block();
-        if (lane == 0) p.cand[nxt_blk] = make_uint4(0u, 0u, 0u, 0u);
+        if (lane == 0) {
+            __threadfence_block();
+            atomicAdd(const_cast<int *>(ctl) + CTL_DONE, 1);
+        }
         if (kProf && lane == 0 && warp == 0) {
             long long *pr = p.prof + 32 * blockIdx.x;
             pr[7] += t_af;
