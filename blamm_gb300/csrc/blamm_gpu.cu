@@ -141,7 +141,7 @@ struct blamm_ctx {
     uint8_t *d_theo = nullptr;  // theoretical histograms: bank, tables, results of a call
     size_t cap_theo = 0;
     // FASTA parsing: tile summaries, the parser before each tile, totals (96 bytes per 16 KB of text)
-    IngTile *d_ing_tiles = nullptr;
+    uint4 *d_ing_tiles = nullptr;  // the tiles' sums (IngTile)
     IngPrefix *d_ing_prefix = nullptr;
     unsigned long long *d_ing_totals = nullptr;
     size_t cap_ing_tiles = 0, cap_ing_prefix = 0, cap_ing_totals = 0;
@@ -589,7 +589,7 @@ static int64_t call_buffer_bytes(const blamm_ctx *ctx)
                      8 * ctx->cap_runs + 8 * (ctx->cap_chunk_runs[0] + ctx->cap_chunk_runs[1]) +
                      ctx->cap_chunk_bases[0] + ctx->cap_chunk_bases[1] + ctx->cap_raw + ctx->cap_stream +
                      8 * (ctx->cap_srun[0] + ctx->cap_srun[1] + ctx->cap_srun[2] + ctx->cap_shdr) +
-                     sizeof(IngTile) * ctx->cap_ing_tiles + sizeof(IngPrefix) * ctx->cap_ing_prefix +
+                     16 * ctx->cap_ing_tiles + sizeof(IngPrefix) * ctx->cap_ing_prefix +
                      8 * ctx->cap_ing_totals + ctx->cap_theo) +
            16 * (ctx->cand_cap > 0 ? ctx->cand_cap + kRecBlock : 0) + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
 }
@@ -2177,16 +2177,22 @@ static int fasta_parse(blamm_ctx *ctx, const char *d_raw, int64_t nraw, bool res
     const int64_t ntiles = (nraw + kIngTile - 1) / kIngTile;
     if (ntiles > 0x7fffffff) return fail(ctx, BLAMM_ERR_UNSUPPORTED, "%lld bytes of text in one call", (long long)nraw);
     const int vec = (reinterpret_cast<uintptr_t>(d_raw) & 15u) == 0 ? 1 : 0;  // 16-byte loads
-    int rc = ensure(ctx, &ctx->d_ing_tiles, &ctx->cap_ing_tiles, (size_t)ntiles);
+    int rc = ensure(ctx, &ctx->d_ing_tiles, &ctx->cap_ing_tiles, (size_t)(kIngTileWords * ntiles));
     if (!rc) rc = ensure(ctx, &ctx->d_ing_prefix, &ctx->cap_ing_prefix, (size_t)ntiles);
     if (!rc) rc = ensure(ctx, &ctx->d_ing_totals, &ctx->cap_ing_totals, (size_t)kIngTotals);
     if (rc) return rc;
-    ingest_tiles_kernel<<<(unsigned)ntiles, kIngThreads, 0, st>>>(d_raw, nraw, vec, ctx->d_ing_tiles);
+    IngTile tiles{};  // (the arrays of 16-byte words first)
+    tiles.e = ctx->d_ing_tiles;
+    tiles.warps = tiles.e + 2 * ntiles;
+    tiles.bases = reinterpret_cast<uint64_t *>(tiles.warps + 2 * kIngWarps * ntiles);
+    tiles.info = reinterpret_cast<uint32_t *>(tiles.bases + kIngThreads * ntiles);
+    tiles.count = (int)ntiles;
+    ingest_tiles_kernel<<<(unsigned)ntiles, kIngThreads, 0, st>>>(d_raw, nraw, vec, tiles);
     CK(cudaGetLastError());
-    ingest_scan_kernel<<<1, kIngScanThreads, 0, st>>>(ctx->d_ing_tiles, (int)ntiles, ctx->d_ing_prefix, ctx->d_ing_totals);
+    ingest_scan_kernel<<<1, kIngScanThreads, 0, st>>>(tiles, ctx->d_ing_prefix, ctx->d_ing_totals);
     CK(cudaGetLastError());
     auto emit = [&]() -> int {
-        ingest_emit_kernel<<<(unsigned)ntiles, kIngThreads, 0, st>>>(d_raw, nraw, vec, ctx->d_ing_prefix, ctx->d_ing_totals,
+        ingest_emit_kernel<<<(unsigned)(ntiles * (kIngThreads / kIngEmit)), kIngEmit, 0, st>>>(d_raw, nraw, vec, tiles, ctx->d_ing_prefix, ctx->d_ing_totals,
                                                                      d_bases, d_run_start, d_run_seq, d_run_seqpos,
                                                                      d_header_pos);
         CK(cudaGetLastError());
