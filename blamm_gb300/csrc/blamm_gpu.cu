@@ -23,6 +23,7 @@
 #include "scan_kernels.cuh"
 #include "scan_tc.cuh"
 #include "hist_kernels.cuh"
+#include "hist_tc.cuh"
 #include "ingest_kernels.cuh"
 #include "plan_kernels.cuh"
 
@@ -1542,6 +1543,47 @@ int blamm_set_softmask(blamm_ctx *ctx, int lowercase_scores)
     return BLAMM_OK;
 }
 
+// Whether the tensor-core form of the histograms takes this call, and its columns' constants.
+// A tile costs it the same for one column as for 64, the plain form costs by the addition and
+// by the bin (about five additions): 8 Mbp, lengths 6-20, ms: 16 columns 0.43 against 0.40,
+// 32 columns 0.47 against 0.65, 64 columns 0.51 against 1.17.  Short streams do not pay for
+// its set-up: 64 columns, 50 kbp 0.082 against 0.069, 200 kbp 0.094 against 0.113.  And A, rows
+// and counts have to fit in shared memory, values to be finite and of usual magnitude, and
+// bins so wide that few scores lie too near a boundary to settle theirs.
+static bool hist_tc_fits(const blamm_ctx *ctx, int64_t n, const float *min_score, const float *width, int nbins,
+                         std::vector<float4> &scale)
+{
+    const int tiles = (ctx->ncols + kHistCols - 1) / kHistCols;
+    int64_t adds = 0;
+    for (int c = 0; c < ctx->ncols; ++c) adds += ctx->len[c] + 5;
+    if (adds < 300 * (int64_t)tiles || n * tiles < 100000 || n >= (int64_t(1) << 32)) return false;
+    if (nbins > 1024 || ctx->lmax > 128 || hist_tc_layout(ctx->lmax, nbins).total > (uint32_t)ctx->max_smem) return false;
+    scale.resize((size_t)ctx->ncols);
+    for (int c = 0; c < ctx->ncols; ++c) {
+        const float *P = &ctx->P[(size_t)c * ctx->p_rows];
+        const int L = ctx->len[c];
+        float top = 0.f;
+        double sum = 0.0;
+        for (int j = 0; j < L; ++j) {
+            float m = 0.f;
+            for (int b = 0; b < 4; ++b) m = std::max(m, std::isnan(P[4 * j + b]) ? INFINITY : std::fabs(P[4 * j + b]));
+            top = std::max(top, m);
+            sum += m;
+        }
+        const double w = width[c], mn = min_score[c];
+        auto usual = [](double x) { return x > 0x1p-60 && x < 0x1p60; };  // (false for NaN)
+        if (!usual(w) || !(std::fabs(mn) < 0x1p60) || !(top == 0.f || usual(top))) return false;
+        const int k = top == 0.f ? 0 : 7 - column_exponent(P, L);
+        // how far the scaled score can be off in bins: the terms' grid, the FP32 sum's own
+        // rounding, the roundings of the factor, the offset and the bin's formula (generous)
+        const double eps = (std::ldexp((double)L, -k - 9) + 0x1p-20 * (sum + std::fabs(mn))) / w + 0x1p-20 * nbins + L * 0x1p-24 * sum / w;
+        // (the rounding to bins holds for |t| < 2^22)
+        if (!(eps < 0.02) || !((sum + std::fabs(mn)) / w < 0x1p21)) return false;
+        scale[c] = make_float4(std::ldexp(1.f, k), (float)(std::ldexp(1.0, -k) / w), (float)(-mn / w - 0.5), (float)(0.5 - eps));
+    }
+    return true;
+}
+
 // The empirical histograms of n bases already on the device (run starts on the host).
 static int score_histograms_on(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t *run_start,
                                int64_t nruns, const float *min_score, const float *width, int nbins,
@@ -1553,54 +1595,74 @@ static int score_histograms_on(blamm_ctx *ctx, const char *d_bases, int64_t n, c
     rc = launch_pack(ctx, d_bases, n);
     if (rc) return rc;
     const size_t nc = (size_t)ctx->ncols;
-    float *d_min = nullptr, *d_w = nullptr;
-    unsigned long long *d_counts = nullptr;
-    auto cleanup = [&]() {
-        if (d_min) cudaFree(d_min);
-        if (d_w) cudaFree(d_w);
-        if (d_counts) cudaFree(d_counts);
-    };
-    cudaError_t e = cudaMalloc(&d_min, sizeof(float) * nc);
-    if (e == cudaSuccess) e = cudaMalloc(&d_w, sizeof(float) * nc);
-    if (e == cudaSuccess) e = cudaMalloc(&d_counts, sizeof(unsigned long long) * nc * nbins);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_min, min_score, sizeof(float) * nc, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_w, width, sizeof(float) * nc, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_counts, 0, sizeof(unsigned long long) * nc * nbins, ctx->stream);
-    if (e != cudaSuccess) {
-        cleanup();
-        return fail(ctx, BLAMM_ERR_CUDA, "%s", cudaGetErrorString(e));
-    }
-    PlainParams p{};
-    p.seq2 = ctx->d_seq2;
-    p.zmask = ctx->d_zmask;
-    p.n = n;
-    p.run_start = ctx->d_runs;
-    p.nruns = nruns;
-    p.P = ctx->d_P;
-    p.p_rows = ctx->p_rows;
-    p.ncols = ctx->ncols;
-    p.lmax = ctx->lmax;
-    p.col_len = ctx->d_len;
-    p.min_score = d_min;
-    p.width = d_w;
-    p.nbins = nbins;
-    p.counts = d_counts;
-    if ((size_t)(p.p_rows + nbins) * 4 + 256 + p.lmax + 64 > (size_t)ctx->max_smem) {
-        cleanup();
+    std::vector<float4> scale;
+    const bool tc = hist_tc_fits(ctx, n, min_score, width, nbins, scale);
+    if ((size_t)(ctx->p_rows + nbins) * 4 + 256 + ctx->lmax + 64 > (size_t)ctx->max_smem)
         return fail(ctx, BLAMM_ERR_UNSUPPORTED, "too many bins for shared memory");
+    // counts and status, columns' values: one workspace
+    const size_t cbytes = sizeof(unsigned long long) * (nc * nbins + 1);
+    auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
+    rc = ensure(ctx, &ctx->d_theo, &ctx->cap_theo, up(cbytes) + 2 * up(sizeof(float) * nc) + sizeof(float4) * nc);
+    if (rc) return rc;
+    unsigned long long *d_counts = reinterpret_cast<unsigned long long *>(ctx->d_theo);
+    float *d_min = reinterpret_cast<float *>(ctx->d_theo + up(cbytes));
+    float *d_w = reinterpret_cast<float *>(ctx->d_theo + up(cbytes) + up(sizeof(float) * nc));
+    float4 *d_scale = reinterpret_cast<float4 *>(ctx->d_theo + up(cbytes) + 2 * up(sizeof(float) * nc));
+    CK(cudaMemcpyAsync(d_min, min_score, sizeof(float) * nc, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(d_w, width, sizeof(float) * nc, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemsetAsync(d_counts, 0, cbytes, ctx->stream));
+    if (tc) {
+        CK(cudaMemcpyAsync(d_scale, scale.data(), sizeof(float4) * nc, cudaMemcpyHostToDevice, ctx->stream));
+        HistTcParams p{};
+        p.seq2 = ctx->d_seq2;
+        p.zmask = ctx->d_zmask;
+        p.n = n;
+        p.run_start = ctx->d_runs;
+        p.nruns = nruns;
+        p.P = ctx->d_P;
+        p.p_rows = ctx->p_rows;
+        p.ncols = ctx->ncols;
+        p.lmax = ctx->lmax;
+        p.col_len = ctx->d_len;
+        p.min_score = d_min;
+        p.width = d_w;
+        p.scale = d_scale;
+        p.nbins = nbins;
+        p.counts = d_counts;
+        p.status = reinterpret_cast<int *>(d_counts + nc * nbins);
+        p.wait_limit = ctx->wait_limit;
+        const int tiles = (ctx->ncols + kHistCols - 1) / kHistCols;
+        p.cols = (ctx->ncols + tiles - 1) / tiles;
+        // (more than 116 KB, so that two blocks, which each allocate all of TMEM, never share an SM)
+        const uint32_t smem = std::max<uint32_t>(hist_tc_layout(ctx->lmax, nbins).total, 116 * 1024);
+        const int64_t blocks = (n + kHistBlock - 1) / kHistBlock;
+        const int64_t per = std::max<int64_t>(1, (int64_t)ctx->sm_count * (tiles > 8 ? 4 : 1) / tiles);
+        CK(cudaFuncSetAttribute(hist_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem));
+        hist_tc_kernel<<<dim3((unsigned)std::min(blocks, per), (unsigned)tiles), kHistThreads, smem, ctx->stream>>>(p);
+        CK(cudaGetLastError());
+    } else {
+        PlainParams p{};
+        p.seq2 = ctx->d_seq2;
+        p.zmask = ctx->d_zmask;
+        p.n = n;
+        p.run_start = ctx->d_runs;
+        p.nruns = nruns;
+        p.P = ctx->d_P;
+        p.p_rows = ctx->p_rows;
+        p.ncols = ctx->ncols;
+        p.lmax = ctx->lmax;
+        p.col_len = ctx->d_len;
+        p.min_score = d_min;
+        p.width = d_w;
+        p.nbins = nbins;
+        p.counts = d_counts;
+        p.shared_bins = plain_smem_bytes(4, p.lmax, nbins) <= (size_t)ctx->max_smem ? 1 : 0;
+        if ((rc = launch_plain<true>(ctx, p))) return rc;
     }
-    p.shared_bins = plain_smem_bytes(4, p.lmax, nbins) <= (size_t)ctx->max_smem ? 1 : 0;
-    if ((rc = launch_plain<true>(ctx, p))) {
-        cleanup();
-        return rc;
-    }
-    std::vector<unsigned long long> host(nc * nbins);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(host.data(), d_counts, sizeof(unsigned long long) * nc * nbins, cudaMemcpyDeviceToHost,
-                            ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cleanup();
-    if (e != cudaSuccess) return fail(ctx, BLAMM_ERR_CUDA, "%s", cudaGetErrorString(e));
+    std::vector<unsigned long long> host(nc * nbins + 1);
+    CK(cudaMemcpyAsync(host.data(), d_counts, cbytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (host[nc * nbins]) return fail(ctx, BLAMM_ERR_TIMEOUT, "histogram kernel: a device wait timed out");
     for (size_t i = 0; i < nc * (size_t)nbins; ++i) counts[i] += host[i];
     return BLAMM_OK;
 }

@@ -147,18 +147,6 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity, l
 }
 
 // ---------------------------------------------------------------- shared memory
-__device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
-{
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-
-__device__ __forceinline__ uint32_t ld_shared(uint32_t a)
-{
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
-}
-
 // A predicated 16-byte store: no branch around it.
 __device__ __forceinline__ void st_global_v4_if(bool f, void *a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
 {
@@ -168,6 +156,13 @@ __device__ __forceinline__ void st_global_v4_if(bool f, void *a, uint32_t x, uin
         "@p st.global.v4.b32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"((int)f),
         "l"(a), "r"(x), "r"(y), "r"(z), "r"(w)
         : "memory");
+}
+
+__device__ __forceinline__ float ld_shared_f32(uint32_t a)
+{
+    float v;
+    asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
 }
 
 __device__ __forceinline__ float4 ld_shared_v4(uint32_t a)
@@ -326,15 +321,18 @@ __device__ __forceinline__ void tmem_ld_max_32x32b_x32(uint32_t taddr, uint32_t 
         : "memory");
 }
 
-// The same for 16 columns.
-__device__ __forceinline__ void tmem_ld_max_32x32b_x16(uint32_t taddr, uint32_t (&r)[16], float &red)
+// The load alone.
+__device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32])
 {
     asm volatile(
-        "tcgen05.ld.red.sync.aligned.32x32b.x16.max.f32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, %16, [%17];"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=f"(red)
+          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
 }
@@ -374,18 +372,11 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
     return r;
 }
 
-// tcgen05.wait::ld that also "redefines" the destination registers of the
-// awaited load, so that the compiler cannot move their uses above the wait.
-__device__ __forceinline__ void tmem_wait_ld_dep(uint32_t (&r)[32])
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
 {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]),
-                   "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]),
-                   "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]),
-                   "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]),
-                   "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
-                 :
-                 : "memory");
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 }  // namespace ptx

@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(PrepParams a)
 // share (a 16-byte load of a warp is four cycles): 32 additions a cycle and SM.  2 Mbp x 256
 // columns: 1.01 ms, 0.93 at that rate (one 4-byte load at a byte-coded address, a branch and an
 // addition per motif position: 2.91); 8 Mbp x 64 columns with 250 bins: 1.09 (2.57 with a
-// division per score).
+// division per score).  Banks of some dozen columns on longer streams are binned by hist_tc_kernel.
 constexpr int kPlainThreads = 256;
 constexpr int kPlainReg = 32;  // motif positions whose offsets are kept in registers
 constexpr int kPlainRow = 5 * 16;  // bytes of one motif position of four columns
