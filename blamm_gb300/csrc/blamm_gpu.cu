@@ -2095,7 +2095,9 @@ int blamm_autotune(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64_t
             ms = ctx->stats.kernel_ms;
         }
         std::sort(t, t + 5);
-        if (t[2] < best) {
+        // (a form is taken over the ones before it only if it is faster by more than such
+        // medians differ from run to run, about 2 %: otherwise the choice would be a toss-up)
+        if (t[2] < 0.97f * best) {
             best = t[2];
             bt = ctx->auto_terms;
         }
