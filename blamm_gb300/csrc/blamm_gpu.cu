@@ -1546,17 +1546,23 @@ int blamm_set_softmask(blamm_ctx *ctx, int lowercase_scores)
 // Whether the tensor-core form of the histograms takes this call, and its columns' constants.
 // A tile costs it the same for one column as for 64, the plain form costs by the addition and
 // by the bin (about five additions): 8 Mbp, lengths 6-20, ms: 16 columns 0.43 against 0.40,
-// 32 columns 0.47 against 0.65, 64 columns 0.51 against 1.17.  Short streams do not pay for
-// its set-up: 64 columns, 50 kbp 0.082 against 0.069, 200 kbp 0.094 against 0.113.  And A, rows
-// and counts have to fit in shared memory, values to be finite and of usual magnitude, and
-// bins so wide that few scores lie too near a boundary to settle theirs.
+// 32 columns 0.47 against 0.65, 64 columns 0.51 against 1.17: a tile is worth about 300
+// additions a position.  And its set-up (A, rows, counts of every tile) has to be paid: the two
+// meet where the additions saved reach about 90 M a tile for up to four tiles, which run side by
+// side on a stream this short, and 180 M beyond (lengths 6-24, us, against the plain form: 64
+// columns 79 against 72 at 64 kbp, 89 against 102 at 150 kbp; 200 columns 132 against 123 and
+// 156 against 177; 800 columns 526 against 468 at 150 kbp; 4000 columns 4540 against 4416 at
+// 100 kbp, 4184 against 4403 at 150 kbp).  And A, rows and counts have to fit in shared memory,
+// values to be finite and of usual magnitude, and bins so wide that few scores lie too near a
+// boundary to settle theirs.
 static bool hist_tc_fits(const blamm_ctx *ctx, int64_t n, const float *min_score, const float *width, int nbins,
                          std::vector<float4> &scale)
 {
     const int tiles = (ctx->ncols + kHistCols - 1) / kHistCols;
     int64_t adds = 0;
     for (int c = 0; c < ctx->ncols; ++c) adds += ctx->len[c] + 5;
-    if (adds < 300 * (int64_t)tiles || n * tiles < 100000 || n >= (int64_t(1) << 32)) return false;
+    const double saved = (double)(adds - 300 * (int64_t)tiles) * (double)n;
+    if (saved < (tiles > 4 ? 180e6 : 90e6) * tiles || n >= (int64_t(1) << 32)) return false;
     if (nbins > 1024 || ctx->lmax > 128 || hist_tc_layout(ctx->lmax, nbins).total > (uint32_t)ctx->max_smem) return false;
     scale.resize((size_t)ctx->ncols);
     for (int c = 0; c < ctx->ncols; ++c) {

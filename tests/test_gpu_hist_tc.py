@@ -2,7 +2,7 @@
 64, lengths around the k-steps of four positions (one is taken by the shifted rows), streams
 around the blocks of 512 positions, runs shorter and longer than a block, masked bases, bins
 from one to many, scores on bin boundaries and beyond the bins.  Exact against a restatement in
-numpy."""
+numpy.  Streams long enough for this form."""
 import numpy as np
 import pytest
 
@@ -29,12 +29,12 @@ def _bins(P, lens, nbins):
     (20, (40, 47), 100), (128, (7, 8), 250)])
 def test_columns_lengths_and_bins(scanner, cols, lengths, nbins):
     P, lens, _ = make_bank(440 + cols, cols, *lengths, rc=False)
-    bases, runs = make_stream(441, 110_011, nruns=9, lower_frac=0.05)
+    bases, runs = make_stream(441, 480_011, nruns=9, lower_frac=0.05)
     _check(scanner, P, lens, bases, runs, *_bins(P, lens, nbins), nbins)
 
 
-@pytest.mark.parametrize("n,nruns,lower", [(102_399, 1, 0.0), (102_400, 1, 0.0), (102_401, 2, 0.5), (102_911, 600, 0.05),
-                                           (120_000, 9_000, 0.0)])
+@pytest.mark.parametrize("n,nruns,lower", [(262_143, 1, 0.0), (262_144, 1, 0.0), (262_145, 2, 0.5), (262_655, 600, 0.05),
+                                           (300_000, 9_000, 0.0)])
 def test_streams_and_runs(scanner, n, nruns, lower):
     P, lens, _ = make_bank(450, 40, 5, 18, rc=False)
     bases, runs = make_stream(451 + nruns, n, nruns=nruns, lower_frac=lower)
@@ -54,5 +54,5 @@ def test_scores_on_boundaries_and_beyond_the_bins(scanner):
     width[8:16] = 0.3
     width[24:32] = 0.05
     width[32:] = (np.float32(0.1) * np.float32(10.0) ** np.arange(-8, 8)).astype(np.float32)
-    bases, runs = make_stream(461, 105_000, nruns=3, lower_frac=0.2)
+    bases, runs = make_stream(461, 350_000, nruns=3, lower_frac=0.2)
     _check(scanner, P, lens, bases, runs, mn, width, 40)
