@@ -16,12 +16,12 @@
 // its columns each), warp 16 makes the entries from the packed stream, warp 17 issues the MMAs
 // and owns TMEM.  The counts stay in shared memory (32 bits) until the block ends.
 //
-// What bounds it: the issue of the binning, about 14 instructions a score with the queueing of
-// the unsettled (8 Mbp x 64 columns of 6-20 positions, 250 bins: 0.8 % of the scores), one of
-// them a shared-memory atomic.  That case: kernel 0.36 ms, call 0.51; the plain form, which is
-// bound by one shared-memory wavefront per addition, 1.09 and 1.17.  With the counts column by
-// column (the lanes' bins in random banks, 4.5 wavefronts an atomic) and a branch around each
-// atomic 0.46 ms.
+// What bounds it: the issue of the binning, 19 instructions a score in all (the queue and the
+// exact sums of the unsettled included: 0.8 % of the scores at 8 Mbp x 64 columns of 6-20
+// positions and 250 bins), one of them a shared-memory atomic.  That case: kernel 0.39 ms under
+// the profiler, call 0.51; the plain form, which is bound by one shared-memory wavefront per
+// addition, 1.09 and 1.17.  With the counts column by column (the lanes' bins in random banks,
+// 4.5 wavefronts an atomic) and a branch around each atomic 22 instructions, 0.49 ms.
 #pragma once
 #include <cstdint>
 
