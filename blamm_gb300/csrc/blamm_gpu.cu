@@ -677,6 +677,7 @@ int blamm_set_motifs(blamm_ctx *ctx, const float *P, int p_rows, int ncols, cons
         lmax = std::max(lmax, (int)col_len[c]);
     }
     CK(cudaSetDevice(ctx->device));
+    CK(cudaStreamSynchronize(ctx->stream));  // (what is enqueued may still read the old bank)
     ctx->ncols = ncols;
     ctx->p_rows = p_rows;
     ctx->lmax = lmax;
@@ -694,9 +695,12 @@ int blamm_set_motifs(blamm_ctx *ctx, const float *P, int p_rows, int ncols, cons
     CK(cudaMalloc(&ctx->d_P, sizeof(float) * ctx->P.size()));
     CK(cudaMalloc(&ctx->d_len, sizeof(int32_t) * ncols));
     CK(cudaMalloc(&ctx->d_thr, sizeof(float) * ncols));
-    CK(cudaMemcpy(ctx->d_P, ctx->P.data(), sizeof(float) * ctx->P.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_len, ctx->len.data(), sizeof(int32_t) * ncols, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->d_thr, ctx->thr.data(), sizeof(float) * ncols, cudaMemcpyHostToDevice));
+    // On the context's stream, ahead of the plan and scan kernels that read these: a plain
+    // cudaMemcpy from pageable memory may return before the data is on the device, and nothing
+    // orders this non-blocking stream behind it.  (The sources stay until the stream is waited for.)
+    CK(cudaMemcpyAsync(ctx->d_P, ctx->P.data(), sizeof(float) * ctx->P.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_len, ctx->len.data(), sizeof(int32_t) * ncols, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_thr, ctx->thr.data(), sizeof(float) * ncols, cudaMemcpyHostToDevice, ctx->stream));
     ctx->plan_valid = false;
     return BLAMM_OK;
 }
@@ -736,8 +740,9 @@ int blamm_set_thresholds(blamm_ctx *ctx, const float *thr)
     if (!ctx || !thr) return BLAMM_ERR_ARG;
     if (ctx->ncols == 0) return fail(ctx, BLAMM_ERR_STATE, "no motif bank");
     CK(cudaSetDevice(ctx->device));
+    CK(cudaStreamSynchronize(ctx->stream));  // (an earlier upload may still read the host copy)
     ctx->thr.assign(thr, thr + ctx->ncols);
-    CK(cudaMemcpy(ctx->d_thr, ctx->thr.data(), sizeof(float) * ctx->ncols, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->d_thr, ctx->thr.data(), sizeof(float) * ctx->ncols, cudaMemcpyHostToDevice, ctx->stream));
     ctx->plan_valid = false;
     return BLAMM_OK;
 }
