@@ -1074,7 +1074,7 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
             }
             int grid = 0;
             const PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 15u);
-            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out != nullptr, &launches, &grid))) return rc;
+            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out || ctx->debug_stall > kStallIssuers, &launches, &grid))) return rc;
             CK(cudaEventRecord(ctx->ev[5], ctx->stream));
             const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
                                                    d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
@@ -1717,7 +1717,8 @@ int blamm_score_histograms_stream(blamm_ctx *ctx, int64_t begin, int64_t n, cons
 int blamm_debug_stall(blamm_ctx *ctx, int enable, long long wait_limit_cycles)
 {
     if (!ctx || wait_limit_cycles < 0) return BLAMM_ERR_ARG;
-    ctx->debug_stall = enable ? 1 : 0;
+    const int role = enable & 255;
+    ctx->debug_stall = enable > 0 && role > kStallIssuers && role < kStallEnd ? enable : enable ? kStallIssuers : 0;
     ctx->wait_limit = wait_limit_cycles > 0 ? wait_limit_cycles : 4000000000LL;
     return BLAMM_OK;
 }

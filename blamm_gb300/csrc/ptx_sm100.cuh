@@ -104,6 +104,23 @@ __device__ __forceinline__ bool mbar_wait_nohint(uint32_t bar, uint32_t parity, 
     }
 }
 
+// The same for a whole warp, with one answer for all of its lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, long long limit_cycles)
+{
+    if (__all_sync(0xffffffffu, mbar_try_wait_nohint(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (uint32_t it = 1;; ++it) {
+        if (__all_sync(0xffffffffu, mbar_try_wait_nohint(bar, parity))) return true;
+        if ((it & 7u) == 0) {
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+            if (__any_sync(0xffffffffu, clock64() - t0 > limit_cycles)) {
+                *abort_flag = 1;
+                return false;
+            }
+        }
+    }
+}
+
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;

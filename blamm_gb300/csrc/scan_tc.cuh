@@ -95,8 +95,11 @@
 // with try_wait without a suspend hint, the loader's try_wait sleeps): on a timeout the
 // CTA raises an abort flag, every role stops, copies and MMAs in flight are drained,
 // TMEM is freed and the status word tells the host.  The hardware barriers have no
-// timeout, but an issuer waits there once per job only, and every drain warp arrives
-// there once per job: a drain warp whose own wait gave up arrives for all its jobs left.
+// timeout and count arrivals, not jobs, so their rule is exact: every drain warp arrives
+// once for each job that was issued, in order, and only after it was (job_ready).  A drain
+// warp whose wait gave up therefore goes on arriving, without looking at the values, until
+// the issuers have left; these leave at their next mbarrier wait that is not yet complete,
+// at most kEStages units later, because the loader stops at the abort.
 #pragma once
 #include <cstdint>
 
@@ -127,6 +130,11 @@ constexpr uint32_t kEmptyThreads = 32 * (kEpiWarps + 1);  // the drain warps and
 constexpr int kChunkBlocks = 8;  // streamed A: k-steps per chunk
 constexpr int kChunks = 4;       // streamed A: chunks in the ring
 
+// Test hook (blamm_debug_stall): the issuers before their first job; and, in the raw-score
+// instance only, at a CTA's unit number u (the value is role | u << 8): all drain warps, one
+// of them, the loader, one issuer, the loader between a unit's entries and its streamed A.
+enum { kStallIssuers = 1, kStallDrains, kStallDrain, kStallLoader, kStallIssuer, kStallChunks, kStallEnd };
+
 // Per-tile description (host-built, read through the read-only path).
 struct TileDesc {
     int32_t g;    // k-steps per term: ceil(longest motif in the tile / 4 (BF16) or 8 (E4M3))
@@ -153,7 +161,7 @@ struct TcParams {
     int64_t cand_cap;                 // record slots available (a multiple of kRecBlock, one spare block behind them)
     int *status;         // bit 0: a device wait timed out
     long long wait_limit;  // clock64 cycles a wait may last
-    int32_t debug_stall;   // test hook: the issuers first wait on a barrier nobody completes
+    int32_t debug_stall;   // test hook: who waits on a barrier nobody completes (kStall*)
     // debug dump of the accumulator (positions [dump_p0, dump_p0+dump_npos))
     float *dump;
     int64_t dump_p0, dump_npos;
@@ -178,7 +186,8 @@ enum {
     CTL_ABORT = 0,     // set by the first wait that times out
     CTL_TMEM = 1,      // TMEM base address
     CTL_DONE = 2,      // drain warps that have finished
-    CTL_BLOCK = 4,     // per drain warp: its next record block (kNoBlock: none yet)
+    CTL_LEFT = 3,      // per accumulator: its issuer has left its loop
+    CTL_BLOCK = 5,     // per drain warp: its next record block (kNoBlock: none yet)
     CTL_WORDS = CTL_BLOCK + kEpiWarps
 };
 
@@ -278,6 +287,20 @@ struct UnitIter {
     }
 };
 
+// For a drain warp after an abort: waits until the job's accumulator is ready (true: the warp
+// arrives for it) or its issuer has left (false: nobody will wait for this accumulator again).
+// Every other wait of the CTA ends at the abort flag, so one of the two comes soon; should an MMA
+// never complete, the wait ends after limit_cycles, with the issuer at the barrier for this job.
+__device__ __noinline__ bool job_ready(uint32_t bar, uint32_t parity, volatile int *left, long long limit_cycles)
+{
+    const long long t0 = clock64();
+    for (;;) {
+        if (__all_sync(0xffffffffu, ptx::mbar_try_wait_nohint(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *left != 0)) return false;
+        if (__any_sync(0xffffffffu, clock64() - t0 > limit_cycles)) return true;
+    }
+}
+
 template <bool kProf>
 __device__ __forceinline__ long long tick()
 {
@@ -340,6 +363,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
     constexpr uint32_t kStep16 = kStepBytes / 16;  // one k-step of A in 16 B units
     UnitIter it;
     it.init(p, ngroups);
+    int unit = 0;  // (test hook) this CTA's units so far
+    auto stalls = [&](int role) { return kDump && p.debug_stall == (role | unit << 8); };
+    auto never = [&]() { return ptx::mbar_wait(bars + 8 * BAR_NEVER, 0, s_abort, p.wait_limit); };
 
     if (warp == kMmaWarp || warp == kMmaWarp2) {
         // ============ MMA issuers: warp 19 the even jobs, warp 18 the odd ones ============
@@ -363,10 +389,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         };
         const uint32_t e_step = (uint32_t)p.erows;  // one E stage in 16 B units
         bool ok = true;
-        if (p.debug_stall) ok = ptx::mbar_wait(bars + 8 * BAR_NEVER, 0, s_abort, p.wait_limit);
+        if (p.debug_stall == kStallIssuers) ok = never();
         ok = __all_sync(0xffffffffu, ok);
         if (kStream && mine == 1u) ok = false;  // one issuer walks the ring
-        for (; it.u < it.end && ok; it.next(p.nblocks)) {
+        for (; it.u < it.end && ok; it.next(p.nblocks), ++unit) {
+            if (stalls(kStallIssuer) && mine == (kStream ? 0u : 1u)) {
+                ok = __all_sync(0xffffffffu, never());
+                if (!ok) break;
+            }
             if (it.group != cur_group) {
                 const long long tb = tick<kProf>();
                 if (!kStream) {
@@ -396,7 +426,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
                 if (kStream || (jc & 1u) == mine) {
                     const uint32_t s = jc & 1u;  // accumulator
                     const long long ta = tick<kProf>();
-                    // (returns after an abort too: the drain warps then arrive for every job left)
+                    // (returns after an abort too: the drain warps still arrive for every job issued)
                     if (jc >= 2u) ptx::named_sync(kBarEmpty + s, kEmptyThreads);
                     if (kProf) t_acc += tick<kProf>() - ta;
                     ptx::tc_fence_after();
@@ -440,6 +470,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
                 eph ^= 1u;
             }
         }
+        // the drain warps need not wait for jobs of this issuer any more
+        if (lane == 0 && (!kStream || mine == 0u)) {
+            ctl[CTL_LEFT + mine] = 1;
+            if (kStream) ctl[CTL_LEFT + 1] = 1;
+        }
         // drain: nothing may still write TMEM or shared memory when they are freed
         ptx::mma_commit_elect(bars + 8 * (BAR_DRAIN + mine));
         if (!ptx::mbar_wait_drain(bars + 8 * (BAR_DRAIN + mine), 0, p.wait_limit)) *s_abort = 1;
@@ -464,7 +499,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         long long t_we = 0, t_tile = 0;
         const uint8_t *a_src = nullptr;
         uint32_t a_len = 0;
-        for (; it.u < it.end && ok; it.next(p.nblocks)) {
+        for (; it.u < it.end && ok; it.next(p.nblocks), ++unit) {
+            if (*s_abort) break;  // (the issuers then run out of entries)
+            if (stalls(kStallLoader) && !never()) break;
             if (it.group != cur_group) {
                 const int t0 = it.group * p.tg, t1 = min(t0 + p.tg, p.ntiles);
                 a_src = p.abuf + (int64_t)p.tiles[t0].off * kStepBytes;
@@ -501,7 +538,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
             }
             if constexpr (kStream) {
                 for (uint32_t o = 0; o < a_len; o += kChunkBlocks * kStepBytes) {
-                    ok = ptx::mbar_wait(bars + 8 * (BAR_CEMPTY + cs), cph ^ 1u, s_abort, p.wait_limit);
+                    if (stalls(kStallChunks)) ok = never();
+                    else ok = ptx::mbar_wait(bars + 8 * (BAR_CEMPTY + cs), cph ^ 1u, s_abort, p.wait_limit);
                     if (!ok) break;
                     const uint32_t len = min((uint32_t)(kChunkBlocks * kStepBytes), a_len - o);
                     ptx::mbar_arrive_expect_tx(bars + 8 * (BAR_CFULL + cs), len);
@@ -530,8 +568,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         }
     } else if (warp == kBlockWarp) {
         // ============ record blocks: one ahead for every drain warp ============
+        long long gone = 0;  // when the abort was seen
         for (bool done = false; !done;) {
             done = ctl[CTL_DONE] == kEpiWarps;  // (read first: no block is taken after that)
+            if (*s_abort) {  // (the drain warps' waits end too; should they not, this one does)
+                if (gone == 0) gone = clock64();
+                done = done || clock64() - gone > 64 * p.wait_limit;
+            }
+            done = __any_sync(0xffffffffu, done);
             if (lane < kEpiWarps) {
                 const uint32_t b = (uint32_t)ctl[CTL_BLOCK + lane];
                 if (done) {  // every reserved block states its count
@@ -578,7 +622,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         int cur_group = -1, t0 = 0, t1 = 0;
         float thr_next = 0.f;
         bool ok = true;
-        for (; it.u < it.end && ok; it.next(p.nblocks)) {
+        for (; it.u < it.end && ok; it.next(p.nblocks), ++unit) {
             if (it.group != cur_group) {
                 cur_group = it.group;
                 t0 = cur_group * p.tg;
@@ -592,13 +636,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
                 thr_next = __ldg(lane_thr + (t + 1 < t1 ? t + 1 : t0) * kTileCols);
                 const uint32_t slot = (uint32_t)t * kTileCols + row;
                 const long long ta = tick<kProf>();
-                ok = ptx::mbar_wait_nohint(bars + 8 * (BAR_AFULL + s), ph, s_abort, p.wait_limit);
-                if (!ok) {  // aborted: the issuers wait once per job, whatever happens
-                    for (; it.u < it.end; it.next(p.nblocks)) {
+                if (t == t0 && (stalls(kStallDrains) || (stalls(kStallDrain) && warp == 5))) ok = never();
+                else ok = ptx::mbar_wait_warp(bars + 8 * (BAR_AFULL + s), ph, s_abort, p.wait_limit);
+                if (!ok) {  // aborted: the jobs already issued, or about to be, are still handed back
+                    for (uint32_t gone = 0; it.u < it.end && gone != 3u; it.next(p.nblocks), t = 0) {
                         t0 = it.group * p.tg;
                         t1 = min(t0 + p.tg, p.ntiles);
-                        for (t = t < t0 ? t0 : t; t < t1; ++t, s ^= 1u) ptx::named_arrive(kBarEmpty + s, kEmptyThreads);
-                        t = 0;
+                        for (t = t < t0 ? t0 : t; t < t1; ++t) {
+                            if (!((gone >> s) & 1u)) {
+                                if (job_ready(bars + 8 * (BAR_AFULL + s), ph, ctl + CTL_LEFT + s, 4 * p.wait_limit))
+                                    ptx::named_arrive(kBarEmpty + s, kEmptyThreads);
+                                else gone |= 1u << s;
+                            }
+                            s ^= 1u;
+                            ph ^= s ^ 1u;
+                        }
                     }
                     break;
                 }

@@ -304,8 +304,11 @@ int blamm_guard_band(const blamm_ctx *ctx, float *out);
  * changes, 15 its candidate test and record writing).  *nctas receives the
  * CTA count.  The timing variant of the kernel is slower than the scan itself. */
 int blamm_debug_profile(blamm_ctx *ctx, int enable);
-/* Failure-path test hook: with enable = 1 the tensor-core scan kernel first
- * waits on a barrier that nothing completes; every wait of the kernel gives up
+/* Failure-path test hook: with enable = 1 the tensor-core scan kernel's MMA issuers
+ * first wait on a barrier that nothing completes; with enable = role | u << 8 a role does
+ * so at unit u of its CTA (2 all drain warps, 3 one of them, 4 the loader, 5 one issuer, 6
+ * the loader between a unit's entries and its streamed motif tile); every wait of the
+ * kernel gives up
  * after wait_limit_cycles (0 = the default, about 2 s of clock64 cycles), the
  * CTAs drain their copies and MMAs, free their tensor memory and the call
  * returns BLAMM_ERR_TIMEOUT; the context stays usable.  enable = 0 restores
