@@ -1585,6 +1585,7 @@ static bool hist_tc_fits(const blamm_ctx *ctx, int64_t n, const float *min_score
         auto usual = [](double x) { return x > 0x1p-60 && x < 0x1p60; };  // (false for NaN)
         if (!usual(w) || !(std::fabs(mn) < 0x1p60) || !(top == 0.f || usual(top))) return false;
         const int k = top == 0.f ? 0 : 7 - column_exponent(P, L);
+        if (std::ldexp((double)top, k) > 128.0) return false;  // (column_exponent stops at 2^40: hi would not be exact)
         // how far the scaled score can be off in bins: the terms' grid, the FP32 sum's own
         // rounding, the roundings of the factor, the offset and the bin's formula (generous)
         const double eps = (std::ldexp((double)L, -k - 9) + 0x1p-20 * (sum + std::fabs(mn))) / w + 0x1p-20 * nbins + L * 0x1p-24 * sum / w;
