@@ -52,7 +52,8 @@ struct blamm_ctx {
     int sm_count = 0;
     int max_smem = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};  // the kernels' start and end, the plain scan's start
+    std::vector<cudaEvent_t> win_ev;  // per timed scan window: its scan kernel's start and end
     std::string err;
     int mode = BLAMM_MODE_AUTO;
     int auto_terms = 1;  // BLAMM_MODE_AUTO: the form in use, 1 or 2 BF16 terms or kE4M3 (1 until tuned)
@@ -568,6 +569,7 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
         if (b) cudaFree(b);
     for (auto &ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
+    for (auto &ev : ctx->win_ev) cudaEventDestroy(ev);
     for (auto &ev : ctx->chunk_ev)
         if (ev) cudaEventDestroy(ev);
     for (auto &ev : ctx->done_ev)
@@ -916,12 +918,48 @@ static void launch_tc(const TcParams &p, bool dump, int grid, uint32_t smem, cud
     else launch_tc_as<false, false, kStream>(p, grid, smem, st);
 }
 
+// Scan windows whose scan kernel is timed: the last one and those before it up to this number (2 Gi
+// positions by default); more are taken to run at the same rate.
+constexpr int64_t kTimedWindows = 128;
+
+static int64_t scan_windows(const blamm_ctx *ctx, int64_t n)
+{
+    const int64_t wb = std::max<int64_t>(1, ctx->ewindow / kBlockPos);
+    return (scan_blocks(n) + wb - 1) / wb;
+}
+
+// The pair of events of window w, -1: it is not timed.
+static int64_t window_pair(int64_t w, int64_t windows)
+{
+    return w == windows - 1 ? std::min(windows, kTimedWindows) - 1 : w < kTimedWindows - 1 ? w : -1;
+}
+
+// Device time of the scan kernels alone (blamm_stats.scan_ms).
+static float scan_kernels_ms(const blamm_ctx *ctx, int64_t n)
+{
+    const int64_t windows = scan_windows(ctx, n), pairs = std::min(windows, kTimedWindows);
+    float sum = 0.f;
+    for (int64_t k = 0; k < pairs; ++k) {
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ctx->win_ev[2 * k], ctx->win_ev[2 * k + 1]);
+        sum += ms;
+    }
+    return windows == pairs ? sum : (float)(sum * (double)n / (double)(n - (windows - pairs) * ctx->ewindow));
+}
+
 // The scan of n bases (p: the plan, candidates, counters, status; a: the packed stream and what
 // the first window sets to zero), window by window: the window's packing and one-hot entries
-// (into e16), then its scan launch.  Returns the largest grid used; adds the launches to
-// *launches.
-static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e16, bool dump, int *launches, int *grid_out)
+// (into e16), then its scan launch (timed: between events).  Returns the largest grid used; adds
+// the launches to *launches.
+static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e16, bool dump, int *launches, int *grid_out,
+                             bool timed = false)
 {
+    const int64_t windows = scan_windows(ctx, a.n);
+    while (timed && (int64_t)ctx->win_ev.size() < 2 * std::min(windows, kTimedWindows)) {
+        cudaEvent_t ev = nullptr;
+        CK(cudaEventCreate(&ev));
+        ctx->win_ev.push_back(ev);
+    }
     const int64_t n = a.n, pack_end = a.pack_end;
     const int64_t nblocks = scan_blocks(n), wb = std::max<int64_t>(1, ctx->ewindow / kBlockPos);
     int gmax = 0;
@@ -951,9 +989,12 @@ static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e1
         const uint32_t smem = std::max<uint32_t>(tc_smem_layout(p.a_bytes, p.erows).total, 116 * 1024);
         if ((int)smem > ctx->max_smem)
             return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", smem, ctx->max_smem);
+        const int64_t pair = timed ? window_pair(b0 / wb, windows) : -1;
+        if (pair >= 0) CK(cudaEventRecord(ctx->win_ev[2 * pair], ctx->stream));
         if (ctx->plan_stream) launch_tc<true>(p, dump, grid, smem, ctx->stream);
         else launch_tc<false>(p, dump, grid, smem, ctx->stream);
         CK(cudaGetLastError());
+        if (pair >= 0) CK(cudaEventRecord(ctx->win_ev[2 * pair + 1], ctx->stream));
         gmax = std::max(gmax, grid);
         if (launches) *launches += 2;
     }
@@ -1056,7 +1097,7 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
     int launches = 0;
     for (int attempt = 0;; ++attempt) {
         launches = 0;
-        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+        CK(cudaEventRecord(ctx->ev[0], ctx->stream));
         if (tc) {
             TcParams p = tc_params(ctx, n);
             p.cand = ctx->d_cand;
@@ -1074,21 +1115,21 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
             }
             int grid = 0;
             const PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 15u);
-            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out || ctx->debug_stall > kStallIssuers, &launches, &grid))) return rc;
-            CK(cudaEventRecord(ctx->ev[5], ctx->stream));
+            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out || ctx->debug_stall > kStallIssuers, &launches, &grid, true)))
+                return rc;
             const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
                                                    d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
             if ((rc = launch_rescore(ctx, r, n, grid))) return rc;
             ctx->prof_ctas = ctx->prof_on ? grid : ctx->prof_ctas;
         } else {
             if ((rc = launch_pack(ctx, d_bases, n, cnt, 15u))) return rc;
-            CK(cudaEventRecord(ctx->ev[5], ctx->stream));
+            CK(cudaEventRecord(ctx->ev[2], ctx->stream));
             PlainParams p = plain_params(ctx, ctx->d_seq2, ctx->d_zmask, n, d_runs, nruns, d_hits, hit_cap, cnt + 1);
             if ((rc = launch_plain<false>(ctx, p))) return rc;
             ++launches;  // (packing)
         }
         ++launches;
-        CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+        CK(cudaEventRecord(ctx->ev[1], ctx->stream));
         CK(cudaMemcpyAsync(back ? back : got, cnt, back ? kHitsAt + fetch : sizeof got, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         if (back) std::memcpy(got, back, sizeof got);
@@ -1108,12 +1149,13 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
     }
     const int64_t nh = (int64_t)got[1];
     if (tc) ctx->stats.candidates = (int64_t)got[3];
-    cudaEventElapsedTime(&ctx->stats.kernel_ms, ctx->ev[1], ctx->ev[2]);
+    cudaEventElapsedTime(&ctx->stats.kernel_ms, ctx->ev[0], ctx->ev[1]);
     if (tc) {
-        cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[1], ctx->ev[5]);
-        cudaEventElapsedTime(&ctx->stats.rescore_ms, ctx->ev[5], ctx->ev[2]);
+        ctx->stats.scan_ms = scan_kernels_ms(ctx, n);
+        const int64_t last = std::min(scan_windows(ctx, n), kTimedWindows) - 1;
+        cudaEventElapsedTime(&ctx->stats.rescore_ms, ctx->win_ev[2 * last + 1], ctx->ev[1]);
     } else {
-        cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[5], ctx->ev[2]);
+        cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[2], ctx->ev[1]);
     }
     ctx->stats.hits = nh;
     ctx->stats.tiles = (int32_t)(tc ? ctx->ntiles : 0);
@@ -1347,7 +1389,7 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         }
         return BLAMM_OK;
     };
-    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if ((rc = issue_in(0))) return rc;
     for (int64_t k = 0; k < nchunks; ++k) {
         const int b = (int)(k & 1);
@@ -1367,7 +1409,7 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         CK(cudaEventRecord(ctx->done_ev[b], ctx->stream));
         if (k >= 1 && (rc = drain_out(k - 1))) return rc;
     }
-    CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+    CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     if ((rc = drain_out(nchunks - 1))) return rc;
     CK(cudaStreamSynchronize(ctx->copy_stream));  // the hits are in host memory
     blamm_stats total{};
@@ -1386,7 +1428,7 @@ static int scan_host_async_steps(blamm_ctx *ctx, const char *bases, int64_t n, c
         if (tc && nc > ctx->cand_cap) *cand_overflow = std::max(*cand_overflow, nc);
         status |= (int)(hc_k[4 * k + 2] & 0xffffffffu);
     }
-    cudaEventElapsedTime(&total.kernel_ms, ctx->ev[1], ctx->ev[2]);
+    cudaEventElapsedTime(&total.kernel_ms, ctx->ev[0], ctx->ev[1]);
     const int64_t nh_total = (int64_t)hc_k[4 * (nchunks - 1) + 1];
     total.hits = nh_total;
     ctx->stats = total;
@@ -1465,6 +1507,7 @@ static int scan_host_once(blamm_ctx *ctx, const char *bases, const char *d_bases
                            ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
     }
+    // (by the host's clock: a pair of events around the copies took 5 us of a 58 us call)
     ctx->stats.total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return rc;
 }

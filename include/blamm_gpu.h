@@ -72,9 +72,9 @@ typedef struct {
     int32_t tiles;       /* motif tiles (up to 128 columns each) */
     int32_t launches;    /* kernels launched by the last scan */
     float kernel_ms;     /* device time of all kernels of the call (CUDA events) */
-    float total_ms;      /* time of the whole call incl. copies (device events; wall time
-                            when blamm_scan pipelines a long stream in chunks) */
-    float scan_ms;       /* device time of the scan (tcgen05: with packing and one-hot entries; or plain FP32) */
+    float total_ms;      /* time of the whole call incl. copies, by the host's clock (scans of
+                            host streams and of the resident stream) */
+    float scan_ms;       /* device time of the scan kernel alone (tcgen05 or plain FP32) */
     float rescore_ms;    /* device time of the rescoring kernel (tcgen05 modes) */
 } blamm_stats;
 
