@@ -876,8 +876,8 @@ def run_ours(a, rank, world, local):
     peak, peak_src = peaks()
     kern_ms = float(np.mean(scan_ms))
     achieved = n * flops_per_bp / (kern_ms / 1e3) / 1e12
-    # a step = packing + (one-hot entries + scan) per scan window + rescoring
-    scan_launches = max(1, (launches // a.steps - 1) // 2)  # per window: preparation and scan; one rescoring
+    # a step = (preparation: packing and one-hot entries; scan) per scan window + rescoring
+    scan_launches = max(1, (launches // a.steps - 1) // 2)
     traffic = profile_traffic(int(round(n / scan_launches)), terms)
 
     line = {
@@ -916,7 +916,7 @@ def run_ours(a, rank, world, local):
                              + (f"{terms} BF16 term(s) issue {terms} MMA(s) per flop (ceiling {1 / terms:g} "
                                 if terms in (1, 2) else "one E4M3 term: half the BF16 MMA instructions per flop "
                                 "at twice the BF16 rate (ceiling 2 of the BF16 peak ")
-                             + f"before padding and the bias MMA); peak {peak_src}"},
+                             + f"before padding); peak {peak_src}"},
         "modes": modes,
         "score_error_vs_fp64": precision,
         "clocks": clk,
