@@ -10,9 +10,10 @@
 //     min { sum(q) : sum(P) >= thr' } >= lambda thr' + sum_j min_b (q_jb - lambda P_jb)
 // (Lagrangian bound; a masked base is a fifth choice with q = P = 0).  lambda = 1 is the worst
 // case above; the best lambda is usually a few thousandths (BF16) or hundredths (E4M3) more.
-// A warp takes the largest bound over 64 values of lambda, less a margin for its own FP32
-// arithmetic, or the worst case where that is larger.  Candidates per hit on a 512-motif bank:
-// E4M3 1.87 -> 1.13 at p = 1e-4 and 1.96 -> 1.01 at 1e-5, one BF16 term 1.24 -> 1.06.
+// A warp compares 64 values of lambda in FP32 and then forms the bound of the best one in FP64, or
+// takes the worst case where that is larger.  (Which lambda it is decides how tight the bound is,
+// not whether it holds.)  Candidates per hit, 512 motifs x 16 Mi positions at p = 1e-4, by the worst
+// case and so: E4M3 2.03, 1.17; one BF16 term 1.25, 1.11.
 #pragma once
 #include <cstdint>
 
@@ -49,6 +50,30 @@ __device__ __forceinline__ float e4m3_units_f(uint32_t code)
     return code & 0x80u ? -a : a;
 }
 
+// Entry b of motif position j of a column, in units of 2^-s: the quantised value and P.
+struct PlanEntry {
+    double q, x;
+};
+__device__ __forceinline__ PlanEntry plan_entry(const PlanParams &p, const float *P, uint32_t o, int s, int i)
+{
+    PlanEntry e;
+    e.x = ldexp((double)__ldg(P + i), s);
+    if (p.terms == kE4M3) {
+        e.q = (double)e4m3_units_f(__ldg(p.e8 + o + i));
+    } else {
+        e.q = ldexp((double)__uint_as_float((uint32_t)__ldg(p.hi + o + i) << 16), s);
+        if (p.terms == 2) e.q += ldexp((double)__uint_as_float((uint32_t)__ldg(p.lo + o + i) << 16), s);  // exact
+    }
+    return e;
+}
+
+__device__ __forceinline__ double warp_sum(double v)
+{
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    return v;
+}
+
 // One warp per slot: its threshold.
 __global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
 {
@@ -63,7 +88,7 @@ __global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
     const int L = p.col_len[c], s = p.k[c] + (e8 ? 9 : 8);  // everything below in units of 2^-s
     const float *P = p.P + (size_t)c * p.p_rows;
     const uint32_t o = p.off[c];
-    // lambda: 0, 1 - d, 1, 1 + d with d in powers of 2^(3/8) from 2^-14
+    // lambda: 0, 1 - d for 14 values of d from 1/2 down to 2^-12.4, 1, 1 + d for 48 from 2^-14 up to 3.9
     float lam[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -73,25 +98,21 @@ __global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
                  : i < 16  ? 1.0f - exp2f(-1.0f - 0.875f * (float)(i - 2))
                            : 1.0f + exp2f(-14.0f + 0.34f * (float)(i - 16));
     }
-    float sum[2] = {0.f, 0.f}, mag = 0.f, maxabs = 0.f;
+    // each lane's two lambdas, in FP32: which one is best
+    float sum[2] = {0.f, 0.f};
     for (int j = 0; j < L; ++j) {
-        float q[4], x[4], mq = 0.f, mx = 0.f;
+        float q[4], x[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const float v = __ldg(P + 4 * j + b);
-            const uint32_t at = o + 4 * j + b;
-            x[b] = ldexpf(v, s);
+            const int i = 4 * j + b;
+            x[b] = ldexpf(__ldg(P + i), s);
             if (e8) {
-                q[b] = e4m3_units_f(__ldg(p.e8 + at));
+                q[b] = e4m3_units_f(__ldg(p.e8 + o + i));
             } else {
-                q[b] = ldexpf(__uint_as_float((uint32_t)__ldg(p.hi + at) << 16), s);
-                if (p.terms == 2) q[b] += ldexpf(__uint_as_float((uint32_t)__ldg(p.lo + at) << 16), s);  // exact
+                q[b] = ldexpf(__uint_as_float((uint32_t)__ldg(p.hi + o + i) << 16), s);
+                if (p.terms == 2) q[b] += ldexpf(__uint_as_float((uint32_t)__ldg(p.lo + o + i) << 16), s);
             }
-            mq = fmaxf(mq, fabsf(q[b]));
-            mx = fmaxf(mx, fabsf(x[b]));
         }
-        maxabs += mx;
-        mag += mq + mx;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float m = 0.f;
@@ -100,24 +121,43 @@ __global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
             sum[h] += m;
         }
     }
-    // the reference's own rounding: |fl(sum) - sum| <= (L - 1) 2^-24 sum |P| (1 + 2^-14)
-    const float thr = ldexpf(p.thr[c], s) - (float)L * 0x1p-24f * maxabs;
-    float best = __int_as_float(0xff800000);
+    const float thr32 = ldexpf(p.thr[c], s);
+    const float v0 = fmaf(lam[0], thr32, sum[0]), v1 = fmaf(lam[1], thr32, sum[1]);
+    float best = v1 > v0 ? v1 : v0, l32 = v1 > v0 ? lam[1] : lam[0];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const float l = fmaxf(lam[h], 1.0f);
-        const float margin = (float)(L + 8) * 0x1p-23f * l * (fabsf(thr) + mag);
-        best = fmaxf(best, fmaf(lam[h], thr, sum[h]) - margin);  // (NaN: not taken)
+    for (int d = 16; d > 0; d >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, d), ol = __shfl_xor_sync(0xffffffffu, l32, d);
+        if (ob > best || (ob == best && ol < l32) || best != best) best = ob, l32 = ol;
     }
+    // its bound in FP64, motif positions over the lanes (all lanes then have the sums)
+    const double l = __shfl_sync(0xffffffffu, l32, 0);
+    double sum64 = 0.0, mag = 0.0, maxabs = 0.0;
+    for (int j = lane; j < L; j += 32) {
+        double m = 0.0, mq = 0.0, mx = 0.0;
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, d));
+        for (int b = 0; b < 4; ++b) {
+            const PlanEntry e = plan_entry(p, P, o, s, 4 * j + b);
+            m = fmin(m, fma(-l, e.x, e.q));
+            mq = fmax(mq, fabs(e.q));
+            mx = fmax(mx, fabs(e.x));
+        }
+        sum64 += m;
+        maxabs += mx;
+        mag += mq + l * mx;
+    }
+    sum64 = warp_sum(sum64);
+    mag = warp_sum(mag);
+    maxabs = warp_sum(maxabs);
     if (lane != 0) return;
+    // the reference's own rounding: |fl(sum) - sum| <= (L - 1) 2^-24 sum |P| (1 + 2^-14)
+    const double thr = ldexp((double)p.thr[c], s) - (double)L * 0x1p-24 * maxabs;
+    const double bound = fma(l, thr, sum64) - (double)(L + 8) * 0x1p-51 * (l * fabs(thr) + mag);  // (FP64's own rounding)
     // down to the grid, kept within the scores a window can reach (2^23 units; 64 L scaled):
     // below them every window is a candidate, above them none is
     const double worst = ((double)p.thr[c] - p.guard[c]) * exp2((double)s);
     const double lim = e8 ? (double)(64 * L + 1) * 512.0 : 8388608.0;
     double t = worst;
-    if ((double)best > t) t = (double)best;
+    if (bound > t) t = bound;  // (NaN: not taken)
     const double units = isnan(t) ? lim : floor(fmax(-lim, fmin(lim, t)));
     p.slot_thr[slot] = ldexpf((float)units, e8 ? -9 : -s);  // exact: |units| <= 2^23
 }
