@@ -142,7 +142,7 @@ struct blamm_ctx {
     int64_t stream_n = 0, stream_nruns = 0, stream_nseqs = 0;
     uint8_t *d_theo = nullptr;  // theoretical histograms: bank, tables, results of a call
     size_t cap_theo = 0;
-    // FASTA parsing: tile summaries, the parser before each tile, totals (96 bytes per 16 KB of text)
+    // FASTA parsing: tile summaries, the parser before each tile, totals (4,704 bytes per 32 KB of text)
     uint4 *d_ing_tiles = nullptr;  // the tiles' sums (IngTile)
     IngPrefix *d_ing_prefix = nullptr;
     unsigned long long *d_ing_totals = nullptr;

@@ -233,8 +233,9 @@ int blamm_fasta_parse_device(blamm_ctx *ctx, const char *d_raw, int64_t nraw, ch
  * (FastaBatch's filtered stream, src/sequence.cpp:142-293); the stream, its run table and
  * the header offsets replace the context's previous resident stream.  *n_bases, *nruns,
  * *nseqs and nucl_counts[4] (may be NULL) as blamm_fasta_parse_device returns them.
- * Device memory: nraw + n_bases + 8 x (3 nruns + nseqs) bytes kept, and 96 bytes per 16 KB
- * of text.  blamm_release_buffers drops the resident stream.
+ * Device memory: nraw + n_bases + 8 x (3 nruns + nseqs) bytes, and 4,704 bytes for every 32 KB
+ * of text begun (a seventh of it) as the parser's workspace; both are kept until
+ * blamm_release_buffers, which drops the resident stream.
  *
  * blamm_stream_tables: the run table (stream position, sequence index, position inside
  * the sequence; nruns entries each) and the header offsets (byte offset of each '>' in
