@@ -254,10 +254,6 @@ namespace {
 // up to 256 motif positions is an integer multiple of 2^-(k+8) below 2^24 of
 // those units, i.e. exactly representable in FP32: the tensor-core
 // accumulation is exact, whatever its internal rounding.
-struct ColQuant {
-    int k;
-};
-
 int column_exponent(const float *col, int L)
 {
     double mx = 0.0;

@@ -57,22 +57,16 @@
 // hand-off: commit -> drain warps awake (~250 cycles) -> their TMEM loads (~180) ->
 // all 16 have handed back -> the issuer issues (~120).  A drain warp that met a
 // candidate is late for the next job, and one of the 16 nearly always has, so the
-// rare path's latency counts in full.  Measured over 16 Mi positions x 1024 columns,
-// ms (BF16, E4M3, two BF16 terms): motifs as columns of 256-wide tiles, bias MMAs
-// 2.04, 2.05, 2.80; motifs as rows, hand-back by mbarrier arrivals 1.59, 1.56, 2.51;
-// hand-back by hardware barriers (16 arrivals on a shared-memory mbarrier queue behind
-// the tensor cores' operand reads; the issuer saw the last one ~300 cycles late) 1.51,
-// 1.48, 2.48; masks in eight short chains, predicated stores, one room check per round,
-// no shared memory in the issuers' loop, issuers off the loader's sub-partition 1.42,
-// 1.33, 2.41; fewer candidates (tighter thresholds) 1.40, 1.20, 2.41; record blocks
-// reserved by a warp of their own and a warp index that is known to be uniform 1.35,
-// 1.15, 2.39.  Of that, E4M3: without the mask arithmetic 0.96, without the whole rare
-// path 0.78; the records' stores cost nothing.  MMAs alone 1.20, 0.74, 2.39.
-// Measured and not kept: accumulators of 128 columns (four stages; an MMA of N = 128
-// takes 1.1-1.2 times its share and every barrier is met twice as often) with 16, 20 or
-// 24 drain warps 1.5-1.9; TMEM loads of 16 columns, so that a candidate costs half a mask,
-// 1.28 against 1.15 (E4M3), of 64 columns 1.35 against 1.33; the rare values through a
-// shared-memory queue 2.2; one issuer 1.64 (BF16).
+// rare path's latency counts in full: masks in eight short chains, predicated stores,
+// record blocks reserved by a warp of their own, no shared memory in the issuers' loop.
+// The hand-back is a hardware barrier because 16 arrivals on a shared-memory mbarrier
+// queue behind the tensor cores' operand reads.  16 Mi positions x 1024 columns, ms, scan
+// kernel alone (BF16, E4M3, two BF16 terms): 1.31, 1.11, 2.34, of which MMAs alone 1.20,
+// 0.74, 2.34.  With the motifs as columns of 256-wide tiles and bias MMAs the scan took
+// 2.0, 2.0, 2.8 with the entries' kernel in it.
+// Slower: accumulators of 128 columns (an MMA of N = 128 takes 1.1-1.2 times its share and
+// every barrier is met twice as often), TMEM loads of 16 or 64 columns, the rare values
+// through a shared-memory queue, one issuer.
 //
 // A drain warp hands its accumulator back right after its two TMEM loads; a chunk
 // holds a candidate iff the maximum that the load returns reaches the lane's
