@@ -61,8 +61,8 @@
 // record blocks reserved by a warp of their own, no shared memory in the issuers' loop.
 // The hand-back is a hardware barrier because 16 arrivals on a shared-memory mbarrier
 // queue behind the tensor cores' operand reads.  16 Mi positions x 1024 columns, ms, scan
-// kernel alone (BF16, E4M3, two BF16 terms): 1.31, 1.11, 2.34, of which MMAs alone 1.20,
-// 0.74, 2.34.  With the motifs as columns of 256-wide tiles and bias MMAs the scan took
+// kernel alone (BF16, E4M3, two BF16 terms): 1.31, 1.11, 2.34, the tensor pipe busy for
+// 87, 56 and 97 % of it.  With the motifs as columns of 256-wide tiles and bias MMAs the scan took
 // 2.0, 2.0, 2.8 with the entries' kernel in it.
 // Slower: accumulators of 128 columns (an MMA of N = 128 takes 1.1-1.2 times its share and
 // every barrier is met twice as often), TMEM loads of 16 or 64 columns, the rare values
