@@ -978,6 +978,14 @@ static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e1
         p.tg = (ctx->ntiles + ng - 1) / ng;
         const int grid = (int)std::min<int64_t>(ctx->sm_count, (int64_t)ng * nb);
         p.contiguous = nb < grid ? 1 : 0;
+        // Two BF16 terms, a few tiles a unit, the longest of them (2 g MMAs of 128 cycles) longer than
+        // the hand-off of an accumulator (about 1200 cycles): every other unit takes its tiles in
+        // reverse.  Taken in one order, the short tiles follow one another on the same accumulator
+        // and a unit's last job is too short to hide the hand-off of the long one before it.  30 Mbp,
+        // scan kernel, ms: 130 columns of 5-30 positions 1.26 -> 1.20, 140 of 8-30 1.37 -> 1.21, 300
+        // 1.89 -> 1.67; no gain from six tiles on (1024 columns: 1.157, 1.155 at 8 Mbp), a loss with
+        // short motifs (130 of 8-14, 8 Mbp: 0.180, 0.207) and with one term or E4M3 (0.67, 0.82).
+        p.turn = p.terms == 2 && p.tg >= 2 && p.tg <= 5 && ctx->tiles[0].g >= 6 ? 1 : 0;
         // (the longest tiles come first: the first group is the largest)
         const int steps = ctx->tiles[std::min(p.tg, ctx->ntiles)].off;
         p.a_bytes = (uint32_t)(ctx->plan_stream ? kChunks * kChunkBlocks : steps) * kStepBytes;

@@ -144,6 +144,7 @@ struct TcParams {
     int32_t ntiles;
     int32_t tg;          // tiles per group
     int32_t contiguous;  // 1: each CTA takes consecutive units
+    int32_t turn;        // 1 (two BF16 terms only): every other unit takes its tiles in reverse
     int32_t terms;       // 1 (hi) or 2 (hi + lo) or kE4M3
     const uint8_t *abuf; // A tiles
     const int32_t *slot_col;  // per slot (tile * 128 + row): motif column, -1 for padding
@@ -357,6 +358,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
     constexpr uint32_t kStep16 = kStepBytes / 16;  // one k-step of A in 16 B units
     UnitIter it;
     it.init(p, ngroups);
+    const bool turn = kTerms == 2 && !kStream && p.turn != 0;
     int unit = 0;  // (test hook) this CTA's units so far
     auto stalls = [&](int role) { return kDump && p.debug_stall == (role | unit << 8); };
     auto never = [&]() { return ptx::mbar_wait(bars + 8 * BAR_NEVER, 0, s_abort, p.wait_limit); };
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
             else ptx::mma_bf16_elect(d, a, b, idesc, acc);
         };
         const uint32_t e_step = (uint32_t)p.erows;  // one E stage in 16 B units
-        bool ok = true;
+        bool ok = true, down = false;
         if (p.debug_stall == kStallIssuers) ok = never();
         ok = __all_sync(0xffffffffu, ok);
         if (kStream && mine == 1u) ok = false;  // one issuer walks the ring
@@ -412,9 +414,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
             if (kProf) t_w += tick<kProf>() - te;
             if (!ok) break;
             const uint64_t bdesc = bdesc_e + es * e_step;
-            int2 td = __ldg(reinterpret_cast<const int2 *>(p.tiles) + t0);
-            for (int t = t0; t < t1; ++t, ++jc) {
-                const int2 tn = __ldg(reinterpret_cast<const int2 *>(p.tiles) + t + 1);
+            int2 td = __ldg(reinterpret_cast<const int2 *>(p.tiles) + (down ? t1 - 1 : t0));
+            for (int t = t0; t < t1; ++t, ++jc) {  // (down: tile t0 + t1 - 1 - t)
+                const int2 tn = __ldg(reinterpret_cast<const int2 *>(p.tiles) + (down ? max(t0 + t1 - 2 - t, 0) : t + 1));
                 if (kProf)
                     t_jobs += 2 - (((int64_t)p.chunk0 + it.block * 8 + 4) * 32 >= p.n ? 1 : 0);
                 if (kStream || (jc & 1u) == mine) {
@@ -458,6 +460,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
                 td = tn;
             }
             if (!ok) break;
+            down = turn && !down;
             ptx::mma_commit_elect(bars + 8 * (BAR_EEMPTY + es));
             if (++es == (uint32_t)kEStages) {
                 es = 0;
@@ -615,20 +618,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         const float *lane_thr = p.slot_thr + row;
         int cur_group = -1, t0 = 0, t1 = 0;
         float thr_next = 0.f;
-        bool ok = true;
-        for (; it.u < it.end && ok; it.next(p.nblocks), ++unit) {
+        bool ok = true, down = false;
+        for (; it.u < it.end && ok; it.next(p.nblocks), ++unit, down = turn && !down) {
             if (it.group != cur_group) {
                 cur_group = it.group;
                 t0 = cur_group * p.tg;
                 t1 = min(t0 + p.tg, p.ntiles);
-                thr_next = __ldg(lane_thr + t0 * kTileCols);
+                thr_next = __ldg(lane_thr + (down ? t1 - 1 : t0) * kTileCols);
             }
             const uint32_t chunk = p.chunk0 + (uint32_t)it.block * 8u + 2u * grp;
             for (int t = t0; t < t1; ++t) {
                 // this job's threshold; the next one's arrives during this job
                 const float thr = thr_next;
-                thr_next = __ldg(lane_thr + (t + 1 < t1 ? t + 1 : t0) * kTileCols);
-                const uint32_t slot = (uint32_t)t * kTileCols + row;
+                const int tile = down ? t0 + t1 - 1 - t : t;
+                // (turning, a unit begins with the tile that the one before it ended with)
+                const int tile_next = t + 1 < t1 ? (down ? tile - 1 : t + 1) : turn ? tile : t0;
+                thr_next = __ldg(lane_thr + tile_next * kTileCols);
+                const uint32_t slot = (uint32_t)tile * kTileCols + row;
                 const long long ta = tick<kProf>();
                 if (t == t0 && (stalls(kStallDrains) || (stalls(kStallDrain) && warp == 5))) ok = never();
                 else ok = ptx::mbar_wait_warp(bars + 8 * (BAR_AFULL + s), ph, s_abort, p.wait_limit);
