@@ -44,6 +44,9 @@ using namespace blamm;
 
 static_assert(sizeof(blamm_hit) == sizeof(HitRec), "hit record layout");
 
+// A synchronous scan's counters, and behind them the times that its kernels note (KernelTimes).
+constexpr int kCounts = 4, kTimes = 4;
+
 // Default scan window (positions): see launch_tc_windows.
 constexpr int64_t kEWindowDefault = int64_t(16) << 20;
 
@@ -53,7 +56,6 @@ struct blamm_ctx {
     int max_smem = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};  // the kernels' start and end, the plain scan's start
-    std::vector<cudaEvent_t> win_ev;  // per timed scan window: its scan kernel's start and end
     std::string err;
     int mode = BLAMM_MODE_AUTO;
     int auto_terms = 1;  // BLAMM_MODE_AUTO: the form in use, 1 or 2 BF16 terms or kE4M3 (1 until tuned)
@@ -117,7 +119,7 @@ struct blamm_ctx {
     int64_t cand_cap = 0;     // record slots
     blamm_hit *d_hits = nullptr;
     int64_t hits_cap = 0;
-    unsigned long long *d_counters = nullptr;  // record slots, hits, status (bit 0: a wait timed out), candidates
+    unsigned long long *d_counters = nullptr;  // record slots, hits, status (bit 0: a wait timed out), candidates; times
     // hit filtering of one chunk of a pipelined blamm_scan: hits at chunk positions >=
     // keep_below are dropped (0: none), pos_base is added to the positions written
     int64_t keep_below = 0, pos_base = 0;
@@ -536,7 +538,7 @@ int blamm_ctx_create(int device, blamm_ctx **out)
                                 ctx->max_smem));
         CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         for (auto &ev : ctx->ev) CK(cudaEventCreate(&ev));
-        CK(cudaMalloc(&ctx->d_counters, 4 * sizeof(unsigned long long)));
+        CK(cudaMalloc(&ctx->d_counters, (kCounts + kTimes) * sizeof(unsigned long long)));
         return BLAMM_OK;
     };
     rc = init();
@@ -565,7 +567,6 @@ void blamm_ctx_destroy(blamm_ctx *ctx)
         if (b) cudaFree(b);
     for (auto &ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
-    for (auto &ev : ctx->win_ev) cudaEventDestroy(ev);
     for (auto &ev : ctx->chunk_ev)
         if (ev) cudaEventDestroy(ev);
     for (auto &ev : ctx->done_ev)
@@ -914,48 +915,12 @@ static void launch_tc(const TcParams &p, bool dump, int grid, uint32_t smem, cud
     else launch_tc_as<false, false, kStream>(p, grid, smem, st);
 }
 
-// Scan windows whose scan kernel is timed: the last one and those before it up to this number (2 Gi
-// positions by default); more are taken to run at the same rate.
-constexpr int64_t kTimedWindows = 128;
-
-static int64_t scan_windows(const blamm_ctx *ctx, int64_t n)
-{
-    const int64_t wb = std::max<int64_t>(1, ctx->ewindow / kBlockPos);
-    return (scan_blocks(n) + wb - 1) / wb;
-}
-
-// The pair of events of window w, -1: it is not timed.
-static int64_t window_pair(int64_t w, int64_t windows)
-{
-    return w == windows - 1 ? std::min(windows, kTimedWindows) - 1 : w < kTimedWindows - 1 ? w : -1;
-}
-
-// Device time of the scan kernels alone (blamm_stats.scan_ms).
-static float scan_kernels_ms(const blamm_ctx *ctx, int64_t n)
-{
-    const int64_t windows = scan_windows(ctx, n), pairs = std::min(windows, kTimedWindows);
-    float sum = 0.f;
-    for (int64_t k = 0; k < pairs; ++k) {
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, ctx->win_ev[2 * k], ctx->win_ev[2 * k + 1]);
-        sum += ms;
-    }
-    return windows == pairs ? sum : (float)(sum * (double)n / (double)(n - (windows - pairs) * ctx->ewindow));
-}
-
 // The scan of n bases (p: the plan, candidates, counters, status; a: the packed stream and what
 // the first window sets to zero), window by window: the window's packing and one-hot entries
-// (into e16), then its scan launch (timed: between events).  Returns the largest grid used; adds
-// the launches to *launches.
-static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e16, bool dump, int *launches, int *grid_out,
-                             bool timed = false)
+// (into e16), then its scan launch.  Returns the largest grid used; adds the launches to
+// *launches.
+static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e16, bool dump, int *launches, int *grid_out)
 {
-    const int64_t windows = scan_windows(ctx, a.n);
-    while (timed && (int64_t)ctx->win_ev.size() < 2 * std::min(windows, kTimedWindows)) {
-        cudaEvent_t ev = nullptr;
-        CK(cudaEventCreate(&ev));
-        ctx->win_ev.push_back(ev);
-    }
     const int64_t n = a.n, pack_end = a.pack_end;
     const int64_t nblocks = scan_blocks(n), wb = std::max<int64_t>(1, ctx->ewindow / kBlockPos);
     int gmax = 0;
@@ -965,6 +930,7 @@ static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e1
         a.pack_end = b0 + nb < nblocks ? base + nb * kBlockPos : pack_end;
         a.e = e16;
         a.ne = std::min(nb * kBlockPos, n - base) + kStreamPad - 64;
+        a.first = b0 == 0 ? 1 : 0;
         CK(launch_prep(a, p.terms == kE4M3 ? kE4M3 : 1, ctx->stream));
         a.zero = 0;
         p.e16 = e16;
@@ -993,12 +959,9 @@ static int launch_tc_windows(blamm_ctx *ctx, TcParams p, PrepParams a, uint4 *e1
         const uint32_t smem = std::max<uint32_t>(tc_smem_layout(p.a_bytes, p.erows).total, 116 * 1024);
         if ((int)smem > ctx->max_smem)
             return fail(ctx, BLAMM_ERR_UNSUPPORTED, "shared memory plan %u > %d", smem, ctx->max_smem);
-        const int64_t pair = timed ? window_pair(b0 / wb, windows) : -1;
-        if (pair >= 0) CK(cudaEventRecord(ctx->win_ev[2 * pair], ctx->stream));
         if (ctx->plan_stream) launch_tc<true>(p, dump, grid, smem, ctx->stream);
         else launch_tc<false>(p, dump, grid, smem, ctx->stream);
         CK(cudaGetLastError());
-        if (pair >= 0) CK(cudaEventRecord(ctx->win_ev[2 * pair + 1], ctx->stream));
         gmax = std::max(gmax, grid);
         if (launches) *launches += 2;
     }
@@ -1069,7 +1032,7 @@ static int launch_rescore(blamm_ctx *ctx, const RescoreParams &r, int64_t n, int
 // A host scan's hits lie behind its counters in one buffer, so that the first of them come
 // back in the same copy.
 constexpr size_t kHitsAt = 64;
-static_assert(kHitsAt % sizeof(blamm_hit) == 0, "hits behind the counters");
+static_assert(kHitsAt % sizeof(blamm_hit) == 0 && kHitsAt >= (kCounts + kTimes) * sizeof(unsigned long long), "hits behind the counters");
 
 // Raw accumulators of some positions (the raw-score hook).
 struct ScanDump {
@@ -1087,7 +1050,7 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
 {
     if (ctx->ncols == 0) return fail(ctx, BLAMM_ERR_STATE, "blamm_set_motifs was not called");
     const bool tc = ctx->mode != BLAMM_MODE_FP32;
-    unsigned long long *cnt = d_counters ? d_counters : ctx->d_counters;  // record slots, hits, status, candidates
+    unsigned long long *cnt = d_counters ? d_counters : ctx->d_counters;  // record slots, hits, status, candidates; times
     ctx->stats = blamm_stats{};
     ctx->stats.positions = n;
     ctx->stats.columns = scanned_columns(ctx);
@@ -1097,7 +1060,7 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
         if (ctx->cand_cap == 0 && (rc = ensure_cand(ctx, record_slots_guess(ctx, n)))) return rc;
     }
     if ((rc = ensure_packed(ctx, n, tc))) return rc;
-    unsigned long long got[4] = {0, 0, 0, 0};
+    unsigned long long got[kCounts + kTimes] = {0, 0, 0, 0, 0, 0, 0, 0};
     int launches = 0;
     for (int attempt = 0;; ++attempt) {
         launches = 0;
@@ -1118,11 +1081,13 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
                 p.prof = ctx->d_prof;
             }
             int grid = 0;
-            const PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 15u);
-            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out || ctx->debug_stall > kStallIssuers, &launches, &grid, true)))
+            PrepParams a = prep_params(ctx, d_bases, n, ctx->d_seq2, ctx->d_zmask, cnt, 15u);
+            a.times = p.times = cnt + kCounts;
+            if ((rc = launch_tc_windows(ctx, p, a, ctx->d_e16, dump.out || ctx->debug_stall > kStallIssuers, &launches, &grid)))
                 return rc;
-            const RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
-                                                   d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
+            RescoreParams r = rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
+                                             d_runs, nruns, d_hits, cnt + 1, hit_cap, cnt + 3);
+            r.times = p.times;
             if ((rc = launch_rescore(ctx, r, n, grid))) return rc;
             ctx->prof_ctas = ctx->prof_on ? grid : ctx->prof_ctas;
         } else {
@@ -1155,9 +1120,10 @@ static int scan_core(blamm_ctx *ctx, const char *d_bases, int64_t n, const int64
     if (tc) ctx->stats.candidates = (int64_t)got[3];
     cudaEventElapsedTime(&ctx->stats.kernel_ms, ctx->ev[0], ctx->ev[1]);
     if (tc) {
-        ctx->stats.scan_ms = scan_kernels_ms(ctx, n);
-        const int64_t last = std::min(scan_windows(ctx, n), kTimedWindows) - 1;
-        cudaEventElapsedTime(&ctx->stats.rescore_ms, ctx->win_ev[2 * last + 1], ctx->ev[1]);
+        // the kernels' own clock: preparation begins, scan kernels together, -, rescoring begins
+        const unsigned long long *t = got + kCounts;
+        ctx->stats.scan_ms = 1e-6f * (float)t[1];
+        ctx->stats.rescore_ms = std::max(0.f, ctx->stats.kernel_ms - 1e-6f * (float)(t[3] - t[0]));
     } else {
         cudaEventElapsedTime(&ctx->stats.scan_ms, ctx->ev[2], ctx->ev[1]);
     }

@@ -12,6 +12,14 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The device's clock in ns.
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 {

@@ -79,6 +79,15 @@ __device__ __forceinline__ int64_t run_end_of(const int64_t *run_start, int64_t 
     return lo < nruns ? __ldg(run_start + lo) : n;
 }
 
+// Times of a synchronous scan's kernels, in ns of the device's clock, each noted by one thread of a
+// kernel as it begins: [0] the first preparation, [1] the scan kernels' times added up (a scan lasts
+// until the next kernel begins), [2] the current scan kernel, [3] the rescoring.  (An event between
+// two kernels costs a short call 2 to 7 us; these cost nothing.)
+__device__ __forceinline__ void note_scan_end(unsigned long long *times)
+{
+    times[1] += ptx::global_ns() - times[2];
+}
+
 // ------------------------------------------------------------------------
 // 1. prepare: filtered ASCII bases -> 2-bit codes + zero mask, and the one-hot entries of a
 //    scan window
@@ -122,6 +131,8 @@ struct PrepParams {
     int32_t lower_scores;
     uint32_t zero;       // bit i: counts[i] = 0
     unsigned long long *counts;
+    unsigned long long *times;  // may be null
+    int32_t first;       // the scan's first window
 };
 
 constexpr int kPrepThreads = 256;
@@ -177,6 +188,14 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(PrepParams a)
 {
     __shared__ uint32_t s_code[kPrepThreads + 1], s_zero[kPrepThreads + 1];
     if (blockIdx.x == 0 && threadIdx.x < 4 && ((a.zero >> threadIdx.x) & 1u)) a.counts[threadIdx.x] = 0ull;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.times) {
+        if (a.first) {
+            a.times[0] = ptx::global_ns();
+            a.times[1] = 0ull;
+        } else {
+            note_scan_end(a.times);
+        }
+    }
     const int64_t tile = a.base + (int64_t)blockIdx.x * kPrepTile;
     const int64_t p = tile + threadIdx.x * 16;
     const uint2 v = prep_pack16(a, p);
@@ -448,6 +467,7 @@ struct RescoreParams {
     int64_t hit_cap;
     int64_t keep_below;  // hits at positions >= keep_below are dropped (0: none are)
     int64_t pos_base;    // added to the positions written
+    unsigned long long *times;  // may be null
 };
 
 // One thread per record slot; the candidates of a warp's 32 records are then shared out
@@ -465,6 +485,10 @@ __global__ void __launch_bounds__(kRescoreThreads) rescore_kernel(RescoreParams 
     __shared__ HitRec s_hits[kRescoreThreads / 32][kRescoreBuf];
     __shared__ unsigned int s_cand;
     if (threadIdx.x == 0) s_cand = 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.times) {
+        note_scan_end(p.times);
+        p.times[3] = ptx::global_ns();
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     HitRec *buf = s_hits[threadIdx.x >> 5];

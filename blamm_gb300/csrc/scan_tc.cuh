@@ -154,6 +154,7 @@ struct TcParams {
     uint4 *cand;                      // candidate record slots: blocks of kRecBlock
     unsigned long long *cand_count;   // record slots reserved
     int64_t cand_cap;                 // record slots available (a multiple of kRecBlock, one spare block behind them)
+    unsigned long long *times;  // may be null
     int *status;         // bit 0: a device wait timed out
     long long wait_limit;  // clock64 cycles a wait may last
     int32_t debug_stall;   // test hook: who waits on a barrier nobody completes (kStall*)
@@ -326,6 +327,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
     // ---- set-up
     if (threadIdx.x < CTL_WORDS && threadIdx.x != CTL_TMEM) ctl[threadIdx.x] = threadIdx.x >= CTL_BLOCK ? (int)kNoBlock : 0;
     if (threadIdx.x == 0) {
+        if (p.times && blockIdx.x == 0) p.times[2] = ptx::global_ns();
         for (int s = 0; s < kEStages; ++s) {
             ptx::mbar_init(bars + 8 * (BAR_EFULL + s), 1);
             ptx::mbar_init(bars + 8 * (BAR_EEMPTY + s), kStream ? 1 : 2);
