@@ -520,11 +520,16 @@ int blamm_ctx_create(int device, blamm_ctx **out)
         cudaFuncAttributes fa;
         // fails if no sm_103a image fits
         // (the raw-score and role-timing instances are set up when they are launched)
-        for (const void *k : {(const void *)scan_tc_kernel<false, false, 1, false>,
-                              (const void *)scan_tc_kernel<false, false, 2, false>,
-                              (const void *)scan_tc_kernel<false, false, kE4M3, false>,
-                              (const void *)scan_tc_kernel<false, false, 1, true>,
-                              (const void *)scan_tc_kernel<false, false, 2, true>}) {
+        for (const void *k : {(const void *)scan_tc_kernel<false, false, 1, false, false>,
+                              (const void *)scan_tc_kernel<false, false, 2, false, false>,
+                              (const void *)scan_tc_kernel<false, false, kE4M3, false, false>,
+                              (const void *)scan_tc_kernel<false, false, 1, true, false>,
+                              (const void *)scan_tc_kernel<false, false, 2, true, false>,
+                              (const void *)scan_tc_kernel<false, false, 1, false, true>,
+                              (const void *)scan_tc_kernel<false, false, 2, false, true>,
+                              (const void *)scan_tc_kernel<false, false, kE4M3, false, true>,
+                              (const void *)scan_tc_kernel<false, false, 1, true, true>,
+                              (const void *)scan_tc_kernel<false, false, 2, true, true>}) {
             CK(cudaFuncGetAttributes(&fa, k));
             if (fa.maxThreadsPerBlock < kTcThreads)
                 return fail(ctx, BLAMM_ERR_UNSUPPORTED,
@@ -851,6 +856,10 @@ static int check_jobs(blamm_ctx *ctx, int64_t n)
                             : BLAMM_OK;
 }
 
+// Spare blocks of an enqueued scan, two per drain warp: whoever enqueued it learns from the counts how
+// many candidates there were, also of records that did not fit.
+static int64_t spare_slots(const blamm_ctx *ctx) { return (int64_t)ctx->sm_count * kEpiWarps * 2 * kRecBlock; }
+
 // Record slots a scan with this grid reserves beyond its records: every drain warp holds
 // one block it fills and one reserved ahead.
 static int64_t record_slots_reserved(int grid) { return (int64_t)grid * kEpiWarps * 2 * kRecBlock; }
@@ -894,7 +903,7 @@ static RescoreParams rescore_params(const blamm_ctx *ctx, const uint4 *cand, con
 }
 
 // One launch of the scan kernel instance that p asks for.
-template <bool kDump, bool kProf, bool kStream>
+template <bool kDump, bool kProf, bool kStream, bool kCount>
 static void launch_tc_as(const TcParams &p, int grid, uint32_t smem, cudaStream_t st)
 {
     auto go = [&](auto *kernel) {
@@ -902,17 +911,18 @@ static void launch_tc_as(const TcParams &p, int grid, uint32_t smem, cudaStream_
             cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kernel<<<grid, kTcThreads, smem, st>>>(p);
     };
-    if (p.terms == 2) go(scan_tc_kernel<kDump, kProf, 2, kStream>);
-    else if (!kStream && p.terms == kE4M3) go(scan_tc_kernel<kDump, kProf, kE4M3, false>);
-    else go(scan_tc_kernel<kDump, kProf, 1, kStream>);
+    if (p.terms == 2) go(scan_tc_kernel<kDump, kProf, 2, kStream, kCount>);
+    else if (!kStream && p.terms == kE4M3) go(scan_tc_kernel<kDump, kProf, kE4M3, false, kCount>);
+    else go(scan_tc_kernel<kDump, kProf, 1, kStream, kCount>);
 }
 
 template <bool kStream>
 static void launch_tc(const TcParams &p, bool dump, int grid, uint32_t smem, cudaStream_t st)
 {
-    if (dump) launch_tc_as<true, false, kStream>(p, grid, smem, st);
-    else if (p.prof) launch_tc_as<false, true, kStream>(p, grid, smem, st);
-    else launch_tc_as<false, false, kStream>(p, grid, smem, st);
+    if (dump) launch_tc_as<true, false, kStream, false>(p, grid, smem, st);
+    else if (p.prof) launch_tc_as<false, true, kStream, false>(p, grid, smem, st);
+    else if (p.ncand) launch_tc_as<false, false, kStream, true>(p, grid, smem, st);
+    else launch_tc_as<false, false, kStream, false>(p, grid, smem, st);
 }
 
 // The scan of n bases (p: the plan, candidates, counters, status; a: the packed stream and what
@@ -1965,7 +1975,7 @@ int blamm_reserve(blamm_ctx *ctx, int64_t max_positions, int64_t max_candidates)
         if ((rc = ensure_plan(ctx))) return rc;
         // record slots: at most one record per candidate, plus the blocks the warps reserve
         const int64_t slots = std::min(max_candidates + record_slots_reserved(ctx->sm_count), kMaxRecordSlots);
-        if ((rc = ensure_cand(ctx, slots))) return rc;
+        if ((rc = ensure_cand(ctx, slots + spare_slots(ctx)))) return rc;
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return BLAMM_OK;
@@ -1983,7 +1993,8 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
                     (long long)n);
     const bool tc = ctx->mode != BLAMM_MODE_FP32;
     const int terms = mode_terms(ctx);
-    if (tc && (!(ctx->plan_valid && ctx->plan_terms == terms) || ctx->cand_cap <= 0 ||
+    const int64_t cand_cap = ctx->cand_cap - spare_slots(ctx);  // (the spare blocks lie behind it)
+    if (tc && (!(ctx->plan_valid && ctx->plan_terms == terms) || cand_cap <= 0 ||
                (size_t)e16_entries(ctx, n) > ctx->cap_e16))
         return fail(ctx, BLAMM_ERR_STATE, "blamm_scan_enqueue: call blamm_reserve after changing the bank, "
                                           "columns, thresholds or mode");
@@ -2005,11 +2016,12 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
     TcParams p = tc_params(ctx, n);
     p.cand = ctx->d_cand;
     p.cand_count = cnt;
-    p.cand_cap = ctx->cand_cap;
+    p.cand_cap = cand_cap;
+    p.ncand = cnt + 3;
     p.status = reinterpret_cast<int *>(cnt + 2);
     int grid = 0;
     if (int rc = launch_tc_windows(ctx, p, a, ctx->d_e16, false, nullptr, &grid)) return rc;
-    return launch_rescore(ctx, rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
+    return launch_rescore(ctx, rescore_params(ctx, ctx->d_cand, cnt, cand_cap, ctx->d_seq2, ctx->d_zmask, n,
                                               d_run_start, nruns, d_hits, cnt + 1, hit_cap, cnt + 3), n, grid);
 }
 

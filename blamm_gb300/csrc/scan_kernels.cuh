@@ -447,6 +447,13 @@ __global__ void __launch_bounds__(kPlainThreads) plain_scores_kernel(PlainParams
 // it (the rest of the block is unused).
 constexpr int kRecBlockSlots = 128;
 
+// A chunk's positions before the end of the stream (those behind it are no candidates).
+__device__ __forceinline__ uint32_t valid_positions(int64_t n, uint32_t chunk)
+{
+    const int64_t room = n - (int64_t)chunk * 32;
+    return room >= 32 ? 0xffffffffu : room > 0 ? (1u << room) - 1u : 0u;
+}
+
 struct RescoreParams {
     const uint4 *cand;                // record slots
     const int32_t *slot_col;          // tile slot -> motif column
@@ -463,7 +470,7 @@ struct RescoreParams {
     const float *thr;
     void *hits;
     unsigned long long *hit_count;
-    unsigned long long *ncand;  // candidates (set mask bits), added up
+    unsigned long long *ncand;  // candidates (set mask bits), added up (the scan adds those of records that did not fit)
     int64_t hit_cap;
     int64_t keep_below;  // hits at positions >= keep_below are dropped (0: none are)
     int64_t pos_base;    // added to the positions written
@@ -517,9 +524,7 @@ __global__ void __launch_bounds__(kRescoreThreads) rescore_kernel(RescoreParams 
             chunk = r.x;
             slot = r.y;
             mask = r.z;
-            // positions past the end of the stream are no candidates
-            const int64_t room = p.n - (int64_t)chunk * 32;
-            if (room < 32) mask &= room > 0 ? (1u << room) - 1u : 0u;
+            mask &= valid_positions(p.n, chunk);
         }
         const int c = __popc(mask);
         my_cand += (unsigned int)c;

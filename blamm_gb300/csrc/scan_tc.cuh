@@ -112,6 +112,7 @@ constexpr int kLoadWarp = 17;    // TMA bulk copies of A tiles and E windows
 constexpr int kMmaWarp2 = 18;    // issuer of the odd jobs
 constexpr int kMmaWarp = 19;     // issuer of the even jobs; TMEM allocation
 constexpr int kRecBlock = kRecBlockSlots;  // candidate record slots a drain warp reserves at a time
+constexpr uint32_t kBlockTries = 1u << 24;  // looks for the next record block before a drain warp gives up (about 0.3 s)
 constexpr uint32_t kNoBlock = 0xFFFFFFFFu;  // no slot index: the capacity is below 2^31
 constexpr int kTcThreads = 640;  // 20 warps (registers are allocated per 4 warps)
 constexpr int kEStages = 6;      // E windows in flight
@@ -153,7 +154,9 @@ struct TcParams {
     uint32_t a_bytes;    // shared memory for A
     uint4 *cand;                      // candidate record slots: blocks of kRecBlock
     unsigned long long *cand_count;   // record slots reserved
-    int64_t cand_cap;                 // record slots available (a multiple of kRecBlock, one spare block behind them)
+    int64_t cand_cap;                 // record slots available (a multiple of kRecBlock); behind them: one spare
+                                      // block, or (ncand: kCount) two per drain warp, whose candidates
+    unsigned long long *ncand;        // are added to *ncand (the rescoring adds the others)
     unsigned long long *times;  // may be null
     int *status;         // bit 0: a device wait timed out
     long long wait_limit;  // clock64 cycles a wait may last
@@ -245,11 +248,36 @@ __device__ __forceinline__ uint32_t ge_mask(const uint32_t (&v)[32], uint64_t nt
 }
 
 // One block of record slots.  The capacity is a multiple of kRecBlock below 2^31; a block
-// reserved beyond it becomes the spare block behind the buffer, which nothing reads.
+// reserved beyond it becomes a spare block behind the buffer, which the rescoring does not read.
 __device__ __forceinline__ uint32_t reserve_block(const TcParams &p)
 {
     const unsigned long long b = atomicAdd(p.cand_count, (unsigned long long)kRecBlock);
     return b < (unsigned long long)p.cand_cap ? (uint32_t)b : (uint32_t)p.cand_cap;
+}
+
+// Spare block k (0, 1) of a drain warp.
+__device__ __forceinline__ uint32_t spare_block(const TcParams &p, int warp, int k)
+{
+    return (uint32_t)p.cand_cap + (((uint32_t)blockIdx.x * kEpiWarps + warp) * 2u + k) * kRecBlock;
+}
+
+// Adds the candidates of closed spare blocks to *ncand; block: per lane (kNoBlock or below the
+// capacity: none).  A whole warp.
+__device__ __noinline__ void count_spare(const TcParams &p, uint32_t block)
+{
+    const int lane = threadIdx.x & 31;
+    __threadfence_block();
+    for (uint32_t m = __ballot_sync(0xffffffffu, block != kNoBlock && block >= (uint32_t)p.cand_cap); m; m &= m - 1u) {
+        const uint4 *b = p.cand + __shfl_sync(0xffffffffu, block, __ffs(m) - 1);
+        const uint32_t n = __ldcg(&b->x);
+        uint32_t c = 0;
+        for (uint32_t k = 1u + lane; k <= n; k += 32) {
+            const uint4 r = __ldcg(b + k);
+            c += (uint32_t)__popc(r.z & valid_positions(p.n, r.x));
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0 && c) atomicAdd(p.ncand, (unsigned long long)c);
+    }
 }
 
 // The units of one CTA: unit u = group * nblocks + block, advanced without divisions after
@@ -306,11 +334,12 @@ __device__ __forceinline__ long long tick()
 
 // kDump: also write the raw accumulator of some positions (test hook);
 // kProf: role timing into p.prof; kTerms: p.terms (1 or 2 BF16 terms, or kE4M3,
-// one E4M3 term); kStream: A in chunks through a ring (tg == 1).  The scan itself
-// is <false, false, p.terms, *>.  The issuing threads run once per MMA and per
+// one E4M3 term); kStream: A in chunks through a ring (tg == 1); kCount: candidates of
+// records that do not fit are counted (p.ncand).  The scan itself is <false, false,
+// p.terms, *, *>.  The issuing threads run once per MMA and per
 // job, so every branch taken out of their loops at compile time shows in the
 // scan time (runtime mode switches cost 2-4 %).
-template <bool kDump, bool kProf, int kTerms, bool kStream>
+template <bool kDump, bool kProf, int kTerms, bool kStream, bool kCount>
 __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -567,24 +596,41 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         }
     } else if (warp == kBlockWarp) {
         // ============ record blocks: one ahead for every drain warp ============
+        // Lane k serves drain warp k.  That the block handed last was taken says that the one before
+        // it is closed: if it is a spare block, its candidates are counted, and it can be handed again.
+        // (One load and one vote a look: the loop shares its issue slots with four drain warps.)
+        const int word = lane < kEpiWarps ? CTL_BLOCK + lane : lane == kEpiWarps ? CTL_DONE : CTL_ABORT;
         long long gone = 0;  // when the abort was seen
+        uint32_t last = kNoBlock, before = kNoBlock;
+        int which = 0;
         for (bool done = false; !done;) {
-            done = ctl[CTL_DONE] == kEpiWarps;  // (read first: no block is taken after that)
+            const int v = ctl[word];
+            if (!__any_sync(0xffffffffu, lane < kEpiWarps ? v == (int)kNoBlock : lane == kEpiWarps ? v == kEpiWarps : v != 0)) {
+                __nanosleep(500);
+                continue;
+            }
+            done = ctl[CTL_DONE] == kEpiWarps;  // (read before the blocks: none is taken after that)
             if (*s_abort) {  // (the drain warps' waits end too; should they not, this one does)
                 if (gone == 0) gone = clock64();
                 done = done || clock64() - gone > 64 * p.wait_limit;
             }
             done = __any_sync(0xffffffffu, done);
-            if (lane < kEpiWarps) {
-                const uint32_t b = (uint32_t)ctl[CTL_BLOCK + lane];
-                if (done) {  // every reserved block states its count
-                    if (b != kNoBlock) p.cand[b] = make_uint4(0u, 0u, 0u, 0u);
-                } else if (b == kNoBlock) {
-                    ctl[CTL_BLOCK + lane] = (int)reserve_block(p);
-                }
+            const uint32_t b = lane < kEpiWarps ? (uint32_t)ctl[CTL_BLOCK + lane] : 0u;
+            const bool taken = b == kNoBlock;
+            if (kCount) {
+                count_spare(p, taken || done ? before : kNoBlock);
+                if (done) count_spare(p, taken ? last : kNoBlock);
+            }
+            if (done) {  // every reserved block states its count
+                if (lane < kEpiWarps && !taken) p.cand[b] = make_uint4(0u, 0u, 0u, 0u);
+            } else if (taken) {
+                uint32_t next = reserve_block(p);
+                if (kCount && next >= (uint32_t)p.cand_cap) next = spare_block(p, lane, which ^= 1);
+                before = last;
+                last = next;
+                ctl[CTL_BLOCK + lane] = (int)next;
             }
             __syncwarp();
-            if (!done) __nanosleep(500);
         }
     } else if (warp < kEpiWarps) {
         // ===================== epilogue (warps 0-15) ======================
@@ -604,11 +650,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
         };
         auto next_block = [&]() {
             close_block();
-            uint32_t b = (uint32_t)ctl[CTL_BLOCK + warp];
-            __syncwarp();
-            if (lane == 0) {
-                if (b == kNoBlock) b = reserve_block(p);
-                else ctl[CTL_BLOCK + warp] = (int)kNoBlock;
+            uint32_t b = 0;
+            if constexpr (kCount) {  // every block comes from warp 16, which counts the spare ones
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) {
+                    for (uint32_t k = 0; (b = (uint32_t)ctl[CTL_BLOCK + warp]) == kNoBlock; ++k)
+                        if (k == kBlockTries) {
+                            *s_abort = 1;
+                            b = (uint32_t)p.cand_cap;  // (the spare area)
+                            break;
+                        }
+                    ctl[CTL_BLOCK + warp] = (int)kNoBlock;
+                }
+            } else {
+                b = (uint32_t)ctl[CTL_BLOCK + warp];
+                __syncwarp();
+                if (lane == 0) {
+                    if (b == kNoBlock) b = reserve_block(p);
+                    else ctl[CTL_BLOCK + warp] = (int)kNoBlock;
+                }
             }
             rec = __shfl_sync(0xffffffffu, b, 0) + 1u;
             left = (uint32_t)(kRecBlock - 1);
@@ -710,8 +771,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) scan_tc_kernel(TcParams p)
             }
         }
         close_block();
+        __threadfence_block();
+        __syncwarp();
         if (lane == 0) {
-            __threadfence_block();
             atomicAdd(const_cast<int *>(ctl) + CTL_DONE, 1);
         }
         if (kProf && lane == 0 && warp == 0) {

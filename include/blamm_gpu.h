@@ -156,7 +156,8 @@ int blamm_filter_score(blamm_ctx *ctx, float *d_R, int m, int n, const float *d_
  * returns.  counts is device memory of 4 uint64, set when the stream gets
  * there: [0] candidate record slots used (a record holds the candidates of one
  * column in a 32-position chunk; each CTA's warps take slots in blocks), [1]
- * hits, [2] status (non-zero: a device wait timed out), [3] candidates.  Hits
+ * hits, [2] status (non-zero: a device wait timed out), [3] candidates, also
+ * those of records that did not fit.  Hits
  * beyond hit_cap and records beyond the reservation (max_candidates plus the
  * blocks the warps hold) are counted but not stored; the caller compares counts
  * with its capacities and scans again with more room.  BLAMM_ERR_STATE when the reservation or plan does not
