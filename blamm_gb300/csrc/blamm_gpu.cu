@@ -117,6 +117,7 @@ struct blamm_ctx {
     size_t cap_runs = 0;
     uint4 *d_cand = nullptr;  // candidate record slots (scan_tc.cuh: blocks of kRecBlock)
     int64_t cand_cap = 0;     // record slots
+    int64_t cand_spare = 0;   // spare ones behind them
     blamm_hit *d_hits = nullptr;
     int64_t hits_cap = 0;
     unsigned long long *d_counters = nullptr;  // record slots, hits, status (bit 0: a wait timed out), candidates; times
@@ -230,17 +231,24 @@ static void copy_out(void *dst, const void *src, size_t bytes)
         if (t.joinable()) t.join();
 }
 
-// Candidate record slots: `need` rounded up to whole blocks (the scan counts on it), and a
-// spare block behind them, where the scan puts what does not fit.
-static int ensure_cand(blamm_ctx *ctx, int64_t need)
+// Spare record slots of an enqueued scan, two blocks per drain warp: its counts say how many
+// candidates there were, also of records that did not fit.
+static int64_t spare_slots(const blamm_ctx *ctx) { return (int64_t)ctx->sm_count * kEpiWarps * 2 * kRecBlock; }
+
+// Candidate record slots: `need` rounded up to whole blocks (the scan counts on it), and behind
+// them spare ones, where the scan puts what does not fit.
+static int ensure_cand(blamm_ctx *ctx, int64_t need, int64_t spare = kRecBlock)
 {
     need = std::max<int64_t>(1, (need + kRecBlock - 1) / kRecBlock) * kRecBlock;
-    if (ctx->d_cand && need <= ctx->cand_cap) return BLAMM_OK;
-    size_t cap = ctx->d_cand ? (size_t)(ctx->cand_cap + kRecBlock) : 0;
-    ctx->cand_cap = 0;
-    const int rc = ensure(ctx, &ctx->d_cand, &cap, (size_t)(need + kRecBlock));
-    if (!rc) ctx->cand_cap = need;
-    return rc;
+    if (ctx->d_cand && need <= ctx->cand_cap && spare <= ctx->cand_spare) return BLAMM_OK;
+    need = std::max(need, ctx->cand_cap);
+    spare = std::max(spare, ctx->cand_spare);
+    size_t cap = (size_t)(ctx->cand_cap + ctx->cand_spare);
+    ctx->cand_cap = ctx->cand_spare = 0;
+    if (int rc = ensure(ctx, &ctx->d_cand, &cap, (size_t)(need + spare))) return rc;
+    ctx->cand_cap = need;
+    ctx->cand_spare = spare;
+    return BLAMM_OK;
 }
 
 static int scanned_columns(const blamm_ctx *ctx)
@@ -596,7 +604,7 @@ static int64_t call_buffer_bytes(const blamm_ctx *ctx)
                      8 * (ctx->cap_srun[0] + ctx->cap_srun[1] + ctx->cap_srun[2] + ctx->cap_shdr) +
                      16 * ctx->cap_ing_tiles + sizeof(IngPrefix) * ctx->cap_ing_prefix +
                      8 * ctx->cap_ing_totals + ctx->cap_theo) +
-           16 * (ctx->cand_cap > 0 ? ctx->cand_cap + kRecBlock : 0) + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
+           16 * (ctx->cand_cap + ctx->cand_spare) + (int64_t)sizeof(blamm_hit) * ctx->hits_cap;
 }
 
 int blamm_ctx_call_bytes(const blamm_ctx *ctx, int64_t *bytes)
@@ -637,7 +645,7 @@ int blamm_release_buffers(blamm_ctx *ctx)
     ctx->stream_n = ctx->stream_nruns = ctx->stream_nseqs = 0;
     if (ctx->d_cand) cudaFreeAsync(ctx->d_cand, ctx->stream);
     ctx->d_cand = nullptr;
-    ctx->cand_cap = 0;
+    ctx->cand_cap = ctx->cand_spare = 0;
     if (ctx->d_hits) cudaFreeAsync(ctx->d_hits, ctx->stream);
     ctx->d_hits = nullptr;
     ctx->hits_cap = 0;
@@ -855,10 +863,6 @@ static int check_jobs(blamm_ctx *ctx, int64_t n)
                                    "scan the stream in parts", njobs, (long long)kMaxJobs)
                             : BLAMM_OK;
 }
-
-// Spare blocks of an enqueued scan, two per drain warp: whoever enqueued it learns from the counts how
-// many candidates there were, also of records that did not fit.
-static int64_t spare_slots(const blamm_ctx *ctx) { return (int64_t)ctx->sm_count * kEpiWarps * 2 * kRecBlock; }
 
 // Record slots a scan with this grid reserves beyond its records: every drain warp holds
 // one block it fills and one reserved ahead.
@@ -1975,7 +1979,7 @@ int blamm_reserve(blamm_ctx *ctx, int64_t max_positions, int64_t max_candidates)
         if ((rc = ensure_plan(ctx))) return rc;
         // record slots: at most one record per candidate, plus the blocks the warps reserve
         const int64_t slots = std::min(max_candidates + record_slots_reserved(ctx->sm_count), kMaxRecordSlots);
-        if ((rc = ensure_cand(ctx, slots + spare_slots(ctx)))) return rc;
+        if ((rc = ensure_cand(ctx, slots, spare_slots(ctx)))) return rc;
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return BLAMM_OK;
@@ -1993,8 +1997,7 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
                     (long long)n);
     const bool tc = ctx->mode != BLAMM_MODE_FP32;
     const int terms = mode_terms(ctx);
-    const int64_t cand_cap = ctx->cand_cap - spare_slots(ctx);  // (the spare blocks lie behind it)
-    if (tc && (!(ctx->plan_valid && ctx->plan_terms == terms) || cand_cap <= 0 ||
+    if (tc && (!(ctx->plan_valid && ctx->plan_terms == terms) || ctx->cand_cap <= 0 ||
                (size_t)e16_entries(ctx, n) > ctx->cap_e16))
         return fail(ctx, BLAMM_ERR_STATE, "blamm_scan_enqueue: call blamm_reserve after changing the bank, "
                                           "columns, thresholds or mode");
@@ -2016,12 +2019,12 @@ int blamm_scan_enqueue(blamm_ctx *ctx, const char *d_bases, int64_t n, const int
     TcParams p = tc_params(ctx, n);
     p.cand = ctx->d_cand;
     p.cand_count = cnt;
-    p.cand_cap = cand_cap;
-    p.ncand = cnt + 3;
+    p.cand_cap = ctx->cand_cap;
+    p.ncand = ctx->cand_spare >= spare_slots(ctx) ? cnt + 3 : nullptr;  // (room that blamm_reserve makes)
     p.status = reinterpret_cast<int *>(cnt + 2);
     int grid = 0;
     if (int rc = launch_tc_windows(ctx, p, a, ctx->d_e16, false, nullptr, &grid)) return rc;
-    return launch_rescore(ctx, rescore_params(ctx, ctx->d_cand, cnt, cand_cap, ctx->d_seq2, ctx->d_zmask, n,
+    return launch_rescore(ctx, rescore_params(ctx, ctx->d_cand, cnt, ctx->cand_cap, ctx->d_seq2, ctx->d_zmask, n,
                                               d_run_start, nruns, d_hits, cnt + 1, hit_cap, cnt + 3), n, grid);
 }
 

@@ -52,3 +52,31 @@ def test_candidates_beyond_the_reservation_are_counted(mode, long):
     finally:
         ref.close()
         sc.close()
+
+
+def test_enqueue_behind_a_scan_without_a_reservation():
+    """The buffers that an ordinary scan of the same stream left behind hold an enqueued one too."""
+    torch = pytest.importorskip("torch")
+    from blamm_gb300 import GpuScanner
+    P, lens, thr = make_bank(961, 60, 5, 20, rel=0.9)
+    bases, runs = make_stream(962, 1_000_003, nruns=4)
+    sc = GpuScanner(0, "bf16")
+    try:
+        sc.set_motifs(P, lens, thr)
+        d_b, d_r = torch.from_numpy(bases).cuda(), torch.from_numpy(runs).cuda()
+        cap = 1 << 20
+        d_h = torch.zeros(cap * HIT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+        d_c = torch.zeros(4, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        args = (d_b.data_ptr(), len(bases), d_r.data_ptr(), len(runs), d_h.data_ptr(), cap)
+        nh = sc.scan_device(*args)
+        want = d_h.cpu().numpy().view(HIT_DTYPE)[:nh].copy()
+        d_h.zero_()
+        torch.cuda.synchronize()
+        sc.enqueue(*args, d_c.data_ptr())
+        torch.cuda.synchronize()
+        assert int(d_c[1]) == nh > 10_000
+        ok, msg = same_hits(d_h.cpu().numpy().view(HIT_DTYPE)[:nh], want)
+        assert ok, msg
+    finally:
+        sc.close()
