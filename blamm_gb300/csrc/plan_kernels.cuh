@@ -10,8 +10,9 @@
 //     min { sum(q) : sum(P) >= thr' } >= lambda thr' + sum_j min_b (q_jb - lambda P_jb)
 // (Lagrangian bound; a masked base is a fifth choice with q = P = 0).  lambda = 1 is the worst
 // case above; the best lambda is usually a few thousandths (BF16) or hundredths (E4M3) more.
-// A warp compares 64 values of lambda in FP32 and then forms the bound of the best one in FP64, or
-// takes the worst case where that is larger.  (Which lambda it is decides how tight the bound is,
+// A warp compares 64 values of lambda in FP32 and then forms the bound of the best one in 64-bit
+// fixed point (the FP64 units are slow here: a plan of 4000 columns takes 58 us in FP32 alone, 83
+// with the bound in FP64, 62 so), or takes the worst case (FP64) where that is larger.  (Which lambda it is decides how tight the bound is,
 // not whether it holds.)  Candidates per hit, 512 motifs x 16 Mi positions at p = 1e-4, by the worst
 // case and so: E4M3 2.03, 1.17; one BF16 term 1.25, 1.11.
 #pragma once
@@ -50,24 +51,24 @@ __device__ __forceinline__ float e4m3_units_f(uint32_t code)
     return code & 0x80u ? -a : a;
 }
 
-// Entry b of motif position j of a column, in units of 2^-s: the quantised value and P.
+// Entry i of a column in units of 2^-s: the quantised value (a whole number below 2^16) and P.
 struct PlanEntry {
-    double q, x;
+    float q, x;
 };
 __device__ __forceinline__ PlanEntry plan_entry(const PlanParams &p, const float *P, uint32_t o, int s, int i)
 {
     PlanEntry e;
-    e.x = ldexp((double)__ldg(P + i), s);
+    e.x = ldexpf(__ldg(P + i), s);
     if (p.terms == kE4M3) {
-        e.q = (double)e4m3_units_f(__ldg(p.e8 + o + i));
+        e.q = e4m3_units_f(__ldg(p.e8 + o + i));
     } else {
-        e.q = ldexp((double)__uint_as_float((uint32_t)__ldg(p.hi + o + i) << 16), s);
-        if (p.terms == 2) e.q += ldexp((double)__uint_as_float((uint32_t)__ldg(p.lo + o + i) << 16), s);  // exact
+        e.q = ldexpf(__uint_as_float((uint32_t)__ldg(p.hi + o + i) << 16), s);
+        if (p.terms == 2) e.q += ldexpf(__uint_as_float((uint32_t)__ldg(p.lo + o + i) << 16), s);  // exact
     }
     return e;
 }
 
-__device__ __forceinline__ double warp_sum(double v)
+__device__ __forceinline__ long long warp_sum(long long v)
 {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
@@ -101,23 +102,14 @@ __global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
     // each lane's two lambdas, in FP32: which one is best
     float sum[2] = {0.f, 0.f};
     for (int j = 0; j < L; ++j) {
-        float q[4], x[4];
+        PlanEntry e[4];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int i = 4 * j + b;
-            x[b] = ldexpf(__ldg(P + i), s);
-            if (e8) {
-                q[b] = e4m3_units_f(__ldg(p.e8 + o + i));
-            } else {
-                q[b] = ldexpf(__uint_as_float((uint32_t)__ldg(p.hi + o + i) << 16), s);
-                if (p.terms == 2) q[b] += ldexpf(__uint_as_float((uint32_t)__ldg(p.lo + o + i) << 16), s);
-            }
-        }
+        for (int b = 0; b < 4; ++b) e[b] = plan_entry(p, P, o, s, 4 * j + b);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float m = 0.f;
 #pragma unroll
-            for (int b = 0; b < 4; ++b) m = fminf(m, fmaf(-lam[h], x[b], q[b]));
+            for (int b = 0; b < 4; ++b) m = fminf(m, fmaf(-lam[h], e[b].x, e[b].q));
             sum[h] += m;
         }
     }
@@ -129,35 +121,41 @@ __global__ void __launch_bounds__(256) plan_thr_kernel(PlanParams p)
         const float ob = __shfl_xor_sync(0xffffffffu, best, d), ol = __shfl_xor_sync(0xffffffffu, l32, d);
         if (ob > best || (ob == best && ol < l32) || best != best) best = ob, l32 = ol;
     }
-    // its bound in FP64, motif positions over the lanes (all lanes then have the sums)
-    const double l = __shfl_sync(0xffffffffu, l32, 0);
-    double sum64 = 0.0, mag = 0.0, maxabs = 0.0;
+    // Its bound in whole numbers, motif positions over the lanes: lambda = l 2^-20, P = X 2^-15 to
+    // within 2^-16, so the sum is one of multiples of 2^-35 and off by at most L lambda 2^-16; |q|,
+    // |P| <= 2^15 and L <= 256 keep it below 2^62.
+    const int l = __float2int_rn(__shfl_sync(0xffffffffu, l32, 0) * 0x1p20f);
+    long long sum64 = 0, maxabs = 0;
+    bool fits = true;
     for (int j = lane; j < L; j += 32) {
-        double m = 0.0, mq = 0.0, mx = 0.0;
+        long long m = 0;
+        int mx = 0;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const PlanEntry e = plan_entry(p, P, o, s, 4 * j + b);
-            m = fmin(m, fma(-l, e.x, e.q));
-            mq = fmax(mq, fabs(e.q));
-            mx = fmax(mx, fabs(e.x));
+            fits = fits && fabsf(e.x) <= 32768.0f;
+            const int X = __float2int_rn(e.x * 0x1p15f);
+            m = min(m, ((long long)__float2int_rn(e.q) << 35) - (long long)l * X);
+            mx = max(mx, abs(X));
         }
         sum64 += m;
         maxabs += mx;
-        mag += mq + l * mx;
     }
     sum64 = warp_sum(sum64);
-    mag = warp_sum(mag);
     maxabs = warp_sum(maxabs);
+    fits = __all_sync(0xffffffffu, fits);
     if (lane != 0) return;
+    const double lambda = (double)l * 0x1p-20;
     // the reference's own rounding: |fl(sum) - sum| <= (L - 1) 2^-24 sum |P| (1 + 2^-14)
-    const double thr = ldexp((double)p.thr[c], s) - (double)L * 0x1p-24 * maxabs;
-    const double bound = fma(l, thr, sum64) - (double)(L + 8) * 0x1p-51 * (l * fabs(thr) + mag);  // (FP64's own rounding)
+    const double thr = ldexp((double)p.thr[c], s) - (double)L * 0x1p-24 * ((double)maxabs * 0x1p-15 + 1.0);
+    double bound = lambda * thr + (double)sum64 * 0x1p-35;
+    bound -= (double)L * lambda * 0x1p-16 + 0x1p-48 * (lambda * fabs(thr) + fabs((double)sum64) * 0x1p-35);  // (FP64's own rounding)
     // down to the grid, kept within the scores a window can reach (2^23 units; 64 L scaled):
     // below them every window is a candidate, above them none is
     const double worst = ((double)p.thr[c] - p.guard[c]) * exp2((double)s);
     const double lim = e8 ? (double)(64 * L + 1) * 512.0 : 8388608.0;
     double t = worst;
-    if (bound > t) t = bound;  // (NaN: not taken)
+    if (fits && bound > t) t = bound;  // (NaN: not taken)
     const double units = isnan(t) ? lim : floor(fmax(-lim, fmin(lim, t)));
     p.slot_thr[slot] = ldexpf((float)units, e8 ? -9 : -s);  // exact: |units| <= 2^23
 }
