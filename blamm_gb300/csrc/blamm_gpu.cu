@@ -1484,11 +1484,13 @@ static int scan_host_once(blamm_ctx *ctx, const char *bases, const char *d_bases
         cudaStreamSynchronize(ctx->stream);
         return rc;
     }
-    const int64_t ncopy = std::min<int64_t>(*n_hits, hit_cap), now = std::min(ncopy, first);
-    if (now > 0) std::memcpy(hits, ctx->h_stage + back_at + kHitsAt, sizeof(blamm_hit) * (size_t)now);
-    if (ncopy > now) {
-        CK(cudaMemcpyAsync(hits + now, d_hits + now, sizeof(blamm_hit) * (size_t)(ncopy - now), cudaMemcpyDeviceToHost,
-                           ctx->stream));
+    const int64_t ncopy = std::min<int64_t>(*n_hits, hit_cap);
+    if (ncopy <= first) {
+        if (ncopy > 0) std::memcpy(hits, ctx->h_stage + back_at + kHitsAt, sizeof(blamm_hit) * (size_t)ncopy);
+    } else {
+        // All of them in one copy: where the caller's pages are fresh, a copy behind a first part that
+        // the CPU has written takes longer (6.5 M hits into a new array: the call 4.7 ms, 4.0 so).
+        CK(cudaMemcpyAsync(hits, d_hits, sizeof(blamm_hit) * (size_t)ncopy, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
     }
     // (by the host's clock: a pair of events around the copies took 5 us of a 58 us call)
