@@ -190,6 +190,13 @@ __device__ __forceinline__ float ld_shared_f32(uint32_t a)
     return v;
 }
 
+__device__ __forceinline__ float2 ld_shared_v2(uint32_t a)
+{
+    float2 v;
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+
 __device__ __forceinline__ float4 ld_shared_v4(uint32_t a)
 {
     float4 v;

@@ -12,6 +12,7 @@
 // lengths and thresholds.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "blamm_gpu.h"
 
@@ -26,13 +27,6 @@ constexpr int kColBits = 20;       // a bank has fewer than 2^20 columns
 // ------------------------------------------------------------------------
 // helpers
 // ------------------------------------------------------------------------
-__device__ __forceinline__ int base_code_at(const uint32_t *seq2, const uint32_t *zmask, int64_t i)
-{
-    uint32_t z = (zmask[i >> 5] >> (i & 31)) & 1u;
-    uint32_t b = (seq2[i >> 4] >> (2 * (i & 15))) & 3u;
-    return z ? 4 : (int)b;
-}
-
 // Sequential FP32 score of the window at pos (motif position order, __fadd_rn: the
 // reference's sum), zero-masked bases adding nothing (adding +0 changes no sum that starts
 // at +0).  The 2-bit codes and mask bits of 16 positions come from two words of each array
@@ -246,9 +240,14 @@ __global__ void __launch_bounds__(kPrepThreads) prep_kernel(PrepParams a)
 // changes no sum that starts at +0.
 // What bounds it: shared memory, which delivers 128 bytes a cycle and SM whatever the lanes
 // share (a 16-byte load of a warp is four cycles): 32 additions a cycle and SM.  2 Mbp x 256
-// columns: 1.01 ms, 0.93 at that rate (one 4-byte load at a byte-coded address, a branch and an
+// columns: 1.02 ms, 0.93 at that rate (one 4-byte load at a byte-coded address, a branch and an
 // addition per motif position: 2.91); 8 Mbp x 64 columns with 250 bins: 1.09 (2.57 with a
 // division per score).  Banks of some dozen columns on longer streams are binned by hist_tc_kernel.
+// Motif positions from 32 on take their codes from two words per 32 bases, for each column group
+// anew (10 Mbp x 4 columns of 100-130 positions 0.65 ms; with two loads per position 1.30; with
+// byte codes in shared memory 1.22), and a group of one or two columns loads 4 or 8 bytes (10 Mbp x
+// 1 column of 12: 0.110 ms, 0.149 with 16, 0.123 in the byte-coded form; that is still ahead for one
+// column of more than 32 positions, 0.20 against 0.18 ms with 40-60).
 constexpr int kPlainThreads = 256;
 constexpr int kPlainReg = 32;  // motif positions whose offsets are kept in registers
 constexpr int kPlainRow = 5 * 16;  // bytes of one motif position of four columns
@@ -280,6 +279,28 @@ struct PlainParams {
     int32_t shared_bins;         // 1: the block's counts are in shared memory until it ends
     unsigned long long *counts;  // ncols x nbins
 };
+
+// The 32 bases from a position on: codes and zero mask; row16: 16 times the row of one of them.
+struct PlainCodes {
+    uint32_t code[2], zero;
+    __device__ __forceinline__ uint32_t row16(int i) const
+    {
+        const int sh = 2 * (i & 15) - 4;
+        const uint32_t c = (sh < 0 ? code[i >> 4] << -sh : code[i >> 4] >> sh) & 0x30u;
+        return (zero >> i) & 1u ? 0x40u : c;
+    }
+};
+__device__ __forceinline__ PlainCodes plain_codes(const uint32_t *seq2, const uint32_t *zmask, int64_t pos)
+{
+    const int64_t w = pos >> 4, wz = pos >> 5;
+    const uint32_t s = 2 * (uint32_t)(pos & 15);
+    const uint32_t w0 = __ldg(seq2 + w), w1 = __ldg(seq2 + w + 1), w2 = __ldg(seq2 + w + 2);
+    PlainCodes c;
+    c.code[0] = __funnelshift_r(w0, w1, s);
+    c.code[1] = __funnelshift_r(w1, w2, s);
+    c.zero = __funnelshift_r(__ldg(zmask + wz), __ldg(zmask + wz + 1), (uint32_t)(pos & 31));
+    return c;
+}
 
 struct alignas(16) HitRec {
     int64_t pos;
@@ -330,7 +351,7 @@ __device__ __forceinline__ int bin_of(float x, float w, float r)
 }
 
 template <bool kHist>
-__global__ void __launch_bounds__(kPlainThreads) plain_scores_kernel(PlainParams p)
+__global__ void __launch_bounds__(kPlainThreads, 4) plain_scores_kernel(PlainParams p)
 {
     extern __shared__ __align__(16) uint8_t smem_plain[];
     const int cpb = p.cols_per_block, ngrp = cpb / 4, lmax = p.lmax;
@@ -368,15 +389,11 @@ __global__ void __launch_bounds__(kPlainThreads) plain_scores_kernel(PlainParams
         // offsets of the 32 bases from pos on (the padded stream covers the reads)
         uint32_t off[kPlainReg];
         {
-            const int64_t w = pos >> 4, wz = pos >> 5;
-            const uint32_t s = 2 * (uint32_t)(pos & 15);
-            const uint32_t w0 = __ldg(p.seq2 + w), w1 = __ldg(p.seq2 + w + 1), w2 = __ldg(p.seq2 + w + 2);
-            const uint32_t code[2] = {__funnelshift_r(w0, w1, s), __funnelshift_r(w1, w2, s)};
-            const uint32_t zero = __funnelshift_r(__ldg(p.zmask + wz), __ldg(p.zmask + wz + 1), (uint32_t)(pos & 31));
+            const PlainCodes c = plain_codes(p.seq2, p.zmask, pos);
 #pragma unroll
             for (int j = 0; j < kPlainReg; ++j) {
-                const uint32_t b = (zero >> j) & 1u ? 4u : (code[j >> 4] >> (2 * (j & 15))) & 3u;
-                off[j] = base + (uint32_t)(j * kPlainRow) + 16u * b;
+                if ((j & 3) == 0 && j >= lmax) break;
+                off[j] = base + (uint32_t)(j * kPlainRow) + c.row16(j);
             }
         }
         for (int g = 0; g < ngrp; ++g) {
@@ -384,23 +401,50 @@ __global__ void __launch_bounds__(kPlainThreads) plain_scores_kernel(PlainParams
             const int L = max(max(len.x, len.y), max(len.z, len.w));
             const uint32_t at = (uint32_t)(g * lmax * kPlainRow);
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-            auto add = [&](uint32_t a) {
-                const float4 v = ptx::ld_shared_v4(a);
-                s.x = __fadd_rn(s.x, v.x);
-                s.y = __fadd_rn(s.y, v.y);
-                s.z = __fadd_rn(s.z, v.z);
-                s.w = __fadd_rn(s.w, v.w);
-            };
+            // (W: the group's columns that exist, 1, 2 or more; less is loaded for fewer)
+            auto scores = [&](auto W) {
+                auto add = [&](uint32_t a) {
+                    if constexpr (decltype(W)::value == 1) {
+                        s.x = __fadd_rn(s.x, ptx::ld_shared_f32(a));
+                    } else if constexpr (decltype(W)::value == 2) {
+                        const float2 v = ptx::ld_shared_v2(a);
+                        s.x = __fadd_rn(s.x, v.x);
+                        s.y = __fadd_rn(s.y, v.y);
+                    } else {
+                        const float4 v = ptx::ld_shared_v4(a);
+                        s.x = __fadd_rn(s.x, v.x);
+                        s.y = __fadd_rn(s.y, v.y);
+                        s.z = __fadd_rn(s.z, v.z);
+                        s.w = __fadd_rn(s.w, v.w);
+                    }
+                };
 #pragma unroll
-            for (int j = 0; j < kPlainReg; j += 4) {
-                if (j >= L) break;
-                add(off[j] + at);
-                if (j + 1 < L) add(off[j + 1] + at);
-                if (j + 2 < L) add(off[j + 2] + at);
-                if (j + 3 < L) add(off[j + 3] + at);
-            }
-            for (int j = kPlainReg; j < L; ++j)
-                add(base + at + (uint32_t)(j * kPlainRow) + 16u * (uint32_t)base_code_at(p.seq2, p.zmask, pos + j));
+                for (int j = 0; j < kPlainReg; j += 4) {
+                    if (j >= L) break;
+                    add(off[j] + at);
+                    if (j + 1 < L) add(off[j + 1] + at);
+                    if (j + 2 < L) add(off[j + 2] + at);
+                    if (j + 3 < L) add(off[j + 3] + at);
+                }
+                // longer motifs: 32 bases at a time, offsets made for this group
+                for (int j0 = kPlainReg; j0 < L; j0 += 32) {
+                    const PlainCodes c = plain_codes(p.seq2, p.zmask, pos + j0);
+                    const uint32_t row = base + at + (uint32_t)(j0 * kPlainRow);
+                    const int left = L - j0;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        if (i >= left) break;
+                        add(row + (uint32_t)(i * kPlainRow) + c.row16(i));
+                        if (i + 1 < left) add(row + (uint32_t)((i + 1) * kPlainRow) + c.row16(i + 1));
+                        if (i + 2 < left) add(row + (uint32_t)((i + 2) * kPlainRow) + c.row16(i + 2));
+                        if (i + 3 < left) add(row + (uint32_t)((i + 3) * kPlainRow) + c.row16(i + 3));
+                    }
+                }
+            };
+            const int width = nc - 4 * g;
+            if (width > 2) scores(std::integral_constant<int, 4>());
+            else if (width == 2) scores(std::integral_constant<int, 2>());
+            else scores(std::integral_constant<int, 1>());
             const float sc[4] = {s.x, s.y, s.z, s.w};
             const int ln[4] = {len.x, len.y, len.z, len.w};
             if (kHist) {
